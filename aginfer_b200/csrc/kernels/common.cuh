@@ -27,6 +27,9 @@ enum : unsigned {
   kFlagLayerNorm = 1u << 10, // fused prologue: LayerNorm (no affine) over each activation row before the GEMM
   kFlagLnModulate = 1u << 11, // ... followed by y * (1 + scale[k]) + shift[k] (AdaLN)
   kFlagSlab = 1u << 12,       // bulk-stream GEMM: whole K in one slot, rows unpadded, one copy per operand
+  kFlagSwiglu = 1u << 13,     // the first two matrices are gate and up of the same width: y = silu(gate) * up
+  kFlagMulSilu = 1u << 14,    // y = silu(gate[m, n]) * (...), the gate (bf16, pitch of y) in place of the residual
+  kFlagAmax = 1u << 15,       // fold max |y| of the rounded outputs into a zero-initialised word
 };
 
 // Programmatic dependent launch: when the loader launches with programmatic stream
@@ -48,6 +51,17 @@ __device__ __forceinline__ void grid_dependency_wait_then_release() {
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // release as early as possible, then wait
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ void grid_dependency_only_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// True in exactly one lane of a converged warp, the same one every time.  The compiler knows it to be a single
+// thread, so instructions that take warp-uniform operands (tcgen05.mma, cp.async.bulk) issue without the operand
+// moves that a lane comparison costs: 39 instead of 99 cycles per MMA, 17 instead of 54 per bulk copy.
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -37,7 +37,7 @@ constexpr unsigned kProducers = 128;
 constexpr unsigned kThreads = 160;        // 4 producer/epilogue warps + 1 MMA warp
 constexpr unsigned kMaxStages = 12;
 constexpr int kLag = 2;                   // a stage is published two commits after it was issued
-constexpr unsigned kSpinLimit = 1u << 22;
+constexpr unsigned kSpinLimit = 1u << 20;
 
 enum Status : unsigned { kOkStatus = 0, kTimeoutFull = 0x100, kTimeoutEmpty = 0x200, kTimeoutAccum = 0x300 };
 
@@ -49,20 +49,18 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("{ .reg .b64 t; mbarrier.arrive.shared::cta.b64 t, [%0]; }" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {
-  unsigned done;
-  asm volatile(
-      "{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-// Bounded wait; on expiry writes `code` to the status word once and returns false.
+// Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
+// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
+  const unsigned addr = smem_u32(bar);
   for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
-    if (mbar_test(bar, parity)) return true;
-    if (spin > 64) __nanosleep(32);
+    unsigned done;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
   }
   atomicCAS(status, 0u, code);
   return false;
@@ -284,17 +282,12 @@ __device__ __forceinline__ void finish_rows(const float* partial, size_t slab, u
   }
 }
 
-// kPacked: both operands are stored "K-block-major, swizzled" (see recipes/layout.py): the 128-byte K block kb
-// of row r lives at ((kb * rows_padded + r) * 128) with its 16-byte chunk c at position c ^ (r & 7), i.e. the
-// image of the shared-memory tile.  A ring slot is then filled by two bulk copies (16 KB of weights, TN * 128 B
-// of activations) issued by one thread, instead of 16-byte copies by 128 threads; `ldx` carries the padded
-// row count of the activation matrix.
-template <bool kFp8, int kCluster = 1, bool kPacked = false>
+template <bool kFp8>
 __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, void* y, const bf16* bias,
                                           const bf16* residual, const float* scale_a, const float* scale_w,
                                           float* partial, unsigned* counters, unsigned* status, unsigned M,
                                           unsigned N, unsigned K, unsigned ldx, unsigned ldy, unsigned flags,
-                                          unsigned TN, unsigned stages, unsigned tile_x = 0xffffffffu) {
+                                          unsigned TN, unsigned stages) {
   extern __shared__ unsigned char dynamic_smem[];
   __shared__ __align__(8) unsigned long long full_bar[kMaxStages];
   __shared__ __align__(8) unsigned long long empty_bar[kMaxStages];
@@ -304,8 +297,7 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
 
   const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned elem = kFp8 ? 1u : 2u;
-  if (tile_x == 0xffffffffu) tile_x = blockIdx.x;  // batched launches pass the tile index inside their matrix
-  const unsigned n0 = tile_x * kTileN, m0 = blockIdx.y * TN;
+  const unsigned n0 = blockIdx.x * kTileN, m0 = blockIdx.y * TN;
   const unsigned splits = gridDim.z, split = blockIdx.z;
   const unsigned k_blocks_total = (K * elem) / kRowBytes;
   const unsigned per_split = (k_blocks_total + splits - 1) / splits;
@@ -315,15 +307,12 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
   const unsigned stage_bytes = kATileBytes + TN * kRowBytes;
   const unsigned ring = (smem_u32(dynamic_smem) + 1023u) & ~1023u;  // tiles need 1024-byte alignment
   const unsigned columns = tmem_columns_for(TN);
-  // Cluster mode: [slice][token / kCluster][128 rows] fp32 gather buffer behind the ring.
-  const unsigned gather_cols = (TN + kCluster - 1) / kCluster;
-  const unsigned gather_base = ring + stages * stage_bytes;
   const unsigned Np = gridDim.x * kTileN;  // row stride of the split-K slabs: N rounded up to whole tiles
   if (stages > kMaxStages) stages = kMaxStages;
 
   if (tid == 0) {
     for (unsigned s = 0; s < stages; ++s) {
-      mbar_init(&full_bar[s], kPacked ? 1 : kProducers);
+      mbar_init(&full_bar[s], kProducers);
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&accum_bar, 1);
@@ -334,10 +323,6 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
   __syncthreads();
   tc_fence_after();
   const unsigned tmem_base = tmem_slot;
-  // Cluster split-K: every slice must be running (its shared memory live) before anyone writes into it.
-  // Arrive now, wait only just before the first remote store: by then the barrier has long completed.
-  if (kCluster > 1) cluster_arrive();
-
   // Weights do not depend on the previous kernel: the weight tiles of the first ring slots are requested
   // before the grid-dependency wait (they join the first commit group below).
   const size_t w_row_bytes = size_t(K) * elem, x_row_bytes = size_t(ldx) * elem;
@@ -360,47 +345,13 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
     for (unsigned j = 0; j < 8; ++j)
       if (j < a_rows) cp_async_16(dst + j * 2048, src + j * w_step);
   };
-  // packed operands: tile (first row r0, K block kb) is one contiguous run
-  const unsigned w_rows_padded = ((N + 255u) / 256u) * 256u;   // packed weights are padded to whole 256-row tiles
-  const unsigned b_tile_bytes = TN * kRowBytes;
-  auto packed_weights = [&](unsigned i) {
-    bulk_copy(ring + (i % stages) * stage_bytes, w + (size_t(kb_begin + i) * w_rows_padded + n0) * kRowBytes, kATileBytes,
-              &full_bar[i % stages]);
-  };
-  auto packed_tokens = [&](unsigned i) {
-    bulk_copy(ring + (i % stages) * stage_bytes + kATileBytes, x + (size_t(kb_begin + i) * ldx + m0) * kRowBytes,
-              b_tile_bytes, &full_bar[i % stages]);
-  };
-  if (kPacked) {
-    if (tid == 0)
-      for (unsigned i = 0; i < early; ++i) {
-        expect_bytes(&full_bar[i], kATileBytes + b_tile_bytes);
-        packed_weights(i);
-      }
-  } else if (warp < 4) {
+  if (warp < 4) {
     for (unsigned i = 0; i < early; ++i) load_weights(i);
   }
 
   grid_dependency_wait();
 
-  if (kPacked && warp < 4) {
-    // ---------------- warp 0 is the producer: two bulk copies per ring slot, issued by its lane 0 ----------------
-    // (the whole warp walks the loop so that it reaches the epilogue converged; warps 1-3 go straight there)
-    if (warp == 0) {
-      if (lane == 0)
-        for (unsigned i = 0; i < early; ++i) packed_tokens(i);
-      for (unsigned i = early; i < nkb; ++i) {
-        const unsigned s = i % stages;
-        mbar_wait(&empty_bar[s], (i / stages - 1) & 1, status, kTimeoutEmpty | s);
-        if (lane == 0) {
-          expect_bytes(&full_bar[s], kATileBytes + b_tile_bytes);
-          packed_weights(i);
-          packed_tokens(i);
-        }
-        __syncwarp();
-      }
-    }
-  } else if (warp < 4) {
+  if (warp < 4) {
     // ---------------- producers ----------------
     for (unsigned i = 0; i < nkb + kLag; ++i) {
       if (i < nkb) {
@@ -421,13 +372,13 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
       }
     }
   } else {
-    // ---------------- MMA warp: every lane waits, lane 0 issues ----------------
-    const unsigned idesc = instr_descriptor<kFp8>(TN);
-    for (unsigned i = 0; i < nkb; ++i) {
-      const unsigned s = i % stages, round = i / stages;
-      mbar_wait(&full_bar[s], round & 1, status, kTimeoutFull | s);
-      tc_fence_after();
-      if (lane == 0) {
+    // ---------------- MMA warp: one elected lane walks the ring ----------------
+    if (elect_one()) {
+      const unsigned idesc = instr_descriptor<kFp8>(TN);
+      for (unsigned i = 0; i < nkb; ++i) {
+        const unsigned s = i % stages, round = i / stages;
+        mbar_wait(&full_bar[s], round & 1, status, kTimeoutFull | s);
+        tc_fence_after();
         const unsigned a_base = ring + s * stage_bytes, b_base = a_base + kATileBytes;
         const unsigned long long a_desc = smem_descriptor(a_base), b_desc = smem_descriptor(b_base);
 #pragma unroll
@@ -435,11 +386,9 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
           mma<kFp8>(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (i | k) != 0);
         tc_commit(&empty_bar[s]);
       }
-      __syncwarp();
+      tc_commit(&accum_bar);
     }
-    if (lane == 0) tc_commit(&accum_bar);
     __syncwarp();
-    if (kCluster > 1) cluster_wait();  // every thread pairs its early arrive with one wait
   }
 
   // ---------------- epilogue (warps 0-3: TMEM lanes 32 * warp ... +31) ----------------
@@ -450,9 +399,7 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
     const float alpha = (flags & kFlagScaled) ? (*scale_a) * (*scale_w) : 1.f;
     const float bias_v = ((flags & kFlagBias) && n < N) ? __bfloat162float(bias[n]) : 0.f;
     const unsigned lane_addr = tmem_base + ((warp * 32u) << 16);
-    if (kCluster > 1) cluster_wait();  // peers are running: their gather buffers may be written
     for (unsigned c0 = 0; c0 < TN; c0 += 16) {
-      if (kCluster > 1 && m0 + c0 >= M) break;  // token columns past M carry nothing
       float v[16];
       if (nkb > 0) {
         tmem_load16(lane_addr + c0, v);
@@ -460,7 +407,7 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = 0.f;
       }
-      if (kCluster == 1 && splits == 1) {
+      if (splits == 1) {
         // direct store: bias was fetched once per thread, flags are tested once per 16 tokens
         if (n < N && m0 + c0 < M) {
           const unsigned count = min(16u, M - (m0 + c0));
@@ -474,7 +421,7 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
             else store_tokens16<false, false>(v, count, y, residual, offset, ldy, alpha, bias_v, flags);
           }
         }
-      } else if (kCluster == 1) {
+      } else {
         // split-K slab: one base address per 16 tokens, rows Np apart
         if (n < N && m0 + c0 < M) {
           const unsigned count = min(16u, M - (m0 + c0));
@@ -483,64 +430,15 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
           for (int i = 0; i < 16; ++i)
             if (unsigned(i) < count) __stcg(cell + size_t(i) * Np, v[i]);
         }
-      } else if (n < N) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const unsigned m = m0 + c0 + i;
-          if (m >= M) continue;
-          if (kCluster > 1) {
-            // token m is finished by cluster rank m % kCluster: send it this slice's partial sum,
-            // filed under [this rank][m / kCluster][row of W]
-            const unsigned c = c0 + i, owner = c % kCluster;
-            const unsigned cell = gather_base + (((split * gather_cols) + c / kCluster) * kTileN + warp * 32 + lane) * 4;
-            store_peer_f32(peer_smem(cell, owner), v[i]);
-          }
-        }
       }
     }
-    if (kCluster == 1 && splits > 1) __threadfence();  // partial sums ordered before this CTA's arrival count
+    if (splits > 1) __threadfence();  // partial sums ordered before this CTA's arrival count
     tc_fence_before();
   }
   __syncthreads();
   if (warp == 4) {
     tc_fence_after();
     tmem_free(tmem_base, columns);
-  }
-  if (kCluster > 1) {
-    // ---------------- split-K inside a cluster: partial sums travelled through distributed shared memory ----
-    // This rank finishes tokens split, split + C, ...: their bias and residual values are fetched while the
-    // cluster barrier completes.
-    constexpr int kMine = (64 + kCluster - 1) / kCluster;   // at most 64 tokens in cluster mode
-    const unsigned n = n0 + warp * 32 + lane;
-    const unsigned my_tokens = warp < 4 && n < N && split < min(TN, M - m0)
-                                   ? (min(TN, M - m0) - split + kCluster - 1) / kCluster : 0;
-    bf16 early_bias = __float2bfloat16_rn(0.f), early_res[kMine];
-    if (my_tokens != 0 && (flags & kFlagBias)) early_bias = bias[n];
-#pragma unroll
-    for (int j = 0; j < kMine; ++j)
-      if (unsigned(j) < my_tokens && (flags & kFlagResidual))
-        early_res[j] = residual[size_t(m0 + split + j * kCluster) * ldy + n];
-    cluster_arrive();
-    cluster_wait();  // every slice's stores into this CTA's gather buffer are complete and visible
-    if (my_tokens != 0) {
-      const float alpha = (flags & kFlagScaled) ? (*scale_a) * (*scale_w) : 1.f;
-      const float* mine = reinterpret_cast<const float*>(dynamic_smem + (gather_base - smem_u32(dynamic_smem)));
-#pragma unroll
-      for (int j = 0; j < kMine; ++j) {
-        if (unsigned(j) >= my_tokens) break;
-        float total = 0.f;
-#pragma unroll
-        for (int z = 0; z < kCluster; ++z) total += mine[((z * gather_cols) + j) * kTileN + warp * 32 + lane];  // slice order
-        float r = total * alpha;
-        if (flags & kFlagBias) r += __bfloat162float(early_bias);
-        r = apply_activation(r, flags);
-        if (flags & kFlagResidual) r += __bfloat162float(early_res[j]);
-        const size_t at = size_t(m0 + split + j * kCluster) * ldy + n;
-        if (flags & kFlagOutF32) static_cast<float*>(y)[at] = r;
-        else static_cast<bf16*>(y)[at] = __float2bfloat16_rn(r);
-      }
-    }
-    return;
   }
   if (splits == 1) return;
 
@@ -570,128 +468,6 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
 }
 
 }  // namespace tc
-
-// Cluster split-K variants: grid.z = cluster size = number of K slices (2, 3, 4, 6 or 8); partial sums are
-// exchanged through distributed shared memory, so `partial` and `counters` are unused.  For up to 64 tokens.
-// Dynamic shared memory = stages * (16384 + TN * 128) + 1024 + C * ceil(TN / C) * 512.
-#define AGI_TC_CLUSTER_KERNEL(NAME, TYPE, FP8, C)                                                                     \
-  extern "C" __global__ void __cluster_dims__(1, 1, C) __launch_bounds__(tc::kThreads, 1)                            \
-  NAME(const TYPE* x, const TYPE* w, void* y, const bf16* bias, const bf16* residual, const float* scale_a,         \
-       const float* scale_w, float* partial, unsigned* counters, unsigned* status, unsigned M, unsigned N,          \
-       unsigned K, unsigned ldx, unsigned ldy, unsigned flags, unsigned TN, unsigned stages) {                      \
-    tc::gemm_body<FP8, C>(reinterpret_cast<const uint8_t*>(x), reinterpret_cast<const uint8_t*>(w), y, bias,         \
-                          residual, scale_a, scale_w, partial, counters, status, M, N, K, ldx, ldy, flags, TN,      \
-                          stages);                                                                                   \
-  }
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_bf16_c2, bf16, false, 2)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_bf16_c3, bf16, false, 3)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_bf16_c4, bf16, false, 4)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_bf16_c6, bf16, false, 6)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_bf16_c8, bf16, false, 8)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_e4m3_c2, uint8_t, true, 2)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_e4m3_c4, uint8_t, true, 4)
-AGI_TC_CLUSTER_KERNEL(agi_gemm_tc_e4m3_c8, uint8_t, true, 8)
-#undef AGI_TC_CLUSTER_KERNEL
-
-// Up to 16 independent GEMMs that share the activation matrix (e.g. the K and V projections of every
-// cross-attention block over the same context tokens) as ONE launch: grid.x = segments * ceil(N / 128);
-// segment s multiplies by w[s], adds bias[s] and writes y + s * seg_stride elements.  No split-K.
-extern "C" __global__ void __launch_bounds__(tc::kThreads, 1)
-agi_gemm_tc_bf16_x16(const bf16* x, void* y, unsigned* status, unsigned M, unsigned N, unsigned K, unsigned ldx,
-                     unsigned ldy, unsigned flags, unsigned TN, unsigned stages, unsigned seg_stride,
-                     const bf16* w0, const bf16* w1, const bf16* w2, const bf16* w3, const bf16* w4, const bf16* w5,
-                     const bf16* w6, const bf16* w7, const bf16* w8, const bf16* w9, const bf16* w10,
-                     const bf16* w11, const bf16* w12, const bf16* w13, const bf16* w14, const bf16* w15,
-                     const bf16* b0, const bf16* b1, const bf16* b2, const bf16* b3, const bf16* b4, const bf16* b5,
-                     const bf16* b6, const bf16* b7, const bf16* b8, const bf16* b9, const bf16* b10,
-                     const bf16* b11, const bf16* b12, const bf16* b13, const bf16* b14, const bf16* b15) {
-  const unsigned tiles = (N + tc::kTileN - 1) / tc::kTileN;
-  const unsigned seg = blockIdx.x / tiles;
-  const bf16 *w, *b;
-  switch (seg) {
-    case 0: w = w0; b = b0; break;    case 1: w = w1; b = b1; break;    case 2: w = w2; b = b2; break;
-    case 3: w = w3; b = b3; break;    case 4: w = w4; b = b4; break;    case 5: w = w5; b = b5; break;
-    case 6: w = w6; b = b6; break;    case 7: w = w7; b = b7; break;    case 8: w = w8; b = b8; break;
-    case 9: w = w9; b = b9; break;    case 10: w = w10; b = b10; break; case 11: w = w11; b = b11; break;
-    case 12: w = w12; b = b12; break; case 13: w = w13; b = b13; break; case 14: w = w14; b = b14; break;
-    default: w = w15; b = b15; break;
-  }
-  tc::gemm_body<false>(reinterpret_cast<const uint8_t*>(x), reinterpret_cast<const uint8_t*>(w),
-                       static_cast<bf16*>(y) + size_t(seg) * seg_stride, b, b, nullptr, nullptr, nullptr, nullptr, status,
-                       M, N, K, ldx, ldy, flags, TN, stages, blockIdx.x % tiles);
-}
-
-// Up to three GEMMs over the same activation matrix as ONE launch (Q | K | V, gate | up): part i multiplies
-// by w_i [N_i, K], scales by scale_a * sw_i, adds bias_i and writes y_i with row pitch ldy_i.  The parts'
-// 128-row tiles are laid end to end along grid.x = sum of ceil(N_i / 128); no split-K.
-#define AGI_TC_GROUP_KERNEL(NAME, TYPE, FP8, PACKED)                                                                  \
-  extern "C" __global__ void __launch_bounds__(tc::kThreads, 1)                                                      \
-  NAME(const TYPE* x, const float* scale_a, unsigned* status, unsigned M, unsigned K, unsigned ldx, unsigned flags,   \
-       unsigned TN, unsigned stages, const TYPE* w0, const bf16* bias0, const float* sw0, void* y0, unsigned N0,      \
-       unsigned ldy0, const TYPE* w1, const bf16* bias1, const float* sw1, void* y1, unsigned N1, unsigned ldy1,      \
-       const TYPE* w2, const bf16* bias2, const float* sw2, void* y2, unsigned N2, unsigned ldy2) {                   \
-    const unsigned t0 = (N0 + tc::kTileN - 1) / tc::kTileN, t1 = (N1 + tc::kTileN - 1) / tc::kTileN;                  \
-    const TYPE* w = w0;                                                                                               \
-    const bf16* bias = bias0;                                                                                         \
-    const float* sw = sw0;                                                                                            \
-    void* y = y0;                                                                                                     \
-    unsigned N = N0, ldy = ldy0, tile = blockIdx.x;                                                                   \
-    if (tile >= t0 + t1) {                                                                                            \
-      w = w2; bias = bias2; sw = sw2; y = y2; N = N2; ldy = ldy2; tile -= t0 + t1;                                    \
-    } else if (tile >= t0) {                                                                                          \
-      w = w1; bias = bias1; sw = sw1; y = y1; N = N1; ldy = ldy1; tile -= t0;                                         \
-    }                                                                                                                 \
-    tc::gemm_body<FP8, 1, PACKED>(reinterpret_cast<const uint8_t*>(x), reinterpret_cast<const uint8_t*>(w), y, bias,  \
-                                  bias, scale_a, sw, nullptr, nullptr, status, M, N, K, ldx, ldy, flags, TN, stages,  \
-                                  tile);                                                                              \
-  }
-AGI_TC_GROUP_KERNEL(agi_gemm_tc_bf16_x3, bf16, false, false)
-AGI_TC_GROUP_KERNEL(agi_gemm_tc_e4m3_x3, uint8_t, true, false)
-// the same over packed operands (bulk-copy producers; ldx = padded row count of the activation matrix)
-AGI_TC_GROUP_KERNEL(agi_gemm_tcp_e4m3_x3, uint8_t, true, true)
-#undef AGI_TC_GROUP_KERNEL
-
-// The grouped launch with K slices in a thread-block cluster (up to 64 tokens, bf16): grid = (sum of ceil(N_i / 128),
-// 1, C), cluster (1, 1, C); the slices of a tile exchange partial sums through distributed shared memory as in
-// agi_gemm_tc_bf16_c*.  Three small projections of one layer (queries | keys | values, gate | up) become one launch.
-// Dynamic shared memory = stages * (16384 + TN * 128) + 1024 + C * ceil(TN / C) * 512.
-#define AGI_TC_GROUP_CLUSTER_KERNEL(NAME, C)                                                                          \
-  extern "C" __global__ void __cluster_dims__(1, 1, C) __launch_bounds__(tc::kThreads, 1)                            \
-  NAME(const bf16* x, const float* scale_a, unsigned* status, unsigned M, unsigned K, unsigned ldx, unsigned flags,   \
-       unsigned TN, unsigned stages, const bf16* w0, const bf16* bias0, const float* sw0, void* y0, unsigned N0,      \
-       unsigned ldy0, const bf16* w1, const bf16* bias1, const float* sw1, void* y1, unsigned N1, unsigned ldy1,      \
-       const bf16* w2, const bf16* bias2, const float* sw2, void* y2, unsigned N2, unsigned ldy2) {                   \
-    const unsigned t0 = (N0 + tc::kTileN - 1) / tc::kTileN, t1 = (N1 + tc::kTileN - 1) / tc::kTileN;                  \
-    const bf16* w = w0;                                                                                               \
-    const bf16* bias = bias0;                                                                                         \
-    void* y = y0;                                                                                                     \
-    unsigned N = N0, ldy = ldy0, tile = blockIdx.x;                                                                   \
-    if (tile >= t0 + t1) {                                                                                            \
-      w = w2; bias = bias2; y = y2; N = N2; ldy = ldy2; tile -= t0 + t1;                                              \
-    } else if (tile >= t0) {                                                                                          \
-      w = w1; bias = bias1; y = y1; N = N1; ldy = ldy1; tile -= t0;                                                   \
-    }                                                                                                                 \
-    tc::gemm_body<false, C, false>(reinterpret_cast<const uint8_t*>(x), reinterpret_cast<const uint8_t*>(w), y, bias, \
-                                   bias, nullptr, nullptr, nullptr, nullptr, status, M, N, K, ldx, ldy, flags, TN,    \
-                                   stages, tile);                                                                     \
-  }
-AGI_TC_GROUP_CLUSTER_KERNEL(agi_gemm_tc_bf16_x3_c2, 2)
-AGI_TC_GROUP_CLUSTER_KERNEL(agi_gemm_tc_bf16_x3_c4, 4)
-AGI_TC_GROUP_CLUSTER_KERNEL(agi_gemm_tc_bf16_x3_c8, 8)
-#undef AGI_TC_GROUP_CLUSTER_KERNEL
-
-// Single GEMM over packed operands, split-K slabs as in agi_gemm_tc_*.
-#define AGI_TC_PACKED_KERNEL(NAME, TYPE, FP8)                                                                         \
-  extern "C" __global__ void __launch_bounds__(tc::kThreads, 1)                                                      \
-  NAME(const TYPE* x, const TYPE* w, void* y, const bf16* bias, const bf16* residual, const float* scale_a,          \
-       const float* scale_w, float* partial, unsigned* counters, unsigned* status, unsigned M, unsigned N,           \
-       unsigned K, unsigned ldx, unsigned ldy, unsigned flags, unsigned TN, unsigned stages) {                       \
-    tc::gemm_body<FP8, 1, true>(reinterpret_cast<const uint8_t*>(x), reinterpret_cast<const uint8_t*>(w), y, bias,    \
-                                residual, scale_a, scale_w, partial, counters, status, M, N, K, ldx, ldy, flags, TN,  \
-                                stages);                                                                              \
-  }
-AGI_TC_PACKED_KERNEL(agi_gemm_tcp_e4m3, uint8_t, true)
-#undef AGI_TC_PACKED_KERNEL
 
 extern "C" __global__ void __launch_bounds__(tc::kThreads, 1)
 agi_gemm_tc_bf16(const bf16* x, const bf16* w, void* y, const bf16* bias, const bf16* residual, const float* scale_a,

@@ -75,47 +75,51 @@ __device__ __forceinline__ void persistent_body(const uint8_t* x, const uint8_t*
   grid_dependency_wait();
 
   if (warp == 0) {
-    // ---------------- producer ----------------
-    unsigned g = 0;                                          // ring position, running across tiles
-    for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-      const unsigned n0 = (tile % n_tiles) * kTileN, m0 = (tile / n_tiles) * TN;
-      for (unsigned kb = 0; kb < nkb; ++kb, ++g) {
-        const unsigned s = g % stages, round = g / stages;
-        wait_or_give_up(&empty_bar[s], (round & 1) ^ 1, status, kTimeoutEmpty | s, &gave_up);
-        if (lane == 0) {
+    // ---------------- producer: one elected lane ----------------
+    if (elect_one()) {
+      unsigned s = 0, phase = 1, dst = ring;                 // ring position, running across tiles
+      const size_t w_block = size_t(w_rows_padded) * kRowBytes, x_block = size_t(ldx) * kRowBytes;
+      for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint8_t* w_src = w + size_t((tile % n_tiles) * kTileN) * kRowBytes;
+        const uint8_t* x_src = x + size_t((tile / n_tiles) * TN) * kRowBytes;
+        for (unsigned kb = 0; kb < nkb; ++kb) {
+          wait_or_give_up(&empty_bar[s], phase, status, kTimeoutEmpty | s, &gave_up);
           expect_bytes(&full_bar[s], stage_bytes);
-          bulk_copy(ring + s * stage_bytes, w + (size_t(kb) * w_rows_padded + n0) * kRowBytes, kATileBytes, &full_bar[s]);
-          bulk_copy(ring + s * stage_bytes + kATileBytes, x + (size_t(kb) * ldx + m0) * kRowBytes, TN * kRowBytes,
-                    &full_bar[s]);
+          bulk_copy(dst, w_src, kATileBytes, &full_bar[s]);
+          bulk_copy(dst + kATileBytes, x_src, TN * kRowBytes, &full_bar[s]);
+          w_src += w_block;
+          x_src += x_block;
+          dst += stage_bytes;
+          if (++s == stages) { s = 0; phase ^= 1; dst = ring; }
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    const unsigned idesc = instr_descriptor<true>(TN);
-    unsigned g = 0, it = 0;
-    for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
-      const unsigned buf = it & 1, use = it >> 1;
-      wait_or_give_up(&acc_empty[buf], (use & 1) ^ 1, status, kTimeoutAccum | 0x10 | buf, &gave_up);
-      tc_fence_after();
-      const unsigned acc = tmem_base + buf * acc_columns;
-      for (unsigned kb = 0; kb < nkb; ++kb, ++g) {
-        const unsigned s = g % stages, round = g / stages;
-        wait_or_give_up(&full_bar[s], round & 1, status, kTimeoutFull | s, &gave_up);
+    // ---------------- MMA issuer: one elected lane ----------------
+    if (elect_one()) {
+      const unsigned idesc = instr_descriptor<true>(TN);
+      const unsigned long long first = smem_descriptor(ring), to_b = kATileBytes >> 4, to_next = stage_bytes >> 4;
+      unsigned s = 0, phase = 0, it = 0;
+      unsigned long long a_desc = first;
+      for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+        const unsigned buf = it & 1, use = it >> 1;
+        wait_or_give_up(&acc_empty[buf], (use & 1) ^ 1, status, kTimeoutAccum | 0x10 | buf, &gave_up);
         tc_fence_after();
-        if (lane == 0) {
-          const unsigned a_base = ring + s * stage_bytes, b_base = a_base + kATileBytes;
-          const unsigned long long a_desc = smem_descriptor(a_base), b_desc = smem_descriptor(b_base);
+        const unsigned acc = tmem_base + buf * acc_columns;
+        for (unsigned kb = 0; kb < nkb; ++kb) {
+          wait_or_give_up(&full_bar[s], phase, status, kTimeoutFull | s, &gave_up);
+          tc_fence_after();
 #pragma unroll
-          for (unsigned k = 0; k < 4; ++k) mma<true>(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
+          for (unsigned k = 0; k < 4; ++k) mma<true>(acc, a_desc + 2 * k, a_desc + to_b + 2 * k, idesc, (kb | k) != 0);
           tc_commit(&empty_bar[s]);
+          a_desc += to_next;
+          if (++s == stages) { s = 0; phase ^= 1; a_desc = first; }
         }
-        __syncwarp();
+        tc_commit(&acc_full[buf]);
       }
-      if (lane == 0) tc_commit(&acc_full[buf]);
-      __syncwarp();
     }
+    __syncwarp();
   } else {
     // ---------------- epilogue warps 2-5: TMEM lane quarter = warp % 4 ----------------
     const unsigned quarter = warp & 3;

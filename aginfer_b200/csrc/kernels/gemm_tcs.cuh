@@ -140,19 +140,18 @@ __device__ __forceinline__ void body(const bf16* x, const Parts& parts, bf16* y,
     // ---------------- MMA warp ----------------
     const unsigned idesc = tc::instr_descriptor<false>(kTokens);
     tc::mbar_wait(&tokens_bar, 0, status, kTimeoutTokens);
-    for (unsigned i = 0; i < nkb; ++i) {
-      tc::mbar_wait(&weights_bar[i], 0, status, kTimeoutWeights | i);
-      tc::tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {
+      for (unsigned i = 0; i < nkb; ++i) {
+        tc::mbar_wait(&weights_bar[i], 0, status, kTimeoutWeights | i);
+        tc::tc_fence_after();
         const unsigned long long a_desc = tc::smem_descriptor(ring + i * kATile);
         const unsigned long long b_desc = tc::smem_descriptor(tokens_base + i * kBTile);
 #pragma unroll
         for (unsigned k = 0; k < 4; ++k)   // the four 16-element steps of a K block go to four accumulators
           tc::mma<false>(tmem_base + kTokens * k, a_desc + 2 * k, b_desc + 2 * k, idesc, i != 0);
       }
-      __syncwarp();
+      tc::tc_commit(&accum_bar);
     }
-    if (lane == 0) tc::tc_commit(&accum_bar);
     __syncwarp();
     if (kCluster > 1) tc::cluster_wait();
   }

@@ -15,6 +15,7 @@ use is recorded for ``tactics.json``.
 """
 from __future__ import annotations
 
+import functools
 import math
 from dataclasses import dataclass, field
 from typing import Any, Mapping, Sequence
@@ -29,6 +30,7 @@ SM_COUNT = 148
 
 FLAG_BIAS, FLAG_RESIDUAL, FLAG_OUT_F32, FLAG_SCALED = 1, 2, 1 << 8, 1 << 9
 FLAG_LAYERNORM, FLAG_LN_MODULATE, FLAG_SLAB = 1 << 10, 1 << 11, 1 << 12
+FLAG_SWIGLU, FLAG_MUL_SILU, FLAG_AMAX = 1 << 13, 1 << 14, 1 << 15
 ACT = {None: 0, "gelu_tanh": 1 << 4, "silu": 2 << 4, "relu": 3 << 4}
 PLAN_DTYPE_BYTES = {"F32": 4, "F16": 2, "BF16": 2, "F8_E4M3": 1, "I32": 4}
 
@@ -109,73 +111,134 @@ def tc_tiling(M: int, N: int, K: int, elem: int, splits: int | None = None) -> d
             "shared_bytes": stages * stage_bytes + 1024}
 
 
-def tc_prefill_plan(M: int, N: int, K: int, elem: int) -> dict[str, int]:
-    """Tile shape for a tensor-core GEMM over many tokens: weight rows per CTA (128, or 256 = the wide kernel
-    with two accumulators), token tile TN, K slices.
+# ---- tensor-core GEMM with tokens as the MMA's A operand (csrc/kernels/gemm_tk.cuh) ------------------------
+TK_SMEM_BUDGET = 226 * 1024
+TK_PAIR_BUDGET = 112 * 1024                       # shared memory of a CTA that shares its SM with another
+# CTAs in whole clusters that the GPCs hold, one CTA per SM
+TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 138, 4: 132, 5: 120, 6: 126, 8: 120}
+TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3, 4, 5, 6, 8), "agi_gemm_tc_e4m3_x3": (1,),
+               "agi_gemm_tcpk_e4m3": (1, 2, 3, 4, 6, 8), "agi_gemm_tc_bf16_x3": (1, 2, 4, 8)}
+TK_MAX_RING = 8
 
-    The kernels fill shared memory from L2 with 16-byte asynchronous copies, measured at about 32 bytes per
-    clock and SM, which is slower than the tensor core consumes it; so the estimate per CTA is
-    K blocks x max(fill, MMA) + set-up + epilogue, times the number of waves over 148 SMs, plus the
-    slab pass of the finishing CTA when K is sliced.  The cheapest candidate wins."""
+
+def _run_estimate(rows: int, tn: int, n_tiles: int, m_tiles: int, k_blocks: int, runs: int) -> float:
+    per = ceil_div(k_blocks, runs)
+    cost = ceil_div(n_tiles * m_tiles * runs, SM_COUNT) * (per * max((rows + tn) * 128 / 28, rows // 128 * tn * 2) + 5000 + tn * 25)
+    return cost + (4000 + rows * tn * (runs + 1) // 8 if runs > 1 else 0)
+
+
+@functools.lru_cache(maxsize=4096)
+def k_runs(M: int, N: int, K: int, elem: int, packed: bool = False) -> int:
+    """Into how many runs K is cut when a product of this shape is summed (each run by the tensor core in fp32, then the
+    runs in order).  Part of a recipe's numerics, a function of the shape alone: FP8 block stacks turn one flipped
+    rounding into another quantisation of a whole tensor, so tiles and clusters may change with the hardware's costs, the
+    order of the sum may not.  More runs where a product has few output tiles for its K."""
     k_blocks = K * elem // 128
-    best: dict[str, int] | None = None
+    if M <= 64 and not packed:
+        c = tc_cluster_tiling(M, N, K, elem, "e4m3" if elem == 1 else "bf16")
+        return c["cluster"] if c is not None else 1
+    if M < 128 and not packed:
+        runs = tc_tiling(M, N, K, elem)["splits"]
+        while runs > 1 and runs * M * ceil_div(N, 128) * 512 > TC_SCRATCH_BYTES:
+            runs = tc_tiling(M, N, K, elem, runs // 2)["splits"]
+        return runs
+    best: tuple[float, int] | None = None
     for rows in (128, 256):
         if rows == 256 and N < 256:
             continue
-        n_tiles = ceil_div(N, rows)
-        seen = set()
+        n_tiles, seen = ceil_div(N, rows), set()
         for cap in range(256, 48, -16):
             m_tiles = ceil_div(M, cap)
-            TN = ceil_div(ceil_div(M, m_tiles), 16) * 16
-            if TN in seen:
+            tn = ceil_div(ceil_div(M, m_tiles), 16) * 16
+            if tn in seen:
                 continue
-            seen.add(TN)
-            for splits in (1, 2, 3, 4, 6, 8):
-                per = ceil_div(k_blocks, splits)
-                if ceil_div(k_blocks, per) != splits or (splits > 1 and per < 4):
-                    continue
-                if splits > 1 and splits * M * n_tiles * rows * 4 > TC_SCRATCH_BYTES:
+            seen.add(tn)
+            for runs in (1, 2, 3, 4, 6, 8):
+                per = ceil_div(k_blocks, runs)
+                if ceil_div(k_blocks, per) != runs or (runs > 1 and (per < 4 or runs * M * n_tiles * rows * 4 > TC_SCRATCH_BYTES)):
                     continue
                 if n_tiles * m_tiles * 4 > TC_COUNTER_BYTES:
                     continue
-                stage_bytes = rows * 128 + TN * 128
-                fill = stage_bytes / 28
-                mma = (rows // 128) * TN * 2
-                ctas = n_tiles * m_tiles * splits
-                cost = ceil_div(ctas, SM_COUNT) * (per * max(fill, mma) + 5000 + TN * 25)
-                if splits > 1:      # slab stores of every slice, then one CTA per tile reads them all back
-                    cost += 4000 + rows * TN * (splits + 1) // 8
-                if best is None or cost < best["cost"]:
-                    stages = max(3, min(12, TC_SMEM_BUDGET // stage_bytes, max(per, 3)))
-                    best = {"rows": rows, "TN": TN, "m_tiles": m_tiles, "n_tiles": n_tiles, "splits": splits,
-                            "stages": stages, "shared_bytes": stages * stage_bytes + 1024, "cost": int(cost)}
+                cost = _run_estimate(rows, tn, n_tiles, m_tiles, k_blocks, runs)
+                if best is None or cost < best[0]:
+                    best = (cost, runs)
     assert best is not None
-    return best
+    runs = best[1]
+    if packed and runs > 1:
+        # one run while K is short, or where enough tokens fill the SMs without cutting it
+        tiles, least = 0, None
+        for mt in range(ceil_div(M, 256), ceil_div(M, 256) + PERSIST_TOKEN_SPLITS):
+            tn = ceil_div(ceil_div(M, mt), 16) * 16
+            cost = ceil_div(ceil_div(N, 128) * mt, SM_COUNT) * max((16384 + tn * 128) / 40, 2 * tn)
+            if tn >= 16 and (least is None or cost < least):
+                least, tiles = cost, ceil_div(N, 128) * mt
+        if tiles >= 2 * SM_COUNT or k_blocks <= 48 or M >= 768:
+            return 1
+    return runs
 
 
-def tc_group_tiling(M: int, n_tiles: int, K: int, elem: int) -> dict[str, int]:
-    """Token tile and ring depth of the grouped tensor-core GEMM (128-row tiles, no K slices): the token tile
-    with the cheapest estimate under the same model as ``tc_prefill_plan``."""
+@functools.lru_cache(maxsize=4096)
+def tk_tiling(M: int, widths: tuple[int, ...], K: int, elem: int, swiglu: bool = False, runs: int | None = None,
+              clusters: tuple[int, ...] = (1, 2, 4, 8), rows_per_tile: int | None = None) -> Mapping[str, int]:
+    """Tile of ``agi_gemm_tk_*`` for matrices of ``widths`` rows side by side over M tokens: weight rows ``NB``,
+    token group ``tg``, cluster size ``C``, ring depth.  ``runs``: see ``k_runs``; None = one run per cluster rank,
+    whatever cluster is chosen.  ``rows_per_tile`` fixes NB.
+
+    Every CTA takes in NB weight rows and its tokens, and that intake sets the time, so the estimate per CTA is
+    K blocks x max(intake at 57 B per clock, 650 cycles: what one SM's outstanding loads give) + set-up, epilogue and
+    exchange between ranks, times the rounds over the SMs.  Half-size rings put two CTAs on an SM, whose set-up and
+    epilogue then overlap.  The constants are fitted to 30 000 timed tiles of 70 shapes (36 - 1024 tokens): the tile
+    chosen is 3.5 % slower than the fastest one on average, 28 % at worst."""
     k_blocks = K * elem // 128
     best: dict[str, int] | None = None
-    for cap in range(256, 15, -16):
-        m_tiles = ceil_div(M, cap)
-        TN = ceil_div(ceil_div(M, m_tiles), 16) * 16
-        stage_bytes = 16384 + TN * 128
-        cost = ceil_div(n_tiles * m_tiles, SM_COUNT) * (k_blocks * max(stage_bytes / 28, TN * 2) + 5000 + TN * 25)
-        if best is None or cost < best["cost"]:
-            stages = max(3, min(12, TC_SMEM_BUDGET // stage_bytes, max(k_blocks, 3)))
-            best = {"TN": TN, "m_tiles": m_tiles, "stages": stages, "shared_bytes": stages * stage_bytes + 1024,
-                    "cost": int(cost)}
-    assert best is not None
+    for budget, per_sm in ((TK_SMEM_BUDGET, 1), (TK_PAIR_BUDGET, 2)):
+        for C in clusters:
+            S = runs or C
+            per_run = ceil_div(k_blocks, S)
+            if C > S or ceil_div(k_blocks, per_run) != S or (runs is None and C > 1 and k_blocks < 2 * C):
+                continue
+            held_runs = ceil_div(S, C)             # runs of the busiest rank
+            nkb = min(k_blocks, held_runs * per_run)
+            for NB in ((rows_per_tile,) if rows_per_tile else range(32 if swiglu else 16, 257, 32 if swiglu else 16)):
+                out = NB // 2 if swiglu else NB
+                tiles = sum(ceil_div(n, out) for n in widths)
+                seen = set()
+                for groups in range(1, 17):
+                    tg = ceil_div(ceil_div(M, groups), 8) * 8
+                    if tg in seen or tg > 512 or (tg < 16 and M > 16):
+                        continue
+                    seen.add(tg)
+                    groups = ceil_div(M, tg)
+                    m_tiles = ceil_div(tg, 128)
+                    if held_runs * m_tiles * ceil_div(NB, 32) * 32 > (512 if per_sm == 1 else 256):   # tensor-memory columns
+                        continue
+                    stage = (tg + NB) * 128
+                    overhang = max(0, m_tiles * 16384 - stage)
+                    stages = min(TK_MAX_RING, (budget - 1024 - overhang) // stage, max(2, nkb))
+                    if stages < 2:
+                        continue
+                    rows = min(tg, 128) if C == 1 else ceil_div(tg, 8 * C) * 8
+                    shared = 1024 + max(stages * stage + overhang, rows * (NB + 4) * 4)
+                    if shared > budget or (C > 1 and tiles * groups * S * NB * ceil_div(tg, 32) * 128 > TC_SCRATCH_BYTES):
+                        continue
+                    ctas, held = tiles * groups * C, min(tg, M)
+                    block = max(stage / 57.5, 650 * m_tiles, 4 * m_tiles * NB / 2)
+                    lone = max(block, 1800 / (stages - 1))
+                    over = 2700 + 0.163 * held * NB * (0.7 if swiglu else 1.0)
+                    over += (3000 + 0.083 * held * NB * S / C if C > 1 else 0.02 * held * NB * (S - 1))
+                    rounds = ceil_div(ctas, TK_RESIDENT[C])
+                    if per_sm == 1:
+                        cost = rounds * (nkb * lone + over)
+                    else:
+                        cost = max(rounds * nkb * block, ceil_div(rounds, 2) * nkb * lone) + over * (1 + 0.25 * (rounds - 1))
+                    if best is None or cost < best["cost"]:
+                        best = {"C": C, "NB": NB, "tg": tg, "tiles": tiles, "groups": groups, "stages": stages, "runs": S,
+                                "per_run": per_run, "shared_bytes": shared, "cost": int(cost)}
+    assert best is not None, "no tile of the tensor-core GEMM fits"
     return best
 
 
-# K >= ratio * N counts as K-heavy; 0 (default) disables the rule: in isolation the cluster kernel wins there
-# (17 tokens, 1536 x 6144: 9.4 us against 11.3 us), inside the action-head graph it does not (2.96 ms per chunk
-# against 2.93 ms), because the weight-streaming kernel starts its copies before the previous kernel has finished
-CLUSTER_K_RATIO = 0
-PERSIST_TOKEN_SPLITS = 4             # token-tile counts the persistent GEMM's planner tries beyond the minimum
+PERSIST_TOKEN_SPLITS = 4             # token-tile counts tried beyond the minimum for the persistent GEMM
 FA_HEAD_DIMS = (48, 64, 80, 128)   # compiled widths of agi_attention_fa_bf16_d*
 
 
@@ -594,8 +657,9 @@ class RecipeBuilder:
              bias: Pointer | None = None, residual: Pointer | None = None, act: str | None = None,
              scale_a: Pointer | None = None, scale_w: Pointer | None = None, ldx: int | None = None,
              ldy: int | None = None, out_f32: bool = False, tactic: str = "auto",
-             splits: int | None = None, packed: bool = False) -> None:
+             splits: int | None = None, packed: bool = False, fixed_order: bool = False) -> None:
         """Y[M, N] = epilogue(X[M, K] . W[N, K]^T); ``dtype`` names the operand type (bf16 or e4m3).
+        ``fixed_order``: K is summed as ``k_runs`` says (always so for E4M3), for a bf16 product that feeds an FP8 stack.
         ``packed`` (E4M3 only): both operands are in the packed layout of ``recipes/layout.py`` (weights packed
         at packaging time, activations by ``quantize_e4m3(..., packed=)``) and ring slots are filled by bulk copies."""
         if dtype == "bf16" and self.is_packed(w):
@@ -604,14 +668,15 @@ class RecipeBuilder:
             return
         if packed:
             assert dtype == "e4m3" and K % 128 == 0 and ldx is None
-            t = tc_prefill_plan(M, N, K, 1)
             flags = ACT[act] | (FLAG_BIAS if bias else 0) | (FLAG_RESIDUAL if residual else 0) | \
                 (FLAG_OUT_F32 if out_f32 else 0) | (FLAG_SCALED if scale_a else 0)
             dummy = Arena(0)
-            # more 128 x TN output tiles than SMs: the persistent kernel (one CTA per SM walks the tiles, two
-            # accumulators in tensor memory, epilogue of one tile under the multiplication of the next)
-            # token tile: the split of M whose tile count divides best over the SMs (rounds x bytes per tile;
-            # measured: a K block of 16 KB + TN * 128 B takes ~1 cycle per 40 bytes, the MMA 2 * TN cycles)
+            runs = k_runs(M, N, K, 1, packed=True)
+            t = tk_tiling(M, (N,), K, 1, runs=runs, clusters=TK_CLUSTERS["agi_gemm_tcpk_e4m3"])
+            # the persistent kernel (one CTA per SM walks 128 x TN tiles, two accumulators in tensor memory, the epilogue
+            # of one tile under the multiplication of the next) where its estimate is the lower one: many more tiles than
+            # SMs, so that the overlapped epilogue outweighs its smaller tiles.
+            # Token tile: the split of M whose tile count divides best over the SMs.
             m_tiles, TN, tiles = 0, 0, 0
             best_cost = None
             for mt in range(ceil_div(M, 256), ceil_div(M, 256) + PERSIST_TOKEN_SPLITS):
@@ -619,14 +684,10 @@ class RecipeBuilder:
                 if tn < 16:
                     break
                 count = ceil_div(N, 128) * mt
-                cost = ceil_div(count, SM_COUNT) * max((16384 + tn * 128) / 40, 2 * tn)
+                cost = ceil_div(count, SM_COUNT) * (K // 128) * max((16384 + tn * 128) / 46, 2 * tn, 400) + 5000 + tn * 25
                 if best_cost is None or cost < best_cost:
                     best_cost, m_tiles, TN, tiles = cost, mt, tn, count
-            # also preferred over K slices while K is short (1280 x 3456, 512 tokens: 13.6 us against 18.6 us with two
-            # slices); with 86 or more K blocks per tile the slices win (2048 x 11008, 288 tokens: 24.8 us against 32.5 us)
-            # ... unless there are enough tokens for the tile loop to cover the SMs by itself (1024 tokens: 35.8 us against 42.3 us)
-            short_k = t["splits"] > 1 and (K // 128 <= 48 or M >= 768)
-            if tactic in ("auto", "persistent") and (tiles >= 2 * SM_COUNT or short_k or tactic == "persistent"):
+            if tactic == "persistent" or (tactic == "auto" and runs == 1 and best_cost < t["cost"]):
                 stage_bytes = 16384 + TN * 128
                 stages = max(2, min(12, TC_SMEM_BUDGET // stage_bytes))
                 self.launch("agi_gemm_tcq_e4m3", (min(tiles, SM_COUNT), 1, 1), (192, 1, 1),
@@ -635,14 +696,8 @@ class RecipeBuilder:
                              U32(flags), U32(TN), U32(stages)], shared_bytes=stages * stage_bytes + 1024,
                             op="gemm_e4m3_packed", algorithm=f"tcgen05_persistent_128x{TN}_s{stages}")
                 return
-            partial, counters = self._tc_scratch
-            wide = t["rows"] == 256
-            self.launch("agi_gemm_tcp_wide_e4m3" if wide else "agi_gemm_tcp_e4m3", (t["n_tiles"], t["m_tiles"], t["splits"]),
-                        (288 if wide else 160, 1, 1),
-                        [x, w, y, bias or dummy, residual or dummy, scale_a or dummy, scale_w or dummy, partial, counters,
-                         Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(padded_token_rows(M)), U32(ldy or N), U32(flags),
-                         U32(t["TN"]), U32(t["stages"])], shared_bytes=t["shared_bytes"], op="gemm_e4m3_packed",
-                        algorithm=f"tcgen05_bulk_{t['rows']}x{t['TN']}_s{t['stages']}_k{t['splits']}")
+            self._gemm_tk("agi_gemm_tcpk_e4m3", "gemm_e4m3_packed", t, x, [(w, bias, scale_w, y, N, ldy or N)], M, K,
+                          padded_token_rows(M), flags, scale_a=scale_a, other=residual)
             return
         flags = ACT[act] | (FLAG_BIAS if bias else 0) | (FLAG_RESIDUAL if residual else 0) | \
             (FLAG_OUT_F32 if out_f32 else 0) | (FLAG_SCALED if scale_a else 0)
@@ -653,18 +708,16 @@ class RecipeBuilder:
         elem = 1 if dtype == "e4m3" else 2
         aligned = ((ldx or K) * elem) % 16 == 0
         if tactic == "auto":
-            # <= 64 tokens: weight-streaming kernel (whole 64-byte K windows); otherwise the tensor-core
-            # kernel (whole 128-byte K blocks); anything else falls back to the CUDA-core kernel.
-            if M <= 64 and (K * elem) % 64 == 0 and aligned:
+            # <= 32 tokens: weight-streaming kernel (whole 64-byte K windows); otherwise the tensor-core kernel (whole
+            # 128-byte K blocks), for 33-64 tokens too, where the weight-streaming kernel needs 5-8 token tiles of
+            # accumulators per warp; anything else falls back to the CUDA-core kernel.
+            blocks = (K * elem) % 128 == 0 and aligned
+            if M <= 32 and (K * elem) % 64 == 0 and aligned:
                 tactic = "stream"
-                # 33-64 tokens: the weight-streaming kernel needs 5-8 token tiles of accumulators per warp and
-                # slows down (50 tokens, 4096 x 1024: 18.8 us), while the tensor-core kernel with its K slices in
-                # a thread-block cluster does not care about the token count (8.6 us)
-                k_heavy = CLUSTER_K_RATIO > 0 and K >= CLUSTER_K_RATIO * N
-                if (M > 32 or k_heavy) and tc_cluster_tiling(M, N, K, elem, dtype) is not None:
-                    tactic = "cluster"
-            elif (K * elem) % 128 == 0 and aligned:
-                tactic = "tcgen05_plan" if M >= 128 else "tcgen05"
+            elif blocks:
+                tactic = "tcgen05_plan"
+            elif M <= 64 and (K * elem) % 64 == 0 and aligned:
+                tactic = "stream"
             else:
                 tactic = "simt"
         if tactic == "stream":
@@ -701,42 +754,29 @@ class RecipeBuilder:
             self.launch(f"agi_gemm_simt_{dtype}", (ceil_div(N, 64), ceil_div(M, 64), 1), (256, 1, 1), args,
                         op=f"gemm_{dtype}", algorithm="simt_64x64x16")
             return
-        if tactic == "cluster":
-            # tcgen05 with the K slices of a tile forming a thread-block cluster; partial sums meet in
-            # distributed shared memory (no global scratch, no atomics)
-            t = tc_cluster_tiling(M, N, K, elem, dtype)
-            if t is None:
-                raise ValueError("cluster split-K needs M <= 64, whole 128-byte K blocks and a usable cluster size")
-            self.launch(f"agi_gemm_tc_{dtype}_c{t['cluster']}", (t["n_tiles"], 1, t["cluster"]), (160, 1, 1),
-                        args[:7] + [dummy, dummy, Arena(STATUS_WORD)] + args[7:] + [U32(t["TN"]), U32(t["stages"])],
-                        shared_bytes=t["shared_bytes"], op=f"gemm_{dtype}",
-                        algorithm=f"tcgen05_128x{t['TN']}_s{t['stages']}_cluster{t['cluster']}")
-            return
-        if tactic not in ("tcgen05", "tcgen05_wide", "tcgen05_plan"):
+        if tactic not in ("tcgen05", "tcgen05_wide", "tcgen05_plan", "cluster"):
             raise ValueError(f"unknown GEMM tactic {tactic!r}")
         if (K * elem) % 128 or ((ldx or K) * elem) % 16:
             raise ValueError("tcgen05 GEMM needs K bytes % 128 == 0 and 16-byte aligned rows")
-        partial, counters = self._tc_scratch
-        tc_args = args[:7] + [partial, counters, Arena(STATUS_WORD)] + args[7:]
-        if tactic in ("tcgen05_wide", "tcgen05_plan"):
-            if tactic == "tcgen05_plan":
-                t = tc_prefill_plan(M, N, K, elem)
-            else:   # explicit: 256 rows, the largest token tile, K sliced only on request
-                m_tiles = ceil_div(M, 256)
-                TN = ceil_div(ceil_div(M, m_tiles), 16) * 16
-                k_blocks = K * elem // 128
-                per = ceil_div(k_blocks, max(1, min(splits or 1, 8, k_blocks)))
-                stage_bytes = 32768 + TN * 128
-                stages = max(3, min(12, TC_SMEM_BUDGET // stage_bytes, max(per, 3)))
-                t = {"rows": 256, "TN": TN, "m_tiles": m_tiles, "n_tiles": ceil_div(N, 256),
-                     "splits": ceil_div(k_blocks, per), "stages": stages, "shared_bytes": stages * stage_bytes + 1024}
-                assert t["splits"] == 1 or t["splits"] * M * t["n_tiles"] * 256 * 4 <= TC_SCRATCH_BYTES
-            wide = t["rows"] == 256
-            self.launch(f"agi_gemm_tc_wide_{dtype}" if wide else f"agi_gemm_tc_{dtype}",
-                        (t["n_tiles"], t["m_tiles"], t["splits"]), (288 if wide else 160, 1, 1),
-                        tc_args + [U32(t["TN"]), U32(t["stages"])], shared_bytes=t["shared_bytes"], op=f"gemm_{dtype}",
-                        algorithm=f"tcgen05_{t['rows']}x{t['TN']}_s{t['stages']}_k{t['splits']}")
+        if tactic != "tcgen05":
+            # tcgen05_plan: the planner's tile; cluster: K slices in a cluster as `tc_cluster_tiling` asks for;
+            # tcgen05_wide: 256-row tiles with the K slices asked for
+            if tactic == "cluster":
+                c = tc_cluster_tiling(M, N, K, elem, dtype)
+                if c is None:
+                    raise ValueError("cluster split-K needs M <= 64, whole 128-byte K blocks and a usable cluster size")
+                t = tk_tiling(M, (N,), K, elem, clusters=(max(n for n in (2, 4, 8) if n <= c["cluster"]),))
+            elif tactic == "tcgen05_wide":
+                slices = max(n for n in (1, 2, 4, 8) if n == 1 or (n <= (splits or 1) and K * elem // 128 >= 2 * n))
+                t = tk_tiling(M, (N,), K, elem, clusters=(slices,), rows_per_tile=256)
+            else:
+                runs = k_runs(M, N, K, elem) if fixed_order or dtype == "e4m3" else None
+                clusters = TK_CLUSTERS[f"agi_gemm_tk_{dtype}"] if runs else (1, 2, 4, 8)
+                t = tk_tiling(M, (N,), K, elem, runs=runs, clusters=clusters)
+            self._gemm_tk(f"agi_gemm_tk_{dtype}", f"gemm_{dtype}", t, x, [(w, bias, scale_w, y, N, ldy or N)], M, K, ldx or K,
+                          flags, scale_a=scale_a, other=residual)
             return
+        partial, counters = self._tc_scratch
         t = tc_tiling(M, N, K, elem, splits)
         while t["splits"] > 1 and t["splits"] * M * t["n_tiles"] * 128 * 4 > TC_SCRATCH_BYTES:
             t = tc_tiling(M, N, K, elem, t["splits"] // 2)
@@ -745,6 +785,23 @@ class RecipeBuilder:
                     args[:7] + [partial, counters, Arena(STATUS_WORD)] + args[7:] + [U32(t["TN"]), U32(t["stages"])],
                     shared_bytes=t["shared_bytes"], op=f"gemm_{dtype}",
                     algorithm=f"tcgen05_128x{t['TN']}_s{t['stages']}_k{t['splits']}")
+
+    def _gemm_tk(self, family: str, op: str, t: Mapping[str, int], x: Pointer,
+                 parts: Sequence[tuple[Pointer, Pointer | None, Pointer | None, Pointer, int, int]], M: int, K: int, ldx: int,
+                 flags: int, *, scale_a: Pointer | None = None, other: Pointer | None = None,
+                 amax: Pointer | None = None) -> None:
+        """One launch of ``agi_gemm_tk_*`` (or a family with the same parameters) with the tile ``t``.
+        ``parts``: (weight, bias, weight scale, y, N, ldy); ``other``: residual, or the gate of FLAG_MUL_SILU."""
+        dummy = Arena(0)
+        args: list[Any] = [x, scale_a or dummy, other or dummy, self._tc_scratch[0], amax or dummy, Arena(STATUS_WORD), U32(M),
+                           U32(K), U32(ldx), U32(flags | (FLAG_AMAX if amax is not None else 0)), U32(t["NB"]),
+                           U32(t["stages"]), U32(t["tg"]), U32(t["runs"]), U32(t["per_run"])]
+        for i in range(3):
+            w, bias, scale, y, N, ldy = parts[i] if i < len(parts) else (dummy, None, None, dummy, 0, 0)
+            args += [w, bias or dummy, scale or dummy, y, U32(N), U32(ldy)]
+        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (t["tiles"], t["groups"], t["C"]), (288, 1, 1), args,
+                    shared_bytes=t["shared_bytes"], op=op,
+                    algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_r{t['runs']}_c{t['C']}" + (f"_x{len(parts)}" if len(parts) > 1 else ""))
 
     def gemm_group(self, x: Pointer, parts: Sequence[tuple[Pointer, Pointer | None, Pointer | None, Pointer, int, int]],
                    M: int, K: int, *, dtype: str = "bf16", scale_a: Pointer | None = None, ldx: int | None = None,
@@ -760,45 +817,32 @@ class RecipeBuilder:
         assert all((p[1] is not None) == has_bias for p in parts)
         assert all((p[2] is not None) == (scale_a is not None) for p in parts)
         flags = ACT[act] | (FLAG_BIAS if has_bias else 0) | (FLAG_SCALED if scale_a else 0)
-        t = tc_group_tiling(M, sum(ceil_div(p[4], 128) for p in parts), K, elem)
-        dummy = Arena(0)
         assert not packed or (dtype == "e4m3" and ldx is None)
-        args: list[Any] = [x, scale_a or dummy, Arena(STATUS_WORD), U32(M), U32(K),
-                           U32(padded_token_rows(M) if packed else (ldx or K)), U32(flags), U32(t["TN"]), U32(t["stages"])]
-        for i in range(3):
-            if i < len(parts):
-                w, bias, sw, y, N, ldy = parts[i]
-                args += [w, bias or dummy, sw or dummy, y, U32(N), U32(ldy)]
-            else:
-                args += [dummy, dummy, dummy, dummy, U32(0), U32(0)]
-        grid_x = sum(ceil_div(p[4], 128) for p in parts)
-        if dtype == "bf16" and not packed and M <= 64:
-            # few tokens: too few tiles to fill the SMs, so the K slices of every tile form a cluster (as `cluster`
-            # does for one matrix) and the projections that share the activations still share the launch
-            c = tc_cluster_tiling(M, 128 * grid_x, K, elem, dtype, sizes=(2, 4, 8))
-            if c is not None:
-                args[7:9] = [U32(c["TN"]), U32(c["stages"])]
-                self.launch(f"agi_gemm_tc_bf16_x3_c{c['cluster']}", (grid_x, 1, c["cluster"]), (160, 1, 1), args,
-                            shared_bytes=c["shared_bytes"], op="gemm_bf16_group",
-                            algorithm=f"tcgen05_128x{c['TN']}_s{c['stages']}_cluster{c['cluster']}_x{len(parts)}")
-                return
-        self.launch(f"agi_gemm_tcp_{dtype}_x3" if packed else f"agi_gemm_tc_{dtype}_x3", (grid_x, t["m_tiles"], 1),
-                    (160, 1, 1), args, shared_bytes=t["shared_bytes"], op=f"gemm_{dtype}_group" + ("_packed" if packed else ""),
-                    algorithm=f"tcgen05_{'bulk_' if packed else ''}128x{t['TN']}_s{t['stages']}_x{len(parts)}")
+        widths = tuple(p[4] for p in parts)
+        family = "agi_gemm_tcpk_e4m3" if packed else f"agi_gemm_tc_{dtype}_x3"
+        c = tc_cluster_tiling(M, 128 * sum(ceil_div(n, 128) for n in widths), K, elem, dtype, sizes=(2, 4, 8))
+        if dtype == "bf16" and M <= 64 and c is not None:
+            # few tokens: 128-row tiles would leave most SMs idle, so the K slices of every tile form a cluster
+            t = tk_tiling(M, widths, K, elem, clusters=(c["cluster"],), rows_per_tile=128)
+        else:
+            t = tk_tiling(M, widths, K, elem, clusters=(1,))
+        self._gemm_tk(family, f"gemm_{dtype}_group" + ("_packed" if packed else ""), t, x,
+                      [(w, bias, sw, y, N, ldy) for w, bias, sw, y, N, ldy in parts], M, K,
+                      padded_token_rows(M) if packed else (ldx or K), flags, scale_a=scale_a)
 
     def gemm_batch(self, x: Pointer, parts: Sequence[tuple[Pointer, Pointer]], y: Pointer, M: int, N: int, K: int,
                    seg_stride: int, ldx: int | None = None) -> None:
         """Up to 16 bf16 GEMMs ``y[s] = x . W_s^T + b_s`` over the same ``x`` in one tensor-core launch;
         ``y[s]`` starts ``seg_stride`` elements after ``y[s - 1]``."""
         assert 1 <= len(parts) <= 16 and (K * 2) % 128 == 0
-        t = tc_tiling(M, N, K, 2, 1)
+        t = tk_tiling(M, (N,) * len(parts), K, 2, clusters=(1,))
         dummy = Arena(0)
         ws = [p[0] for p in parts] + [dummy] * (16 - len(parts))
         bs = [p[1] for p in parts] + [dummy] * (16 - len(parts))
-        self.launch("agi_gemm_tc_bf16_x16", (len(parts) * t["n_tiles"], t["m_tiles"], 1), (160, 1, 1),
-                    [x, y, Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(ldx or K), U32(N), U32(FLAG_BIAS), U32(t["TN"]),
-                     U32(t["stages"]), U32(seg_stride), *ws, *bs], shared_bytes=t["shared_bytes"], op="gemm_bf16_batch",
-                    algorithm=f"tcgen05_128x{t['TN']}_s{t['stages']}_x{len(parts)}")
+        self.launch("agi_gemm_tc_bf16_x16", (t["tiles"], t["groups"], 1), (288, 1, 1),
+                    [x, y, Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(ldx or K), U32(N), U32(FLAG_BIAS), U32(t["NB"]),
+                     U32(t["stages"]), U32(t["tg"]), U32(seg_stride), *ws, *bs], shared_bytes=t["shared_bytes"],
+                    op="gemm_bf16_batch", algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_x{len(parts)}")
 
     def is_packed(self, w: Pointer) -> bool:
         """True for a checkpoint matrix stored in the packed layout of ``recipes/layout.py`` ([K blocks, rows, 64])."""

@@ -307,7 +307,7 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
     r.launch("agi_patchify_f32_bf16", (grid_for(P * cfg.patch_k), 1, 1), (256, 1, 1),
              [Tensor("pixels"), patches, vpos, U32(cfg.images), U32(cfg.channels), U32(cfg.image_size), U32(cfg.patch),
               U32(cfg.temporal), U32(cfg.window), U32(cfg.merge), U32(cfg.patch_k), U32(cfg.patch_k)], op="patchify")
-    r.gemm(patches, Weight("visual.patch_embed.proj.weight"), x, P, VH, cfg.patch_k, tactic=gemm_tactic)
+    r.gemm(patches, Weight("visual.patch_embed.proj.weight"), x, P, VH, cfg.patch_k, tactic=gemm_tactic, fixed_order=True)
     snapshot(x, "vision_trace", 0, P * VH * BF)
     half = VD // 2
     for i in range(cfg.v_layers):
