@@ -22,6 +22,9 @@ struct CudaApi {
   Status Check(CUresult result, const std::string& what, Code code = kCudaError) const {
     return result == CUDA_SUCCESS ? Status() : Status(code, Explain(result, what));
   }
+  Status Check(CUresult result, const char* what, Code code = kCudaError) const {   // no string on the path that succeeds
+    return result == CUDA_SUCCESS ? Status() : Status(code, Explain(result, what));
+  }
 
 #define AGI_CUDA_FN(name) decltype(&::name) name = nullptr
   AGI_CUDA_FN(cuInit);

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <string_view>
 
 namespace agi {
 namespace {
@@ -120,6 +121,7 @@ Session::~Session() {
   for (auto& state : states_)
     for (CachedGraph& g : state->graphs)
       if (g.exec != nullptr) cu_->cuGraphExecDestroy(g.exec);
+  if (capture_stream_ != nullptr) cu_->cuStreamDestroy(capture_stream_);
   if (workspace_ != 0) cu_->cuMemFree(workspace_);
   if (arena_ != 0) cu_->cuMemFree(arena_);
   if (weights_ != 0) cu_->cuMemFree(weights_);
@@ -130,27 +132,27 @@ Session::~Session() {
 Status Session::Bind(const TensorArg* views, std::size_t count, std::uint32_t io_kind) {
   for (std::size_t v = 0; v < count; ++v) {
     const TensorArg& view = views[v];
-    const std::string name = view.name != nullptr ? view.name : "";
+    const std::string_view key = view.name != nullptr ? view.name : "";
     const wire::Tensor* want = nullptr;
     std::uint32_t slot = 0;
     for (std::uint32_t i = 0; i < profile_->tensor_count && want == nullptr; ++i) {
       const wire::Tensor& t = plan_.tensors[profile_->first_tensor + i];
-      if (t.io_kind == io_kind && plan_.Text(t.name) == name) {
+      if (t.io_kind == io_kind && plan_.Text(t.name) == key) {
         want = &t;
         slot = i;
       }
     }
-    if (want == nullptr) return Status(kInvalidArgument, "unexpected tensor for selected profile: " + name);
-    if (bound_[slot] != nullptr) return Status(kInvalidArgument, "duplicate TensorView: " + name);
+    if (want == nullptr) return Status(kInvalidArgument, "unexpected tensor for selected profile: " + std::string(key));
+    if (bound_[slot] != nullptr) return Status(kInvalidArgument, "duplicate TensorView: " + std::string(key));
     const std::uint32_t want_location = want->location == wire::kDevice ? kPubDevice : kPubHost;
     if (view.dtype != ToPublicDType(want->dtype) || view.location != want_location)
-      return Status(kInvalidArgument, "dtype or memory location mismatch for tensor: " + name);
+      return Status(kInvalidArgument, "dtype or memory location mismatch for tensor: " + std::string(key));
     if (view.data == nullptr || view.byte_size < want->byte_size || view.rank != want->rank ||
         (view.rank != 0 && (view.shape == nullptr || view.stride == nullptr)))
-      return Status(kInvalidArgument, "buffer, byte size, or rank mismatch for tensor: " + name);
+      return Status(kInvalidArgument, "buffer, byte size, or rank mismatch for tensor: " + std::string(key));
     for (std::uint32_t d = 0; d < want->rank; ++d)
       if (view.shape[d] != want->shape[d] || view.stride[d] != want->stride[d])
-        return Status(kInvalidArgument, "shape or stride is outside the selected profile: " + name);
+        return Status(kInvalidArgument, "shape or stride is outside the selected profile: " + std::string(key));
     bound_[slot] = view.data;
   }
   return {};
@@ -384,21 +386,31 @@ Status Session::Issue(CUstream stream) {
 }
 
 Status Session::Replay(CUstream stream) {
-  const bool graph_safe = (active_->profile->flags & 1u) != 0 && (flags_ & kNoGraphReplay) == 0 && stream != nullptr;
+  const bool graph_safe = (active_->profile->flags & 1u) != 0 && (flags_ & kNoGraphReplay) == 0;
   if (!graph_safe) return Issue(stream);
-  CUstreamCaptureStatus capturing = CU_STREAM_CAPTURE_STATUS_NONE;
-  if (cu_->cuStreamIsCapturing(stream, &capturing) != CUDA_SUCCESS || capturing != CU_STREAM_CAPTURE_STATUS_NONE)
-    return Issue(stream);  // the caller is building its own graph: contribute plain launches
+  if (stream != nullptr) {
+    CUstreamCaptureStatus capturing = CU_STREAM_CAPTURE_STATUS_NONE;
+    if (cu_->cuStreamIsCapturing(stream, &capturing) != CUDA_SUCCESS || capturing != CU_STREAM_CAPTURE_STATUS_NONE)
+      return Issue(stream);  // the caller is building its own graph: contribute plain launches
+  }
 
   CachedGraph* hit = nullptr;
   std::vector<CachedGraph>& graphs_ = active_->graphs;
   for (CachedGraph& g : graphs_)
     if (g.key == bound_) hit = &g;
   if (hit == nullptr) {
-    AGI_RETURN_IF_ERROR(cu_->Check(cu_->cuStreamBeginCapture(stream, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL), "cuStreamBeginCapture"));
-    const Status issued = Issue(stream);
+    // The legacy null stream cannot be captured (a graph can be launched into it): the launches are recorded on a
+    // stream of the session's own.
+    CUstream recorder = stream;
+    if (recorder == nullptr) {
+      if (capture_stream_ == nullptr)
+        AGI_RETURN_IF_ERROR(cu_->Check(cu_->cuStreamCreate(&capture_stream_, CU_STREAM_NON_BLOCKING), "cuStreamCreate"));
+      recorder = capture_stream_;
+    }
+    AGI_RETURN_IF_ERROR(cu_->Check(cu_->cuStreamBeginCapture(recorder, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL), "cuStreamBeginCapture"));
+    const Status issued = Issue(recorder);
     CUgraph graph = nullptr;
-    const CUresult ended = cu_->cuStreamEndCapture(stream, &graph);
+    const CUresult ended = cu_->cuStreamEndCapture(recorder, &graph);
     if (!issued.ok()) {
       if (graph != nullptr) cu_->cuGraphDestroy(graph);
       return issued;

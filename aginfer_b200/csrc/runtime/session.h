@@ -8,8 +8,9 @@
 //     attribute that permits it;
 //   * for a profile the package marks as graph-safe, the recipe is stream-captured on the
 //     caller's stream at the first Enqueue for a given set of tensor addresses and replayed
-//     with one graph launch afterwards (unless the caller is itself capturing, or passed the
-//     legacy null stream, in which case launches are issued one by one as in the reference);
+//     with one graph launch afterwards (unless the caller is itself capturing, in which case
+//     launches are issued one by one as in the reference; for the legacy null stream, which
+//     cannot be captured, they are recorded on a stream of the session's own);
 //   * the device is the current context's when there is one, else ordinal 0;
 //   * kernels whose name starts with "agi_coop_" keep one CTA per SM resident and meet at grid-wide
 //     counters: they are launched with the cooperative attribute, so that the driver refuses a grid that
@@ -120,6 +121,7 @@ class Session {
   bool retained_primary_ = false;
   CUmodule module_ = nullptr;
   CUdeviceptr weights_ = 0, arena_ = 0, workspace_ = 0;
+  CUstream capture_stream_ = nullptr;     // records the launches of callers on the legacy null stream
   std::vector<void*> bound_;              // device address per profile tensor
   std::vector<std::uint64_t> slots_;
   std::vector<void*> params_;

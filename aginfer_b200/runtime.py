@@ -271,7 +271,9 @@ class Session:
         """``options``: a ``run_options(...)`` value, or None for the session's profile as packaged."""
         (ins, n_in, _), (outs, n_out, _) = packed
         raw = C.byref(options[0]) if options is not None else None
-        _check(load_library().agi_session_enqueue(self._h, ins, n_in, outs, n_out, raw, C.c_void_p(stream)))
+        code = _lib.agi_session_enqueue(self._h, ins, n_in, outs, n_out, raw, stream or None)
+        if code:
+            _check(code)
 
     def enqueue(self, inputs: Iterable[TensorView], outputs: Iterable[TensorView], stream: int = 0,
                 options=None) -> None:
