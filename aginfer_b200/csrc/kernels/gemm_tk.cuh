@@ -171,6 +171,50 @@ __device__ __forceinline__ float finish_tile(const float* tile, unsigned P, unsi
   return best;
 }
 
+// Adds `runs` filed partial tiles, in order, over `count` rows and 4 * `quads` columns into the staged tile.  Item =
+// (four columns, row), rows fastest; a thread's items are kEpilogue apart, kBatch at a time, and kRuns loads of each are
+// in flight together (eight 16-byte loads a thread: more spill at the 96 registers that let two CTAs share an SM).
+template <unsigned kBatch, unsigned kRuns, unsigned kEpilogue>
+__device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsigned P, unsigned count, unsigned quads,
+                                         unsigned R, unsigned runs) {
+  if (count == 0) return;
+  const unsigned items = count * quads, step_c = kEpilogue / count, step_r = kEpilogue % count;
+  const unsigned run_step = quads * R;
+  unsigned c4 = threadIdx.x / count, r = threadIdx.x % count;
+  for (unsigned i0 = threadIdx.x; i0 < items; i0 += kEpilogue * kBatch) {
+    float4 a[kBatch][kRuns];
+    unsigned c = c4, q = r;
+#pragma unroll
+    for (unsigned b = 0; b < kBatch; ++b) {
+      const float4* cell = filed + size_t(c) * R + q;
+      const bool live = i0 + b * kEpilogue < items;
+#pragma unroll
+      for (unsigned z = 0; z < kRuns; ++z)
+        if (live && z < runs) a[b][z] = __ldcg(cell + z * run_step);
+      c += step_c;
+      q += step_r;
+      if (q >= count) { q -= count; ++c; }
+    }
+#pragma unroll
+    for (unsigned b = 0; b < kBatch; ++b) {
+      float4 sum = a[b][0];
+#pragma unroll
+      for (unsigned z = 1; z < kRuns; ++z)
+        if (z < runs) { sum.x += a[b][z].x; sum.y += a[b][z].y; sum.z += a[b][z].z; sum.w += a[b][z].w; }
+      if (i0 + b * kEpilogue < items) {
+        for (unsigned z = kRuns; z < runs; ++z) {
+          const float4 more = __ldcg(filed + size_t(c4) * R + r + z * run_step);
+          sum.x += more.x; sum.y += more.y; sum.z += more.z; sum.w += more.w;
+        }
+        *reinterpret_cast<float4*>(tile + r * P + c4 * 4) = sum;
+      }
+      c4 += step_c;
+      r += step_r;
+      if (r >= count) { r -= count; ++c4; }
+    }
+  }
+}
+
 // grid = (weight tiles of all parts, token groups of `tg` rows, ranks), block = threads(kW).  NB: weight rows of a tile, a
 // multiple of 16 (of 32 with kFlagSwiglu) up to 256; tg a multiple of 8, ceil(tg / 128) * NB' * (runs a rank takes) <=
 // 512 with NB' = NB rounded up to 32.  Dynamic shared memory: 1024 + the larger of the ring, stages * (tg + NB) * 128 plus what the last
@@ -464,45 +508,10 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     // ---------------- this rank adds the runs of its share of the rows, in order, and finishes them ----------------
     const unsigned share = ((rows + ranks * 8 - 1) / (ranks * 8)) * 8;
     const unsigned first = min(rank * share, rows), count = min(share, rows - first);
-    // item = (four columns, row), rows fastest; a thread's items are kEpilogue apart, four at a time so that their loads
-    // of four runs are in flight together
-    constexpr unsigned kBatch = 4;
-    const unsigned items = count * (NB / 4), step_c = kEpilogue / max(count, 1u), step_r = kEpilogue % max(count, 1u);
-    const size_t run_step = size_t(NB / 4) * R;
-    unsigned c4 = tid / max(count, 1u), r = tid % max(count, 1u);
-    for (unsigned i0 = tid; i0 < items; i0 += kEpilogue * kBatch) {
-      const float4* cell[kBatch];
-      float* to[kBatch];
-      float4 sum[kBatch];
-#pragma unroll
-      for (unsigned q = 0; q < kBatch; ++q) {
-        const bool live = i0 + q * kEpilogue < items;
-        cell[q] = filed + size_t(live ? c4 : 0u) * R + first + (live ? r : 0u);
-        to[q] = live ? tile_rows + r * P + c4 * 4 : nullptr;
-        sum[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        c4 += step_c;
-        r += step_r;
-        if (r >= count) { r -= count; ++c4; }
-      }
-      for (unsigned z = 0; z < runs; z += 4) {
-        float4 a[kBatch][4];
-#pragma unroll
-        for (unsigned y = 0; y < 4; ++y)
-#pragma unroll
-          for (unsigned q = 0; q < kBatch; ++q)
-            if (z + y < runs) a[q][y] = __ldcg(cell[q] + (z + y) * run_step);
-#pragma unroll
-        for (unsigned y = 0; y < 4; ++y)
-#pragma unroll
-          for (unsigned q = 0; q < kBatch; ++q)
-            if (z + y < runs) {
-              sum[q].x += a[q][y].x; sum[q].y += a[q][y].y; sum[q].z += a[q][y].z; sum[q].w += a[q][y].w;
-            }
-      }
-#pragma unroll
-      for (unsigned q = 0; q < kBatch; ++q)
-        if (to[q] != nullptr) *reinterpret_cast<float4*>(to[q]) = sum[q];
-    }
+    const float4* from = filed + first;
+    if (runs <= 2) add_runs<4, 2, kEpilogue>(from, tile_rows, P, count, NB / 4, R, runs);
+    else if (runs <= 4) add_runs<2, 4, kEpilogue>(from, tile_rows, P, count, NB / 4, R, runs);
+    else add_runs<1, 8, kEpilogue>(from, tile_rows, P, count, NB / 4, R, runs);
     asm volatile("bar.sync 1, %0;" ::"n"(kEpilogue) : "memory");
     finish(count, m0 + first);
   }

@@ -115,7 +115,7 @@ def tc_tiling(M: int, N: int, K: int, elem: int, splits: int | None = None) -> d
 TK_SMEM_BUDGET = 226 * 1024
 TK_PAIR_BUDGET = 112 * 1024                       # shared memory of a CTA that shares its SM with another
 # CTAs in whole clusters that the GPCs hold, one CTA per SM
-TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 138, 4: 132, 5: 120, 6: 126, 8: 120}
+TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 135, 4: 132, 5: 130, 6: 132, 8: 120}
 TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3, 4, 5, 6, 8), "agi_gemm_tc_e4m3_x3": (1,),
                "agi_gemm_tcpk_e4m3": (1, 2, 3, 4, 6, 8), "agi_gemm_tc_bf16_x3": (1, 2, 4, 8)}
 TK_MAX_RING = 8
@@ -659,7 +659,7 @@ class RecipeBuilder:
              ldy: int | None = None, out_f32: bool = False, tactic: str = "auto",
              splits: int | None = None, packed: bool = False, fixed_order: bool = False) -> None:
         """Y[M, N] = epilogue(X[M, K] . W[N, K]^T); ``dtype`` names the operand type (bf16 or e4m3).
-        ``fixed_order``: K is summed as ``k_runs`` says (always so for E4M3), for a bf16 product that feeds an FP8 stack.
+        ``fixed_order``: K is summed as ``k_runs`` says whatever the tile, for products inside a stack of FP8 blocks.
         ``packed`` (E4M3 only): both operands are in the packed layout of ``recipes/layout.py`` (weights packed
         at packaging time, activations by ``quantize_e4m3(..., packed=)``) and ring slots are filled by bulk copies."""
         if dtype == "bf16" and self.is_packed(w):
@@ -671,8 +671,8 @@ class RecipeBuilder:
             flags = ACT[act] | (FLAG_BIAS if bias else 0) | (FLAG_RESIDUAL if residual else 0) | \
                 (FLAG_OUT_F32 if out_f32 else 0) | (FLAG_SCALED if scale_a else 0)
             dummy = Arena(0)
-            runs = k_runs(M, N, K, 1, packed=True)
-            t = tk_tiling(M, (N,), K, 1, runs=runs, clusters=TK_CLUSTERS["agi_gemm_tcpk_e4m3"])
+            runs = k_runs(M, N, K, 1, packed=True) if fixed_order else None
+            t = tk_tiling(M, (N,), K, 1, runs=runs, clusters=TK_CLUSTERS["agi_gemm_tcpk_e4m3"] if runs else (1, 2, 4, 8))
             # the persistent kernel (one CTA per SM walks 128 x TN tiles, two accumulators in tensor memory, the epilogue
             # of one tile under the multiplication of the next) where its estimate is the lower one: many more tiles than
             # SMs, so that the overlapped epilogue outweighs its smaller tiles.
@@ -687,7 +687,7 @@ class RecipeBuilder:
                 cost = ceil_div(count, SM_COUNT) * (K // 128) * max((16384 + tn * 128) / 46, 2 * tn, 400) + 5000 + tn * 25
                 if best_cost is None or cost < best_cost:
                     best_cost, m_tiles, TN, tiles = cost, mt, tn, count
-            if tactic == "persistent" or (tactic == "auto" and runs == 1 and best_cost < t["cost"]):
+            if tactic == "persistent" or (tactic == "auto" and runs in (None, 1) and best_cost < t["cost"]):
                 stage_bytes = 16384 + TN * 128
                 stages = max(2, min(12, TC_SMEM_BUDGET // stage_bytes))
                 self.launch("agi_gemm_tcq_e4m3", (min(tiles, SM_COUNT), 1, 1), (192, 1, 1),
@@ -770,7 +770,7 @@ class RecipeBuilder:
                 slices = max(n for n in (1, 2, 4, 8) if n == 1 or (n <= (splits or 1) and K * elem // 128 >= 2 * n))
                 t = tk_tiling(M, (N,), K, elem, clusters=(slices,), rows_per_tile=256)
             else:
-                runs = k_runs(M, N, K, elem) if fixed_order or dtype == "e4m3" else None
+                runs = k_runs(M, N, K, elem) if fixed_order else None
                 clusters = TK_CLUSTERS[f"agi_gemm_tk_{dtype}"] if runs else (1, 2, 4, 8)
                 t = tk_tiling(M, (N,), K, elem, runs=runs, clusters=clusters)
             self._gemm_tk(f"agi_gemm_tk_{dtype}", f"gemm_{dtype}", t, x, [(w, bias, scale_w, y, N, ldy or N)], M, K, ldx or K,

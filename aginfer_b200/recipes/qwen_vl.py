@@ -297,7 +297,7 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
         """FP8 GEMM over the activations last quantised into ``quant``."""
         bias = Weight(f"{name}.bias") if f"{name}.bias" in weights else None
         r.gemm(quant, Weight(f"{name}.weight"), y, M, N, K, dtype="e4m3", scale_a=scale,
-               scale_w=Weight(f"{name}.weight_scale"), bias=bias, tactic=gemm_tactic, packed=packed, **kw)
+               scale_w=Weight(f"{name}.weight_scale"), bias=bias, tactic=gemm_tactic, packed=packed, fixed_order=True, **kw)
 
     # ---------------- vision tower ----------------
     patches, vpos = r.alloc(P * cfg.patch_k * BF), r.alloc(3 * P * 4)
