@@ -70,3 +70,69 @@ extern "C" __global__ void agi_mrope_bf16(bf16* x, const int* pos, unsigned rows
     p[half] = __float2bfloat16_rn(b * c + a * s);
   }
 }
+
+// The same (1-D or three-stream positions) for head widths that are a multiple of 16 and 16-byte aligned rows.  Bound by
+// the latency of the sine / cosine arithmetic: a block owns a row, its threads compute the row's angles once (one pair a
+// thread, into shared memory) while the row's first vectors are on their way, and turn eight pairs at a time in every
+// head (288 rows x 18 heads of 128: 3.2 us where a thread per pair and a launch per tensor took 8.9).  Heads [0, heads0)
+// are x0's, the rest x1's (queries and keys in different buffers are one launch).
+// grid = rows, block = 128; head_dim a multiple of 16, <= 256; s0 = kRopeOneStream: positions row + pos_offset.
+constexpr unsigned kRopeOneStream = 0xffffffffu;
+extern "C" __global__ void __launch_bounds__(128)
+agi_mrope_pair_bf16(bf16* x0, unsigned heads0, unsigned row_stride0, bf16* x1, unsigned heads1, unsigned row_stride1,
+                    const int* pos, unsigned rows, unsigned head_dim, float log2_theta, unsigned s0, unsigned s1,
+                    unsigned ladder, unsigned pos_offset) {
+  __shared__ __align__(16) float cosine[128], sine[128];
+  grid_dependency_wait();
+  const unsigned row = blockIdx.x, half = head_dim / 2, vecs = half / 8, items = (heads0 + heads1) * vecs;
+  bf16* const base0 = x0 + size_t(row) * row_stride0;
+  bf16* const base1 = x1 + size_t(row) * row_stride1;
+  auto address = [&](unsigned item) {
+    const unsigned head = item / vecs, v = item - head * vecs;
+    return (head < heads0 ? base0 + head * head_dim : base1 + (head - heads0) * head_dim) + v * 8;
+  };
+  // the loads of this thread's first two items do not wait for the angles
+  Bf16x8 lo[2], hi[2];
+  bf16* at[2];
+#pragma unroll
+  for (unsigned u = 0; u < 2; ++u) {
+    const unsigned item = threadIdx.x + u * 128;
+    if (item >= items) continue;
+    at[u] = address(item);
+    lo[u] = *reinterpret_cast<const Bf16x8*>(at[u]);
+    hi[u] = *reinterpret_cast<const Bf16x8*>(at[u] + half);
+  }
+  for (unsigned pair = threadIdx.x; pair < half; pair += 128) {
+    float p;
+    if (s0 == kRopeOneStream) {
+      p = float(row + pos_offset);
+    } else {
+      const unsigned stream = pair < s0 ? 0u : (pair < s0 + s1 ? 1u : 2u);
+      p = float(pos[stream * rows + row]);
+    }
+    const float inv_freq = exp2f(-log2_theta * (float(pair % ladder) / float(ladder)));
+    sincosf(p * inv_freq, &sine[pair], &cosine[pair]);
+  }
+  __syncthreads();
+  auto turn = [&](unsigned item, bf16* to, const Bf16x8& l, const Bf16x8& h) {
+    const unsigned v = (item % vecs) * 8;
+    float a[8], b[8], p[8], q[8];
+    unpack8(l, a);
+    unpack8(h, b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float c = cosine[v + j], s = sine[v + j];
+      p[j] = a[j] * c - b[j] * s;
+      q[j] = b[j] * c + a[j] * s;
+    }
+    *reinterpret_cast<Bf16x8*>(to) = pack8(p);
+    *reinterpret_cast<Bf16x8*>(to + half) = pack8(q);
+  };
+#pragma unroll
+  for (unsigned u = 0; u < 2; ++u)
+    if (threadIdx.x + u * 128 < items) turn(threadIdx.x + u * 128, at[u], lo[u], hi[u]);
+  for (unsigned item = threadIdx.x + 256; item < items; item += 128) {
+    bf16* to = address(item);
+    turn(item, to, *reinterpret_cast<const Bf16x8*>(to), *reinterpret_cast<const Bf16x8*>(to + half));
+  }
+}

@@ -523,11 +523,11 @@ class RecipeBuilder:
         if packed is not None:
             rows, cols = packed
             assert rows * cols == count and cols % 128 == 0
-            self.launch("agi_quantize_e4m3_packed_bf16", (grid_for(count // 16, 256, SM_COUNT * 4), 1, 1), (256, 1, 1),
+            self.launch("agi_quantize_e4m3_packed_bf16", (grid_for(ceil_div(count, 32), 256, SM_COUNT * 4), 1, 1), (256, 1, 1),
                         [x, q, amax, scale_out, U32(rows), U32(cols), U32(padded_token_rows(rows))],
                         op="quantize_e4m3_packed")
             return
-        self.launch("agi_quantize_e4m3_bf16", (blocks, 1, 1), (256, 1, 1), [x, q, amax, scale_out, U32(count)],
+        self.launch("agi_quantize_e4m3_bf16", (grid_for(ceil_div(count, 32), 256, SM_COUNT * 4), 1, 1), (256, 1, 1), [x, q, amax, scale_out, U32(count)],
                     op="quantize_e4m3")
 
     def rmsnorm(self, x: Pointer, gain: Pointer, y: Pointer, rows: int, cols: int, eps: float = 1e-6,
@@ -541,16 +541,35 @@ class RecipeBuilder:
 
     def layernorm(self, x: Pointer, y: Pointer, rows: int, cols: int, eps: float = 1e-5,
                   scale: Pointer | None = None, shift: Pointer | None = None,
-                  x_stride: int | None = None, y_stride: int | None = None) -> None:
+                  x_stride: int | None = None, y_stride: int | None = None, static_modulation: bool = False) -> None:
+        """``static_modulation``: scale and shift were written before the last ``agi_add_rows_bf16`` launch of the profile
+        (which releases its successors only after its own wait) and may be fetched ahead of the dependency wait."""
         assert cols % 8 == 0 and (scale is None) == (shift is None)
         dummy = Arena(0)
         self.launch("agi_layernorm_bf16", (rows, 1, 1), (min(1024, max(32, ceil_div(cols // 8, 32) * 32)), 1, 1),
                     [x, scale or dummy, shift or dummy, y, U32(rows), U32(cols), U32(x_stride or cols),
-                     U32(y_stride or cols), F32(eps), U32(0 if scale is None else 1)],
+                     U32(y_stride or cols), F32(eps), U32(0 if scale is None else 3 if static_modulation else 1)],
                     op="layernorm_modulate" if scale is not None else "layernorm")
+
+    @staticmethod
+    def _rope_vectors(head_dim: int, *operands: tuple[Pointer, int]) -> bool:
+        """Rows of these (pointer, row stride) operands allow the 16-byte rotary kernel (arena addresses are known here)."""
+        return head_dim % 16 == 0 and head_dim <= 256 and all(
+            isinstance(p, Arena) and p.offset % 16 == 0 and stride % 8 == 0 for p, stride in operands)
+
+    def _rope_launch(self, x0: Pointer, heads0: int, row_stride0: int, x1: Pointer, heads1: int, row_stride1: int, rows: int,
+                     head_dim: int, theta: float, *, positions: Pointer | None = None, sections: Sequence[int] = (0, 0, 0),
+                     ladder: int | None = None, pos_offset: int = 0, op: str) -> None:
+        self.launch("agi_mrope_pair_bf16", (rows, 1, 1), (128, 1, 1),
+                    [x0, U32(heads0), U32(row_stride0), x1, U32(heads1), U32(row_stride1), positions or Arena(0), U32(rows),
+                     U32(head_dim), F32(math.log2(theta)), U32(0xffffffff if positions is None else sections[0]),
+                     U32(sections[1]), U32(ladder or head_dim // 2), U32(pos_offset)], op=op, algorithm="row_per_block")
 
     def rope(self, x: Pointer, rows: int, heads: int, head_dim: int, row_stride: int, theta: float,
              pos_offset: int = 0) -> None:
+        if self._rope_vectors(head_dim, (x, row_stride)):
+            self._rope_launch(x, heads, row_stride, x, 0, row_stride, rows, head_dim, theta, pos_offset=pos_offset, op="rope")
+            return
         work = rows * heads * head_dim // 2
         self.launch("agi_rope_bf16", (grid_for(work), 1, 1), (256, 1, 1),
                     [x, U32(rows), U32(heads), U32(head_dim), U32(row_stride), F32(math.log2(theta)), U32(pos_offset)],
@@ -559,20 +578,31 @@ class RecipeBuilder:
     def rope_pair(self, x0: Pointer, heads0: int, row_stride0: int, x1: Pointer, heads1: int, row_stride1: int,
                   rows: int, head_dim: int, theta: float, pos_offset: int = 0) -> None:
         """``rope`` over two tensors (queries and new keys in separate buffers) as one launch."""
+        if self._rope_vectors(head_dim, (x0, row_stride0), (x1, row_stride1)):
+            self._rope_launch(x0, heads0, row_stride0, x1, heads1, row_stride1, rows, head_dim, theta, pos_offset=pos_offset,
+                              op="rope")
+            return
         work = rows * (heads0 + heads1) * head_dim // 2
         self.launch("agi_rope_pair_bf16", (grid_for(work), 1, 1), (256, 1, 1),
                     [x0, U32(heads0), U32(row_stride0), x1, U32(heads1), U32(row_stride1), U32(rows), U32(head_dim),
                      F32(math.log2(theta)), U32(pos_offset)], op="rope")
 
     def mrope(self, x: Pointer, positions: Pointer, rows: int, heads: int, head_dim: int, row_stride: int,
-              theta: float, sections: Sequence[int], ladder: int | None = None) -> None:
+              theta: float, sections: Sequence[int], ladder: int | None = None,
+              second: tuple[Pointer, int, int] | None = None) -> None:
         """``ladder``: rotary pairs per frequency ladder (pair i turns at theta^(-(i mod ladder) / ladder));
-        default head_dim / 2, the single ladder of a language model."""
+        default head_dim / 2, the single ladder of a language model.  ``second``: (pointer, heads, row stride) of
+        another tensor over the same rows (keys beside queries), turned by the same launch where alignment allows."""
         assert sum(sections) == head_dim // 2 and len(sections) == 3
-        work = rows * heads * head_dim // 2
-        self.launch("agi_mrope_bf16", (grid_for(work), 1, 1), (256, 1, 1),
-                    [x, positions, U32(rows), U32(heads), U32(head_dim), U32(row_stride), F32(math.log2(theta)),
-                     U32(sections[0]), U32(sections[1]), U32(ladder or head_dim // 2)], op="mrope")
+        x1, heads1, stride1 = second or (x, 0, row_stride)
+        if self._rope_vectors(head_dim, (x, row_stride), (x1, stride1)):
+            self._rope_launch(x, heads, row_stride, x1, heads1, stride1, rows, head_dim, theta, positions=positions,
+                              sections=sections, ladder=ladder, op="mrope")
+            return
+        for p, n, stride in ((x, heads, row_stride), (x1, heads1, stride1))[:2 if second else 1]:
+            self.launch("agi_mrope_bf16", (grid_for(rows * n * head_dim // 2), 1, 1), (256, 1, 1),
+                        [p, positions, U32(rows), U32(n), U32(head_dim), U32(stride), F32(math.log2(theta)),
+                         U32(sections[0]), U32(sections[1]), U32(ladder or head_dim // 2)], op="mrope")
 
     def attention(self, q: Pointer, k: Pointer, v: Pointer, o: Pointer, *, q_rows: int, kv_rows: int, q_heads: int,
                   kv_heads: int, head_dim: int, q_stride: int, k_stride: int, v_stride: int, o_stride: int,
@@ -896,7 +926,8 @@ class RecipeBuilder:
             src = x
             if ln is not None:
                 assert ln_scratch is not None, "a separate LayerNorm needs a buffer for the normalised activations"
-                self.layernorm(x, ln_scratch, M, K, ln["eps"], scale=ln.get("scale"), shift=ln.get("shift"), x_stride=ldx)
+                self.layernorm(x, ln_scratch, M, K, ln["eps"], scale=ln.get("scale"), shift=ln.get("shift"), x_stride=ldx,
+                               static_modulation=ln.get("static", False))
                 src, ldx = ln_scratch, None
             self.gemm_tcs(src, parts, y, M, K, residual=residual, act=act, ldx=ldx, ldy=ldy)
             return
@@ -907,14 +938,15 @@ class RecipeBuilder:
                 and len({b is None for _, b, _ in parts}) == 1)
         if fuse and fits and ln is not None and not fuse_ln:
             assert ln_scratch is not None, "a separate LayerNorm needs a buffer for the normalised activations"
-            self.layernorm(x, ln_scratch, M, K, ln["eps"], scale=ln.get("scale"), shift=ln.get("shift"), x_stride=ldx)
+            self.layernorm(x, ln_scratch, M, K, ln["eps"], scale=ln.get("scale"), shift=ln.get("shift"), x_stride=ldx,
+                               static_modulation=ln.get("static", False))
             x, ldx, ln = ln_scratch, None, None
         if not (fuse and fits):
             src = x
             if ln is not None:
                 assert ln_scratch is not None, "fallback needs a buffer for the normalised activations"
                 self.layernorm(x, ln_scratch, M, K, ln["eps"], scale=ln.get("scale"), shift=ln.get("shift"),
-                               x_stride=ldx)
+                               x_stride=ldx, static_modulation=ln.get("static", False))
                 src, ldx = ln_scratch, None
             col = 0
             for w, b, n in parts:

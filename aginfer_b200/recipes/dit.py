@@ -288,7 +288,7 @@ def _emit_chunk(r: RecipeBuilder, cfg: DitConfig, profile: str | None, gemm_tact
                          eps=cfg.ln_eps)
         for l in range(0 if block_kernel else cfg.layers):
             b = f"{P}.dit.blocks.{l}"
-            adaln = {"eps": cfg.ln_eps, "scale": mods[l] + mod_row, "shift": mods[l] + (mod_row + D * BF)}
+            adaln = {"eps": cfg.ln_eps, "scale": mods[l] + mod_row, "shift": mods[l] + (mod_row + D * BF), "static": True}
             part = lambda name, n: (Weight(f"{b}.{name}.weight"), Weight(f"{b}.{name}.bias"), n)
             if cfg.is_cross(l):
                 r.fused_linear(seq, [part("attn.to_q", D)], qkv, T, D, ln=adaln, ln_scratch=h, ldy=3 * D, fuse=fuse)
@@ -309,7 +309,7 @@ def _emit_chunk(r: RecipeBuilder, cfg: DitConfig, profile: str | None, gemm_tact
 
         r.fused_linear(seq, [(Weight(f"{P}.dit.proj_out.weight"), Weight(f"{P}.dit.proj_out.bias"), cfg.out_dim)],
                        out_hid, T, D, ln={"eps": cfg.ln_eps, "scale": mods[cfg.layers] + mod_row,
-                                          "shift": mods[cfg.layers] + (mod_row + D * BF)}, ln_scratch=h, fuse=fuse)
+                                          "shift": mods[cfg.layers] + (mod_row + D * BF), "static": True}, ln_scratch=h, fuse=fuse)
         lin(out_hid + cfg.out_dim * BF, f"{P}.action_decoder.fc1", dec_hid, H, cfg.encoder_hidden, cfg.out_dim, act="relu")
         lin(dec_hid, f"{P}.action_decoder.fc2", velocity, H, cfg.action_dim, cfg.encoder_hidden)
         elementwise("agi_euler_step", [x_f32, velocity, x_bf, F32(1.0 / S), U32(H * cfg.action_dim)],

@@ -357,8 +357,8 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
         norm_quantize(h, f"{l}.input_layernorm.weight", hn, S, H)
         group_q([(f"{l}.self_attn.q_proj", q_buf, cfg.q_dim, cfg.q_dim), (f"{l}.self_attn.k_proj", k_cache, cfg.kv_dim,
                   cfg.kv_dim), (f"{l}.self_attn.v_proj", v_cache, cfg.kv_dim, cfg.kv_dim)], S, H)
-        r.mrope(q_buf, Tensor("positions"), S, cfg.heads, D, cfg.q_dim, cfg.theta, cfg.sections)
-        r.mrope(k_cache, Tensor("positions"), S, cfg.kv_heads, D, cfg.kv_dim, cfg.theta, cfg.sections)
+        r.mrope(q_buf, Tensor("positions"), S, cfg.heads, D, cfg.q_dim, cfg.theta, cfg.sections,
+                second=(k_cache, cfg.kv_heads, cfg.kv_dim))
         r.attention(q_buf, k_cache, v_cache, att, q_rows=S, kv_rows=S, q_heads=cfg.heads, kv_heads=cfg.kv_heads,
                     head_dim=D, q_stride=cfg.q_dim, k_stride=cfg.kv_dim, v_stride=cfg.kv_dim, o_stride=cfg.q_dim,
                     mask="causal", amax=(a_max := attention_amax(D)))
