@@ -113,50 +113,6 @@ __device__ __forceinline__ float e4m3_to_float(uint8_t b) {
 // Round-to-nearest-even, saturating to +-448 (never NaN for finite input).
 __device__ __forceinline__ uint8_t float_to_e4m3(float x) { return __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3); }
 
-// Values x -> e4m3(x / scale) (IEEE division, then round to nearest even, saturating), bit for bit, without a
-// division per value.  x * (1 / scale) is within two units in the last place of the quotient, and the E4M3 code of both is
-// the same unless the value lies that close to a midpoint between two codes: then the low 20 bits of its magnitude are
-// within a few of 0x80000 (in E4M3's subnormal range once 2^-6 has been added, which aligns the grids).  Such values, a few
-// in a million, and scales near the ends of the float range take the division.
-struct E4m3Scale {
-  float scale, inverse;
-  bool fast;
-};
-__device__ __forceinline__ E4m3Scale e4m3_scale(float amax) {
-  E4m3Scale s;
-  s.scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
-  s.inverse = __fdiv_rn(1.f, s.scale);
-  s.fast = s.scale > 1e-30f && s.scale < 1e30f;
-  return s;
-}
-__device__ __noinline__ unsigned quantize_e4m3_word(float a, float b, float c, float d, float scale) {
-  return unsigned(float_to_e4m3(__fdiv_rn(a, scale))) | unsigned(float_to_e4m3(__fdiv_rn(b, scale))) << 8 |
-         unsigned(float_to_e4m3(__fdiv_rn(c, scale))) << 16 | unsigned(float_to_e4m3(__fdiv_rn(d, scale))) << 24;
-}
-template <int kCount>   // a multiple of 4
-__device__ __forceinline__ void quantize_e4m3(const float* f, const E4m3Scale& s, unsigned* words) {
-  bool exact = s.fast;
-#pragma unroll
-  for (int w = 0; w < kCount / 4; ++w) {
-    float y[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      y[b] = f[4 * w + b] * s.inverse;
-      const float v = fabsf(y[b]);
-      const unsigned bits = __float_as_uint(v < 0.015625f ? v + 0.015625f : v);
-      exact = exact && ((bits - 0x7fffcu) & 0xfffffu) > 8u;
-    }
-    const unsigned lo = __nv_cvt_float2_to_fp8x2(make_float2(y[0], y[1]), __NV_SATFINITE, __NV_E4M3);
-    const unsigned hi = __nv_cvt_float2_to_fp8x2(make_float2(y[2], y[3]), __NV_SATFINITE, __NV_E4M3);
-    words[w] = lo | hi << 16;
-  }
-  if (!exact) {      // constant indexes only: a loop would put f into local memory
-#pragma unroll
-    for (int w = 0; w < kCount / 4; ++w)
-      words[w] = quantize_e4m3_word(f[4 * w], f[4 * w + 1], f[4 * w + 2], f[4 * w + 3], s.scale);
-  }
-}
-
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float inner = 0.7978845608028654f * (x + 0.044715f * x * x * x);
   return 0.5f * x * (1.f + tanhf(inner));

@@ -46,81 +46,59 @@ extern "C" __global__ void agi_absmax_bf16(const bf16* x, unsigned count, unsign
 
 // Per-tensor dynamic quantisation: scale = amax / 448 (1 when amax is 0), q = e4m3(x / scale)
 // with IEEE division and round-to-nearest-even, saturating.  Block 0 publishes `scale`.
-//
-// Bound by launch latency and one trip through memory (288 x 2048 values: 2.4 us in a chain of launches): a thread
-// converts two groups of 16 values, both in flight.  amax and quantisation of a small tensor as ONE launch, a cluster of
-// eight CTAs exchanging maxima through distributed shared memory, took 5.4 us where the two launches take 3.1.
-extern "C" __global__ void __launch_bounds__(256)
-agi_quantize_e4m3_bf16(const bf16* x, uint8_t* q, const unsigned* amax_bits, float* scale_out, unsigned count) {
+extern "C" __global__ void agi_quantize_e4m3_bf16(const bf16* x, uint8_t* q, const unsigned* amax_bits,
+                                                   float* scale_out, unsigned count) {
   grid_dependency_wait();
-  const E4m3Scale s = e4m3_scale(__uint_as_float(*amax_bits));
-  const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x, groups = count / 16;
-  if (first == 0) *scale_out = s.scale;
+  const float amax = __uint_as_float(*amax_bits);
+  const float scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
+  const unsigned vectors = count / 8;
   const Bf16x8* xv = reinterpret_cast<const Bf16x8*>(x);
-  const bool wide = (reinterpret_cast<size_t>(q) & 15) == 0;
-  for (unsigned i = first; i < groups; i += 2 * step) {
-    Bf16x8 in[2][2];
+  uint2* qv = reinterpret_cast<uint2*>(q);
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < vectors; i += gridDim.x * blockDim.x) {
+    float f[8];
+    unpack8(xv[i], f);
+    unsigned lo = 0, hi = 0;
 #pragma unroll
-    for (unsigned u = 0; u < 2; ++u)
-      if (i + u * step < groups) {
-        in[u][0] = xv[2 * size_t(i + u * step)];
-        in[u][1] = xv[2 * size_t(i + u * step) + 1];
-      }
-#pragma unroll
-    for (unsigned u = 0; u < 2; ++u) {
-      if (i + u * step >= groups) continue;
-      float f[16];
-      unsigned words[4];
-      unpack8(in[u][0], f);
-      unpack8(in[u][1], f + 8);
-      quantize_e4m3<16>(f, s, words);
-      uint2* dst = reinterpret_cast<uint2*>(q + size_t(i + u * step) * 16);
-      if (wide) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
-      } else {
-        dst[0] = make_uint2(words[0], words[1]);
-        dst[1] = make_uint2(words[2], words[3]);
-      }
+    for (int j = 0; j < 4; ++j) {
+      lo |= unsigned(float_to_e4m3(__fdiv_rn(f[j], scale))) << (8 * j);
+      hi |= unsigned(float_to_e4m3(__fdiv_rn(f[4 + j], scale))) << (8 * j);
     }
+    qv[i] = make_uint2(lo, hi);
   }
-  for (unsigned i = groups * 16 + first; i < count; i += step)
-    q[i] = float_to_e4m3(__fdiv_rn(__bfloat162float(x[i]), s.scale));
+  for (unsigned i = vectors * 8 + blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    q[i] = float_to_e4m3(__fdiv_rn(__bfloat162float(x[i]), scale));
 }
 
 // The same quantisation, written in the packed operand layout of the bulk-copy tensor-core GEMM
 // ("K-block-major, swizzled"): the 128-byte K block kb of row r goes to ((kb * rows_padded + r) * 128), its
 // 16-byte chunk c to position c ^ (r & 7).  One thread converts 16 consecutive values = one chunk.
 // cols % 16 == 0; rows past `rows` (up to rows_padded) are left as they are: the GEMM never stores them.
-extern "C" __global__ void __launch_bounds__(256)
-agi_quantize_e4m3_packed_bf16(const bf16* x, uint8_t* q, const unsigned* amax_bits, float* scale_out, unsigned rows,
-                              unsigned cols, unsigned rows_padded) {
+extern "C" __global__ void agi_quantize_e4m3_packed_bf16(const bf16* x, uint8_t* q, const unsigned* amax_bits,
+                                                          float* scale_out, unsigned rows, unsigned cols,
+                                                          unsigned rows_padded) {
   grid_dependency_wait();
-  const E4m3Scale s = e4m3_scale(__uint_as_float(*amax_bits));
-  const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-  if (first == 0) *scale_out = s.scale;
-  const unsigned per_row = cols / 16, groups = rows * per_row;
-  const Bf16x8* xv = reinterpret_cast<const Bf16x8*>(x);
-  for (unsigned i = first; i < groups; i += 2 * step) {
-    Bf16x8 in[2][2];
+  const float amax = __uint_as_float(*amax_bits);
+  const float scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
+  const unsigned chunks_per_row = cols / 16;
+  const unsigned total = rows * chunks_per_row;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / chunks_per_row, chunk = i % chunks_per_row;
+    const unsigned kb = chunk / 8, c = chunk % 8;
+    float f[16];
+    unpack8(*reinterpret_cast<const Bf16x8*>(x + size_t(r) * cols + chunk * 16), f);
+    unpack8(*reinterpret_cast<const Bf16x8*>(x + size_t(r) * cols + chunk * 16 + 8), f + 8);
+    unsigned words[4];
 #pragma unroll
-    for (unsigned u = 0; u < 2; ++u)
-      if (i + u * step < groups) {
-        in[u][0] = xv[2 * size_t(i + u * step)];
-        in[u][1] = xv[2 * size_t(i + u * step) + 1];
-      }
+    for (int wd = 0; wd < 4; ++wd) {
+      unsigned word = 0;
 #pragma unroll
-    for (unsigned u = 0; u < 2; ++u) {
-      const unsigned g = i + u * step;
-      if (g >= groups) continue;
-      float f[16];
-      unsigned words[4];
-      unpack8(in[u][0], f);
-      unpack8(in[u][1], f + 8);
-      quantize_e4m3<16>(f, s, words);
-      const unsigned r = g / per_row, chunk = g - r * per_row;
-      uint8_t* dst = q + (size_t(chunk / 8) * rows_padded + r) * 128 + (((chunk % 8) ^ (r & 7)) << 4);
-      *reinterpret_cast<uint4*>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
+      for (int b = 0; b < 4; ++b) word |= unsigned(float_to_e4m3(__fdiv_rn(f[wd * 4 + b], scale))) << (8 * b);
+      words[wd] = word;
     }
+    uint8_t* dst = q + (size_t(kb) * rows_padded + r) * 128 + ((c ^ (r & 7)) << 4);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
   }
 }
 

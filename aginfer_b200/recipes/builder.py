@@ -523,11 +523,11 @@ class RecipeBuilder:
         if packed is not None:
             rows, cols = packed
             assert rows * cols == count and cols % 128 == 0
-            self.launch("agi_quantize_e4m3_packed_bf16", (grid_for(ceil_div(count, 32), 256, SM_COUNT * 4), 1, 1), (256, 1, 1),
+            self.launch("agi_quantize_e4m3_packed_bf16", (grid_for(count // 16, 256, SM_COUNT * 4), 1, 1), (256, 1, 1),
                         [x, q, amax, scale_out, U32(rows), U32(cols), U32(padded_token_rows(rows))],
                         op="quantize_e4m3_packed")
             return
-        self.launch("agi_quantize_e4m3_bf16", (grid_for(ceil_div(count, 32), 256, SM_COUNT * 4), 1, 1), (256, 1, 1), [x, q, amax, scale_out, U32(count)],
+        self.launch("agi_quantize_e4m3_bf16", (blocks, 1, 1), (256, 1, 1), [x, q, amax, scale_out, U32(count)],
                     op="quantize_e4m3")
 
     def rmsnorm(self, x: Pointer, gain: Pointer, y: Pointer, rows: int, cols: int, eps: float = 1e-6,
