@@ -69,6 +69,7 @@ __device__ __forceinline__ void tmem_wait_loads() { asm volatile("tcgen05.wait::
 struct Out {
   void* y;
   const bf16* bias;
+  const bf16* bias2;     // bias of the up matrix of kFlagSwiglu
   const bf16* other;     // residual, or the gate of kFlagMulSilu; row pitch ldy
   unsigned N, ldy, flags;
   float alpha, alpha2;   // alpha2: the up matrix of kFlagSwiglu
@@ -108,7 +109,7 @@ __device__ __forceinline__ float finish_tile(const float* tile, unsigned P, unsi
 #pragma unroll
           for (int j = 0; j < 8; ++j) other[j] = unsigned(j) < live ? __bfloat162float(src[j]) : 0.f;
       }
-      if (kMode == kScaleBias || kMode == kScaleBiasResidual || (kGen && (o.flags & kFlagBias))) {
+      if (kMode == kScaleBias || kMode == kScaleBiasResidual || ((kGen || kPairs) && (o.flags & kFlagBias))) {
         if (vec) unpack8(*reinterpret_cast<const Bf16x8*>(o.bias + n), bias);
         else
 #pragma unroll
@@ -125,8 +126,19 @@ __device__ __forceinline__ float finish_tile(const float* tile, unsigned P, unsi
         const float4 ulo = *reinterpret_cast<const float4*>(up), uhi = *reinterpret_cast<const float4*>(up + 4);
         const float u[8] = {ulo.x, ulo.y, ulo.z, ulo.w, uhi.x, uhi.y, uhi.z, uhi.w};
         float ur[8], gr[8];
+        if (o.flags & kFlagBias) {
+          float bias2[8];
+          if (vec) unpack8(*reinterpret_cast<const Bf16x8*>(o.bias2 + n), bias2);
+          else
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ur[j] = __fmul_rn(u[j], o.alpha2);
+            for (int j = 0; j < 8; ++j) bias2[j] = unsigned(j) < live ? __bfloat162float(o.bias2[n + j]) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            ur[j] = o.one_run ? fmaf(u[j], o.alpha2, bias2[j]) : __fadd_rn(__fmul_rn(u[j], o.alpha2), bias2[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ur[j] = __fmul_rn(u[j], o.alpha2);
+        }
         unpack8(pack8(v), gr);
         unpack8(pack8(ur), ur);
 #pragma unroll
@@ -412,17 +424,17 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
   const unsigned P = NB + 4;
   float* const tile_rows = reinterpret_cast<float*>(dynamic_smem + (ring - smem_u32(dynamic_smem)));
   Out o;
-  o.y = part.y; o.bias = part.bias; o.other = other; o.N = part.N; o.ldy = part.ldy; o.flags = flags;
+  o.y = part.y; o.bias = part.bias; o.bias2 = p1.bias; o.other = other; o.N = part.N; o.ldy = part.ldy; o.flags = flags;
   o.alpha = o.alpha2 = 1.f;
   o.one_run = runs == 1;
   o.vec = (part.ldy & 7) == 0 && ((reinterpret_cast<size_t>(part.y) | reinterpret_cast<size_t>(part.bias) |
-                                   reinterpret_cast<size_t>(other)) & 15) == 0;   // unused pointers are arena-aligned
+                                   reinterpret_cast<size_t>(p1.bias) | reinterpret_cast<size_t>(other)) & 15) == 0;   // unused pointers are arena-aligned
   float best = 0.f;
   const unsigned special = flags & (kFlagSwiglu | kFlagMulSilu);
   int mode = kGeneral;
   if (o.vec && (part.N & 7) == 0 && !(flags & (kFlagOutF32 | kFlagActMask))) {
     const unsigned plain = flags & (kFlagBias | kFlagResidual);
-    if (special == kFlagSwiglu && plain == 0) mode = kGateUp;
+    if (special == kFlagSwiglu && !(plain & kFlagResidual)) mode = kGateUp;
     else if (special == kFlagMulSilu && plain == 0) mode = kTimesSilu;
     else if (special == 0 && !(flags & kFlagAmax)) mode = int(plain);     // kScale ... kScaleBiasResidual
   }
@@ -563,6 +575,9 @@ AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 2)
 AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 4)
 AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 8)
 AGI_TK_KERNEL(agi_gemm_tc_e4m3_x3, , uint8_t, true, false, false)
+AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 2)
+AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 4)
+AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 8)
 #undef AGI_TK_CLUSTER
 #undef AGI_TK_KERNEL
 

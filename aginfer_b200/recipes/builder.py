@@ -116,7 +116,7 @@ TK_SMEM_BUDGET = 226 * 1024
 TK_PAIR_BUDGET = 112 * 1024                       # shared memory of a CTA that shares its SM with another
 # CTAs in whole clusters that the GPCs hold, one CTA per SM
 TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 135, 4: 132, 5: 130, 6: 132, 8: 120}
-TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3, 4, 5, 6, 8), "agi_gemm_tc_e4m3_x3": (1,),
+TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3, 4, 5, 6, 8), "agi_gemm_tc_e4m3_x3": (1, 2, 4, 8),
                "agi_gemm_tcpk_e4m3": (1, 2, 3, 4, 6, 8), "agi_gemm_tc_bf16_x3": (1, 2, 4, 8)}
 TK_MAX_RING = 8
 
@@ -835,8 +835,9 @@ class RecipeBuilder:
 
     def gemm_group(self, x: Pointer, parts: Sequence[tuple[Pointer, Pointer | None, Pointer | None, Pointer, int, int]],
                    M: int, K: int, *, dtype: str = "bf16", scale_a: Pointer | None = None, ldx: int | None = None,
-                   act: str | None = None, packed: bool = False) -> None:
+                   act: str | None = None, packed: bool = False, runs: int | None = None, split: bool = False) -> None:
         """Up to three GEMMs over one activation matrix in one tensor-core launch (Q | K | V, gate | up).
+        ``runs``: see ``k_runs``; ``split``: the planner may cut K over the ranks of a cluster.
         ``parts``: ``(weight, bias or None, weight scale or None, y, N, ldy)``; either every part has a bias
         or none has; with ``scale_a`` every part brings its weight scale."""
         assert 1 <= len(parts) <= 3
@@ -855,10 +856,40 @@ class RecipeBuilder:
             # few tokens: 128-row tiles would leave most SMs idle, so the K slices of every tile form a cluster
             t = tk_tiling(M, widths, K, elem, clusters=(c["cluster"],), rows_per_tile=128)
         else:
-            t = tk_tiling(M, widths, K, elem, clusters=(1,))
+            t = tk_tiling(M, widths, K, elem, runs=runs, clusters=TK_CLUSTERS[family] if split and runs is None else (1,))
         self._gemm_tk(family, f"gemm_{dtype}_group" + ("_packed" if packed else ""), t, x,
                       [(w, bias, sw, y, N, ldy) for w, bias, sw, y, N, ldy in parts], M, K,
                       padded_token_rows(M) if packed else (ldx or K), flags, scale_a=scale_a)
+
+    def gemm_swiglu(self, x: Pointer, gate: tuple[Pointer, Pointer | None, Pointer | None],
+                    up: tuple[Pointer, Pointer | None, Pointer | None], out: Pointer, M: int, I: int, K: int, *,
+                    dtype: str = "bf16", scale_a: Pointer | None = None, packed: bool = False, amax: Pointer | None = None,
+                    scratch: Pointer | None = None, runs: int | None = None) -> None:
+        """``out[M, I] = silu(x . Wg^T) * (x . Wu^T)`` (both products rounded to bf16 first) for (weight, bias, weight
+        scale) triples: the SwiGLU runs in the GEMM's epilogue.  One launch whose tiles hold the gate and up rows of the
+        same features (288 tokens, 2 x 11008 x 2048 packed: 20 us; two launches and a SwiGLU launch 30), or, given
+        ``scratch`` [M, I], two: the gate, then the up product times silu of it.  ``runs``: see ``k_runs``."""
+        assert (gate[1] is None) == (up[1] is None)
+        elem = 1 if dtype == "e4m3" else 2
+        flags = (FLAG_SCALED if scale_a is not None else 0) | (FLAG_BIAS if gate[1] is not None else 0)
+        ldx = padded_token_rows(M) if packed else K
+        if scratch is not None:
+            family = "agi_gemm_tcpk_e4m3" if packed else f"agi_gemm_tk_{dtype}"
+            t = tk_tiling(M, (I,), K, elem, runs=runs, clusters=TK_CLUSTERS[family] if runs else (1, 2, 4, 8))
+            self._gemm_tk(family, f"gemm_{dtype}", t, x, [(*gate, scratch, I, I)], M, K, ldx, flags, scale_a=scale_a)
+            self._gemm_tk(family, f"gemm_{dtype}_swiglu", t, x, [(*up, out, I, I)], M, K, ldx, flags | FLAG_MUL_SILU,
+                          scale_a=scale_a, other=scratch, amax=amax)
+            return
+        family = "agi_gemm_tcpk_e4m3" if packed else f"agi_gemm_tc_{dtype}_x3"
+        if dtype == "bf16" and M <= 64:
+            c = tc_cluster_tiling(M, 2 * 128 * ceil_div(I, 128), K, elem, dtype, sizes=(2, 4, 8))
+            t = tk_tiling(M, (I,), K, elem, swiglu=True, clusters=(c["cluster"] if c is not None else 1,))
+        elif packed and not runs:
+            t = tk_tiling(M, (I,), K, elem, swiglu=True)
+        else:
+            t = tk_tiling(M, (I,), K, elem, swiglu=True, runs=runs or 1, clusters=TK_CLUSTERS[family] if packed else (1,))
+        self._gemm_tk(family, f"gemm_{dtype}_swiglu", t, x, [(*gate, out, I, I), (*up, out, I, I)], M, K, ldx,
+                      flags | FLAG_SWIGLU, scale_a=scale_a, amax=amax)
 
     def gemm_batch(self, x: Pointer, parts: Sequence[tuple[Pointer, Pointer]], y: Pointer, M: int, N: int, K: int,
                    seg_stride: int, ldx: int | None = None) -> None:

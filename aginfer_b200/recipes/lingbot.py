@@ -175,8 +175,12 @@ def build_recipe(cfg: EpisodeConfig, weights, packed: bool = False, trace: bool 
                             kv_static=True, kv_static_rows=prefix)
                 lin(att, f"{l}.self_attn.o_proj", seq2, T, H, H, residual=seq)
                 r.rmsnorm(seq2, Weight(f"{l}.post_attention_layernorm.weight"), hn, T, H, bb.eps)
-                group(hn, [(f"{l}.mlp.gate_proj", gu, I, 2 * I), (f"{l}.mlp.up_proj", gu + I * BF, I, 2 * I)], T, H)
-                r.swiglu(gu, gu + I * BF, act, T, I, 2 * I)
+                if H % 64 == 0 and f"{l}.mlp.gate_proj.bias" not in weights and f"{l}.mlp.up_proj.bias" not in weights:
+                    r.gemm_swiglu(hn, (Weight(f"{l}.mlp.gate_proj.weight"), None, None),
+                                  (Weight(f"{l}.mlp.up_proj.weight"), None, None), act, T, I, H)
+                else:
+                    group(hn, [(f"{l}.mlp.gate_proj", gu, I, 2 * I), (f"{l}.mlp.up_proj", gu + I * BF, I, 2 * I)], T, H)
+                    r.swiglu(gu, gu + I * BF, act, T, I, 2 * I)
                 lin(act, f"{l}.mlp.down_proj", seq, T, H, I, residual=seq2)
             r.rmsnorm(seq, Weight(f"{E}.norm.weight"), hn, T, H, bb.eps)
             lin(hn, f"{E}.action_out", vel, T, PAD, H)

@@ -28,7 +28,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import Sequence
 
-from .builder import RecipeBuilder, Tensor, U32, Weight, ceil_div, grid_for, io
+from .builder import RecipeBuilder, Tensor, U32, Weight, ceil_div, grid_for, io, k_runs
 from .layout import pack_kblock_swizzled, padded_token_rows
 
 
@@ -210,7 +210,7 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
     block-by-block checks: ``vision_trace`` [v_layers + 1, patches, 1280] (the patch embedding, then every
     block's output), ``merged_out`` [merged, hidden] (window order) and ``hidden_trace``
     [layers + 1, tokens, hidden] (the assembled prefix, then every decoder layer's output).  ``group`` runs the
-    projections that share an input (Q | K | V, gate | up) as one launch each.  ``packed``: ``weights`` describes
+    projections that share an input (Q | K | V, gate | up) as one launch each, SwiGLU in the epilogue of gate | up.  ``packed``: ``weights`` describes
     a checkpoint that went through ``pack_checkpoint``; activations are quantised into the same layout and every
     FP8 GEMM fills its ring with bulk copies.  ``tail(recipe, cache, hidden)`` appends launches that consume the
     prefill inside the same profile (an action expert reading the K/V cache), with ``extra_inputs`` /
@@ -276,19 +276,30 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
         """A counter for the attention kernel to leave max |o| in, for the head widths that have such a variant."""
         return r.counter() if head_dim in (80, 128) else None
 
-    def swiglu_quantize(gate, up, out, rows: int, cols: int):
+    def gate_up_quantize(mlp: str, out, scratch, rows: int, cols: int, K: int):
+        """Gate and up projections, SwiGLU and the E4M3 quantisation of its result."""
         amax = r.counter()
-        r.swiglu(gate, up, out, rows, cols, 2 * cols, amax=amax)
+        if group and gemm_tactic == "auto":
+            part = lambda n: (Weight(f"{mlp}.{n}.weight"), Weight(f"{mlp}.{n}.bias") if f"{mlp}.{n}.bias" in weights else None,
+                              Weight(f"{mlp}.{n}.weight_scale"))
+            # narrow pairs sum K in one run, wide ones as one of them alone would; row-major pairs of many wide rows take a
+            # launch each (their tiles then come from one matrix and leave the planner more freedom)
+            runs = 1 if 2 * cols <= 8192 else k_runs(rows, cols, K, 1, packed)
+            two = not packed and 2 * cols > 8192 and rows > 128
+            r.gemm_swiglu(quant, part("gate_proj"), part("up_proj"), out, rows, cols, K, dtype="e4m3", scale_a=scale,
+                          packed=packed, amax=amax, scratch=scratch if two else None, runs=runs)
+        else:
+            linear_q(f"{mlp}.gate_proj", scratch, rows, cols, K, ldy=2 * cols)
+            linear_q(f"{mlp}.up_proj", scratch + cols * BF, rows, cols, K, ldy=2 * cols)
+            r.swiglu(scratch, scratch + cols * BF, out, rows, cols, 2 * cols, amax=amax)
         quantize(out, rows, cols, amax=amax)
 
     def group_q(parts, M: int, K: int) -> None:
         """``parts``: (name, y, N, ldy); FP8 GEMMs over ``quant`` sharing one launch when ``group`` is set."""
-        # wide pairs (the decoder's gate | up: 2 x 11008) run faster as two launches of the 256-row kernel than as one
-        # grouped launch of 128-row tiles (288 tokens: 2 x 13.6 us against 39.5 us); small parts (K, V) gain from sharing
-        if group and gemm_tactic == "auto" and sum(p[2] for p in parts) <= 8192:
+        if group and gemm_tactic == "auto":
             r.gemm_group(quant, [(Weight(f"{n}.weight"), Weight(f"{n}.bias") if f"{n}.bias" in weights else None,
                                   Weight(f"{n}.weight_scale"), y, N, ldy) for n, y, N, ldy in parts], M, K,
-                         dtype="e4m3", scale_a=scale, packed=packed)
+                         dtype="e4m3", scale_a=scale, packed=packed, runs=1)
         else:
             for n, y, N, ldy in parts:
                 linear_q(n, y, M, N, K, ldy=ldy)
@@ -324,8 +335,7 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
         quantize(attn, P, VH, amax=a_max)
         linear_q(f"{b}.attn.proj", x2, P, VH, VH, residual=x)
         norm_quantize(x2, f"{b}.norm2.weight", normed, P, VH)
-        group_q([(f"{b}.mlp.gate_proj", gate_up, VI, 2 * VI), (f"{b}.mlp.up_proj", gate_up + VI * BF, VI, 2 * VI)], P, VH)
-        swiglu_quantize(gate_up, gate_up + VI * BF, act, P, VI)
+        gate_up_quantize(f"{b}.mlp", act, gate_up, P, VI, VH)
         linear_q(f"{b}.mlp.down_proj", x, P, VH, VI, residual=x2)
         snapshot(x, "vision_trace", i + 1, P * VH * BF)
     watch("")
@@ -365,8 +375,7 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
         quantize(att, S, cfg.q_dim, amax=a_max)
         linear_q(f"{l}.self_attn.o_proj", h2, S, H, cfg.q_dim, residual=h)
         norm_quantize(h2, f"{l}.post_attention_layernorm.weight", hn, S, H)
-        group_q([(f"{l}.mlp.gate_proj", gu, I, 2 * I), (f"{l}.mlp.up_proj", gu + I * BF, I, 2 * I)], S, H)
-        swiglu_quantize(gu, gu + I * BF, sw, S, I)
+        gate_up_quantize(f"{l}.mlp", sw, gu, S, I, H)
         linear_q(f"{l}.mlp.down_proj", h, S, H, I, residual=h2)
         snapshot(h, "hidden_trace", i + 1, S * H * BF)
     watch("")
