@@ -401,7 +401,8 @@ agi_attention_rows_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, un
 // grid = (q_heads, ceil(q_rows / 16)), block = 256; head_dim a multiple of 16, <= 64 (agi_attention_mma_bf16_d128: <= 128).
 // dynamic shared memory = 2 * kv16 * (head_dim + 8) * 2 (K and V) + merge area 8 * 16 * (head_dim + 2) * 4,
 // kv16 = kv_rows rounded up to 16.
-template <int kKsteps, int kDtiles, bool kAliasMerge>
+// kExact: head_dim is kKsteps * 16 (the loops over it have no conditions).
+template <int kKsteps, int kDtiles, bool kAliasMerge, bool kExact>
 __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows,
                                                    unsigned kv_rows, unsigned q_heads, unsigned kv_heads, unsigned head_dim,
                                                    unsigned q_stride, unsigned k_stride, unsigned v_stride, unsigned o_stride,
@@ -447,7 +448,7 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
   stage(static_rows, kv16);
   asm volatile("cp.async.commit_group;" ::: "memory");
   // ---- Q fragments (A operand), pre-scaled: rows g, g + 8 of each 16-row tile; zero past q_rows ----
-  const unsigned ksteps = head_dim / 16;   // <= kKsteps
+  const unsigned ksteps = kExact ? kKsteps : head_dim / 16;   // <= kKsteps
   unsigned qa[1][kKsteps][4];
 #pragma unroll
   for (int mt = 0; mt < 1; ++mt)
@@ -475,7 +476,7 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
   for (int nt = 0; nt < kDtiles; ++nt)
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[nt][i] = 0.f;
-  const unsigned dtiles = head_dim / 8;    // <= kDtiles
+  const unsigned dtiles = 2 * ksteps;      // <= kDtiles
   // Few keys (at most two 16-key blocks, e.g. self-attention over 17 tokens): splitting the keys over warps would
   // leave six warps idle and still pay the merge.  Instead every warp w < dtiles scores ALL keys (the same few
   // MMAs in each warp) and multiplies P with the 8 value columns of ITS tile only: no merge, no second barrier,
@@ -487,24 +488,32 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
 
   for (unsigned base = first_key; base < kv16; base += key_step * kGroup) {
     float s[kGroup][2][4];
+    unsigned k_addr[kGroup];   // lanes 0-7 | 8-15 | 16-23 | 24-31: 8 x 8 blocks (keys 0, depth 0) | (0, 8) | (8, 0) | (8, 8)
+#pragma unroll
+    for (int b = 0; b < kGroup; ++b) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) s[b][half][0] = s[b][half][1] = s[b][half][2] = s[b][half][3] = 0.f;
+      // a block past the last one scores the last one's keys again; the mask below discards them by their number
+      const unsigned key0 = min(base + b * key_step, kv16 - 16);
+      k_addr[b] = static_cast<unsigned>(__cvta_generic_to_shared(
+          k_tile + (key0 + (lane >> 4) * 8 + (lane & 7)) * pitch + ((lane >> 3) & 1) * 8));
+    }
+    // depth outermost: the six accumulators are independent, so no MMA waits for the one issued before it
+#pragma unroll
+    for (int ks = 0; ks < kKsteps; ++ks)
+      if (ks < ksteps) {
+#pragma unroll
+        for (int b = 0; b < kGroup; ++b) {
+          unsigned b0, b1, b2, b3;
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(k_addr[b] + ks * 32));
+          skinny_mma_bf16(s[b][0], qa[0][ks][0], qa[0][ks][1], qa[0][ks][2], qa[0][ks][3], b0, b1);
+          skinny_mma_bf16(s[b][1], qa[0][ks][0], qa[0][ks][1], qa[0][ks][2], qa[0][ks][3], b2, b3);
+        }
+      }
 #pragma unroll
     for (int b = 0; b < kGroup; ++b) {
       const unsigned key0 = base + b * key_step;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) s[b][half][0] = s[b][half][1] = s[b][half][2] = s[b][half][3] = -3.0e38f;
-      if (key0 >= kv16) continue;
-      // B fragments of K for the two 8-key tiles: b0 = (d 2t..2t+1, key g), b1 = (d 2t+8.., key g)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        s[b][half][0] = s[b][half][1] = s[b][half][2] = s[b][half][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < kKsteps; ++ks)
-          if (ks < ksteps) {
-            const bf16* row = k_tile + (key0 + half * 8 + g) * pitch + ks * 16 + 2 * t;
-            skinny_mma_bf16(s[b][half], qa[0][ks][0], qa[0][ks][1], qa[0][ks][2], qa[0][ks][3],
-                            *reinterpret_cast<const unsigned*>(row), *reinterpret_cast<const unsigned*>(row + 8));
-          }
-      }
       // mask
 #pragma unroll
       for (int half = 0; half < 2; ++half)
@@ -560,13 +569,27 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
     for (int b = 0; b < kGroup; ++b) {
       const unsigned key0 = base + b * key_step;
       if (key0 >= kv16) continue;
+      if (by_dims) {
 #pragma unroll
-      for (int nt = 0; nt < kDtiles; ++nt)
-        if (nt < dtiles && (!by_dims || nt == int(warp))) {
-          const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(v_tile + (key0 + (lane & 15)) * pitch + nt * 8));
-          unsigned b0, b1;
-          asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
+        for (int nt = 0; nt < kDtiles; ++nt)
+          if (nt == int(warp)) {
+            const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(v_tile + (key0 + (lane & 15)) * pitch + nt * 8));
+            unsigned b0, b1;
+            asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
+            skinny_mma_bf16(out[nt], pa[b][0], pa[b][1], pa[b][2], pa[b][3], b0, b1);
+          }
+        continue;
+      }
+#pragma unroll
+      for (int nt = 0; nt < kDtiles; nt += 2)   // head_dim / 8 is even: two value tiles per load
+        if (nt < dtiles) {
+          const unsigned addr = static_cast<unsigned>(
+              __cvta_generic_to_shared(v_tile + (key0 + (lane & 15)) * pitch + (nt + (lane >> 4)) * 8));
+          unsigned b0, b1, b2, b3;
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
           skinny_mma_bf16(out[nt], pa[b][0], pa[b][1], pa[b][2], pa[b][3], b0, b1);
+          skinny_mma_bf16(out[nt + 1], pa[b][0], pa[b][1], pa[b][2], pa[b][3], b2, b3);
         }
     }
   }
@@ -634,8 +657,12 @@ extern "C" __global__ void __launch_bounds__(256)
 agi_attention_mma_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows, unsigned kv_rows,
                        unsigned q_heads, unsigned kv_heads, unsigned head_dim, unsigned q_stride, unsigned k_stride,
                        unsigned v_stride, unsigned o_stride, float scale, unsigned mask_mode, unsigned mask_arg) {
-  attention_mma_body<4, 8, false>(q, k, v, o, q_rows, kv_rows, q_heads, kv_heads, head_dim, q_stride, k_stride, v_stride,
-                                  o_stride, scale, mask_mode, mask_arg);
+  if (head_dim == 48)
+    attention_mma_body<3, 8, false, true>(q, k, v, o, q_rows, kv_rows, q_heads, kv_heads, 48, q_stride, k_stride, v_stride,
+                                          o_stride, scale, mask_mode, mask_arg);
+  else
+    attention_mma_body<4, 8, false, false>(q, k, v, o, q_rows, kv_rows, q_heads, kv_heads, head_dim, q_stride, k_stride,
+                                           v_stride, o_stride, scale, mask_mode, mask_arg);
 }
 
 // The same for heads up to 128 wide (a 50-token action expert over a 256-token prefix: 8 heads of 128).  The streaming
@@ -647,6 +674,10 @@ extern "C" __global__ void __launch_bounds__(256)
 agi_attention_mma_bf16_d128(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows, unsigned kv_rows,
                             unsigned q_heads, unsigned kv_heads, unsigned head_dim, unsigned q_stride, unsigned k_stride,
                             unsigned v_stride, unsigned o_stride, float scale, unsigned mask_mode, unsigned mask_arg) {
-  attention_mma_body<8, 16, true>(q, k, v, o, q_rows, kv_rows, q_heads, kv_heads, head_dim, q_stride, k_stride, v_stride,
-                                  o_stride, scale, mask_mode, mask_arg);
+  if (head_dim == 128)
+    attention_mma_body<8, 16, true, true>(q, k, v, o, q_rows, kv_rows, q_heads, kv_heads, 128, q_stride, k_stride, v_stride,
+                                          o_stride, scale, mask_mode, mask_arg);
+  else
+    attention_mma_body<8, 16, true, false>(q, k, v, o, q_rows, kv_rows, q_heads, kv_heads, head_dim, q_stride, k_stride,
+                                           v_stride, o_stride, scale, mask_mode, mask_arg);
 }

@@ -1,27 +1,32 @@
 // Tensor-core attention for many query rows (prefill: 288 causal tokens with 128-wide heads; the vision
 // tower: 512 patch tokens, 80-wide heads, block-diagonal windows).  Streaming-softmax formulation on
-// warp-level MMAs:
+// warp-level MMAs, parallel over rows, keys and output columns:
 //
-//   * one block of 1, 2 or 4 warps per (16, 32 or 64 query rows, head): fewer rows per block when the grid
-//     would otherwise leave most SMs idle; warp w owns rows 16w ... 16w + 15 and keeps its Q
-//     fragments, running row maxima / sums and the output accumulators in registers;
-//   * keys are visited in tiles of 64: K and V tiles are staged row-major in shared memory by 16-byte
-//     asynchronous copies, double-buffered so that tile i + 1 lands while tile i is multiplied;
-//   * S = Q.K^T on m16n8k16 (a K row is the "col" B operand as it lies), mask, running maximum, P = exp(S - m)
-//     reused in place as the A operand of P.V, V through ldmatrix.trans;
+//   * one block of 8 warps per (32 query rows, head); warps form two groups of 16 rows, four warps each;
+//   * keys are visited in chunks of four 64-key tiles, staged row-major in shared memory by 16-byte
+//     asynchronous copies (K of the next chunk lands while P.V of this one runs);
+//   * each warp of a group multiplies Q with one tile's keys, masks, and leaves the tile's row maxima in shared
+//     memory; from the maxima of the tiles before it every warp knows the running maximum its tile would have met,
+//     so it forms P = exp(S - m) and the tile's row sums at once and leaves them in shared memory too;
+//   * each warp then adds P.V of the four tiles, in order and with the streaming formulation's rescaling between
+//     them, for a quarter of the head's columns: per output the same operations in the same order as one warp
+//     walking the tiles one by one, which is what this replaced;
 //   * only key tiles a block of rows can see are visited: the causal prefix, or the diagonal block(s).
+//
+// What bounds it: the chain of dependent steps per tile, not bytes or tensor cores, so the tiles of a chunk run
+// side by side and each MMA chain has seven others to hide behind (the depth loop is outermost).
 //
 // Head width is a template parameter (16-element steps); grouped-query attention maps query head h to KV
 // head h / (q_heads / kv_heads).  Pitch of the shared tiles = head_dim + 8 elements: rows stay 16-byte
 // aligned and the eight rows of a fragment fall into different banks.
-// grid = (ceil(q_rows / (16 * warps)), q_heads), block = 32 * warps, dynamic shared memory = 4 * 64 * (head_dim + 8) * 2.
+// grid = (ceil(q_rows / 32), q_heads), block = 256, dynamic shared memory = 4 * 256 * (head_dim + 8) + 17408.
 #pragma once
 
 #include "attention.cuh"
 
 namespace fa {
 
-constexpr unsigned kKeyTile = 64;
+constexpr unsigned kKeyTile = 64, kTiles = 4, kChunk = kKeyTile * kTiles, kRows = 32, kThreads = 256;
 
 template <int HD16>
 __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows,
@@ -29,14 +34,19 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
                                                unsigned k_stride, unsigned v_stride, unsigned o_stride, float scale,
                                                unsigned mask_mode, unsigned mask_arg, unsigned* amax_bits = nullptr) {
   constexpr unsigned head_dim = HD16 * 16, pitch = head_dim + 8, vec_per_row = head_dim / 8;
+  constexpr int kCols = (2 * HD16 + int(kTiles) - 1) / int(kTiles);   // 8-column output tiles of a warp, the last may be absent
   extern __shared__ __align__(16) unsigned char attn_smem[];
-  bf16* tiles = reinterpret_cast<bf16*>(attn_smem);   // [2 buffers][K | V][64][pitch]
+  bf16* k_chunk = reinterpret_cast<bf16*>(attn_smem);                         // [256][pitch]
+  bf16* v_chunk = k_chunk + kChunk * pitch;                                   // [256][pitch]
+  uint4* p_frag = reinterpret_cast<uint4*>(v_chunk + kChunk * pitch);         // [2 groups][4 tiles][4 16-key steps][32 lanes]
+  float* maxima = reinterpret_cast<float*>(p_frag + 2 * kTiles * 4 * 32);     // [2][4][16 rows]
+  float* sums = maxima + 2 * kTiles * 16;                                     // [2][4][16]
   grid_dependency_wait();
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const unsigned group = warp / kTiles, own = warp % kTiles;                  // row group; tile (then columns) of this warp
   const unsigned head = blockIdx.y, kv_head = head / (q_heads / kv_heads);
-  const unsigned rows_per_block = (blockDim.x >> 5) * 16;   // one 16-row MMA tile per warp; 1, 2 or 4 warps
-  const unsigned row_base = blockIdx.x * rows_per_block, warp_row = row_base + warp * 16;
-  const unsigned last_row = min(row_base + rows_per_block, q_rows) - 1;
+  const unsigned row_base = blockIdx.x * kRows, warp_row = row_base + group * 16;
+  const unsigned last_row = min(row_base + kRows, q_rows) - 1, warp_last = min(warp_row + 15, q_rows - 1);
 
   // keys this block of rows can see
   unsigned key_begin = 0, key_end = kv_rows;
@@ -47,25 +57,30 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
   }
   const unsigned tiles_total = key_end > key_begin ? (key_end - key_begin + kKeyTile - 1) / kKeyTile : 0;
 
-  auto stage = [&](unsigned tile, unsigned buffer) {
-    bf16* k_tile = tiles + size_t(buffer) * 2 * kKeyTile * pitch;
-    bf16* v_tile = k_tile + kKeyTile * pitch;
-    const unsigned key0 = key_begin + tile * kKeyTile;
-    for (unsigned i = threadIdx.x; i < kKeyTile * vec_per_row; i += blockDim.x) {
+  auto stage = [&](bf16* dst, const bf16* src, unsigned stride, unsigned first_tile) {   // up to four tiles, one commit group
+    const unsigned keys = first_tile < tiles_total ? min(tiles_total - first_tile, kTiles) * kKeyTile : 0;
+    const unsigned key0 = key_begin + first_tile * kKeyTile;
+    for (unsigned i = threadIdx.x; i < keys * vec_per_row; i += kThreads) {
       const unsigned j = i / vec_per_row, d = (i % vec_per_row) * 8;
       const unsigned key = key0 + j, src_row = min(key, kv_rows - 1), bytes = key < kv_rows ? 16u : 0u;  // zero-fill past the end
-      const unsigned kd = static_cast<unsigned>(__cvta_generic_to_shared(k_tile + j * pitch + d));
-      const unsigned vd = static_cast<unsigned>(__cvta_generic_to_shared(v_tile + j * pitch + d));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd),
-                   "l"(k + size_t(src_row) * k_stride + kv_head * head_dim + d), "r"(bytes) : "memory");
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd),
-                   "l"(v + size_t(src_row) * v_stride + kv_head * head_dim + d), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                       static_cast<unsigned>(__cvta_generic_to_shared(dst + j * pitch + d))),
+                   "l"(src + size_t(src_row) * stride + kv_head * head_dim + d), "r"(bytes) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (tiles_total > 0) stage(0, 0);
+  // does this group of rows see anything of a tile?
+  auto visits = [&](unsigned tile) {
+    const unsigned key0 = key_begin + tile * kKeyTile;
+    bool any = tile < tiles_total && warp_row < q_rows;
+    if (mask_mode == 1) any = any && key0 <= warp_last + mask_arg;
+    if (mask_mode == 2) any = any && key0 < (warp_last / mask_arg + 1) * mask_arg && key0 + kKeyTile > (warp_row / mask_arg) * mask_arg;
+    return any;
+  };
+  stage(k_chunk, k, k_stride, 0);
+  stage(v_chunk, v, v_stride, 0);
 
-  // Q fragments (A operand) as stored: rows g and g + 8 of this warp's 16; zero past q_rows.  The softmax
+  // Q fragments (A operand) as stored: rows g and g + 8 of this group's 16; zero past q_rows.  The softmax
   // scale is applied to the fp32 scores, so no second rounding of Q.
   unsigned qa[HD16][4];
 #pragma unroll
@@ -79,42 +94,37 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
       }
     }
 
-  float row_max[2] = {-3.0e38f, -3.0e38f}, row_sum[2] = {0.f, 0.f}, out[2 * HD16][4];
+  float row_max[2] = {-3.0e38f, -3.0e38f}, row_sum[2] = {0.f, 0.f}, out[kCols][4];
 #pragma unroll
-  for (int nt = 0; nt < 2 * HD16; ++nt)
+  for (int c = 0; c < kCols; ++c)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) out[nt][i] = 0.f;
+    for (int i = 0; i < 4; ++i) out[c][i] = 0.f;
 
-  for (unsigned tile = 0; tile < tiles_total; ++tile) {
-    const unsigned buffer = tile & 1;
-    if (tile + 1 < tiles_total) {
-      stage(tile + 1, buffer ^ 1);                       // that buffer was released by the barrier below
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+  for (unsigned first = 0; first < tiles_total; first += kTiles) {
+    const bool more = first + kTiles < tiles_total;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");   // K of this chunk (V may still be under way)
     __syncthreads();
-    const bf16* k_tile = tiles + size_t(buffer) * 2 * kKeyTile * pitch;
-    const bf16* v_tile = k_tile + kKeyTile * pitch;
-    const unsigned key0 = key_begin + tile * kKeyTile;
-    // a warp whose rows see nothing of this tile skips the arithmetic (but not the barriers)
-    const unsigned warp_last = min(warp_row + 15, q_rows - 1);
-    bool any = warp_row < q_rows;
-    if (mask_mode == 1) any = any && key0 <= warp_last + mask_arg;
-    if (mask_mode == 2) any = any && key0 < (warp_last / mask_arg + 1) * mask_arg && key0 + kKeyTile > (warp_row / mask_arg) * mask_arg;
+
+    // scores of this warp's tile, masked, and their row maxima
+    const bool any = visits(first + own);
+    const unsigned key0 = key_begin + (first + own) * kKeyTile;
+    float s[8][4];
     if (any) {
-      float s[8][4];
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-        const bf16* row = k_tile + (nt * 8 + g) * pitch + 2 * t;
+      for (int nt = 0; nt < 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+      // lanes 0-7 | 8-15 | 16-23 | 24-31 address the 8 x 8 blocks (keys nt, depth 0) | (nt, 8) | (nt + 1, 0) | (nt + 1, 8)
+      const unsigned k_addr = static_cast<unsigned>(__cvta_generic_to_shared(
+          k_chunk + (own * kKeyTile + (lane >> 4) * 8 + (lane & 7)) * pitch + ((lane >> 3) & 1) * 8));
 #pragma unroll
-        for (int ks = 0; ks < HD16; ++ks) {
-          const unsigned b0 = *reinterpret_cast<const unsigned*>(row + ks * 16);
-          const unsigned b1 = *reinterpret_cast<const unsigned*>(row + ks * 16 + 8);
+      for (int ks = 0; ks < HD16; ++ks)
+#pragma unroll
+        for (int nt = 0; nt < 8; nt += 2) {
+          unsigned b0, b1, b2, b3;
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(k_addr + (nt * 8 * pitch + ks * 16) * 2));
           skinny_mma_bf16(s[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
+          skinny_mma_bf16(s[nt + 1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b2, b3);
         }
-      }
       // mask: c0,c1 belong to row g (keys 2t, 2t+1 of the 8-key tile), c2,c3 to row g + 8
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
@@ -126,7 +136,6 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
           if (mask_mode == 2) visible = visible && key / mask_arg == row / mask_arg;
           s[nt][i] = visible ? s[nt][i] * scale : -3.0e38f;
         }
-      unsigned pa[4][4];   // [16-key step][a0..a3]
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {   // hr 0: row g, hr 1: row g + 8
         float tile_max = -3.0e38f;
@@ -134,8 +143,33 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
         for (int nt = 0; nt < 8; ++nt) tile_max = fmaxf(tile_max, fmaxf(s[nt][2 * hr], s[nt][2 * hr + 1]));
         tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 1));
         tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 2));
-        const float new_max = fmaxf(row_max[hr], tile_max);
-        const float rescale = new_max > -1.0e38f ? __expf(row_max[hr] - new_max) : 1.f;
+        if (t == 0) maxima[(group * kTiles + own) * 16 + g + hr * 8] = tile_max;
+      }
+    }
+    __syncthreads();                                       // maxima are there, K is no longer needed
+    if (more) stage(k_chunk, k, k_stride, first + kTiles);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+
+    // running maximum before and after every tile, as a walk over the tiles would meet them
+    float before[kTiles][2], after[kTiles][2];
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {
+      float m = row_max[hr];
+#pragma unroll
+      for (unsigned i = 0; i < kTiles; ++i) {
+        before[i][hr] = m;
+        if (visits(first + i)) m = fmaxf(m, maxima[(group * kTiles + i) * 16 + g + hr * 8]);
+        after[i][hr] = m;
+      }
+      row_max[hr] = m;
+    }
+    if (any) {
+      unsigned pa[4][4];   // [16-key step][a0..a3]
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        float new_max = after[0][hr];
+#pragma unroll
+        for (unsigned i = 1; i < kTiles; ++i) new_max = own == i ? after[i][hr] : new_max;
         float tile_sum = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
@@ -149,27 +183,54 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
         }
         tile_sum += __shfl_xor_sync(0xffffffffu, tile_sum, 1);
         tile_sum += __shfl_xor_sync(0xffffffffu, tile_sum, 2);
-        row_sum[hr] = row_sum[hr] * rescale + tile_sum;
-        row_max[hr] = new_max;
-#pragma unroll
-        for (int nt = 0; nt < 2 * HD16; ++nt) {
-          out[nt][2 * hr] *= rescale;
-          out[nt][2 * hr + 1] *= rescale;
-        }
+        if (t == 0) sums[(group * kTiles + own) * 16 + g + hr * 8] = tile_sum;
       }
-      // O += P (16 x 64 keys) . V (64 keys x head_dim): per 16 keys and 8 dims one MMA; ldmatrix with transpose
-      // turns two 8 x 8 blocks of row-major V into the B fragment
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-        for (int nt = 0; nt < 2 * HD16; ++nt) {
-          const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(v_tile + (kk * 16 + (lane & 15)) * pitch + nt * 8));
-          unsigned b0, b1;
-          asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
-          skinny_mma_bf16(out[nt], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b0, b1);
-        }
+        p_frag[((group * kTiles + own) * 4 + kk) * 32 + lane] = make_uint4(pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3]);
     }
-    __syncthreads();   // everyone is done with this buffer before it is refilled
+    asm volatile("cp.async.wait_group 1;" ::: "memory");   // V of this chunk
+    __syncthreads();
+
+    // O += P (16 x 64 keys) . V (64 keys x this warp's columns), tile after tile; ldmatrix with transpose turns 8 x 8
+    // blocks of row-major V into B fragments, two 16-key steps at a time
+#pragma unroll
+    for (unsigned i = 0; i < kTiles; ++i) {
+      if (!visits(first + i)) continue;
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const float rescale = after[i][hr] > -1.0e38f ? __expf(before[i][hr] - after[i][hr]) : 1.f;
+        row_sum[hr] = row_sum[hr] * rescale + sums[(group * kTiles + i) * 16 + g + hr * 8];
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          out[c][2 * hr] *= rescale;
+          out[c][2 * hr + 1] *= rescale;
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; kk += 2) {
+        const uint4 pa = p_frag[((group * kTiles + i) * 4 + kk) * 32 + lane], pb = p_frag[((group * kTiles + i) * 4 + kk + 1) * 32 + lane];
+        unsigned b[kCols][4];
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          const unsigned nt = own + c * kTiles;
+          if (nt >= 2 * HD16) continue;
+          const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(v_chunk + (i * kKeyTile + kk * 16 + lane) * pitch + nt * 8));
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(b[c][0]), "=r"(b[c][1]), "=r"(b[c][2]), "=r"(b[c][3]) : "r"(addr));
+        }
+#pragma unroll
+        for (int c = 0; c < kCols; ++c)
+          if (own + c * kTiles < 2 * HD16) skinny_mma_bf16(out[c], pa.x, pa.y, pa.z, pa.w, b[c][0], b[c][1]);
+#pragma unroll
+        for (int c = 0; c < kCols; ++c)
+          if (own + c * kTiles < 2 * HD16) skinny_mma_bf16(out[c], pb.x, pb.y, pb.z, pb.w, b[c][2], b[c][3]);
+      }
+    }
+    if (more) {
+      __syncthreads();                                     // V, P, sums and maxima are free
+      stage(v_chunk, v, v_stride, first + kTiles);
+    }
   }
 
   float best = 0.f;   // max |o| over this thread's outputs, for a following dynamic quantisation
@@ -180,8 +241,10 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
     const float inv = row_sum[hr] > 0.f ? 1.f / row_sum[hr] : 0.f;
     bf16* dst = o + size_t(row) * o_stride + head * head_dim + 2 * t;
 #pragma unroll
-    for (int nt = 0; nt < 2 * HD16; ++nt) {
-      const float a = out[nt][2 * hr] * inv, b = out[nt][2 * hr + 1] * inv;
+    for (int c = 0; c < kCols; ++c) {
+      const unsigned nt = own + c * kTiles;
+      if (nt >= 2 * HD16) continue;
+      const float a = out[c][2 * hr] * inv, b = out[c][2 * hr + 1] * inv;
       best = fmaxf(best, fmaxf(fabsf(a), fabsf(b)));
       *reinterpret_cast<bf162*>(dst + nt * 8) = __floats2bfloat162_rn(a, b);
     }
@@ -196,7 +259,7 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
 }  // namespace fa
 
 #define AGI_ATTENTION_FA(NAME, HD16)                                                                                 \
-  extern "C" __global__ void __launch_bounds__(128)                                                                  \
+  extern "C" __global__ void __launch_bounds__(256)                                                                  \
   NAME(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows, unsigned kv_rows, unsigned q_heads,    \
        unsigned kv_heads, unsigned head_dim, unsigned q_stride, unsigned k_stride, unsigned v_stride,               \
        unsigned o_stride, float scale, unsigned mask_mode, unsigned mask_arg) {                                      \
@@ -205,7 +268,7 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
   }
 // the same, also folding max |o| into *amax_bits (a zero-initialised word)
 #define AGI_ATTENTION_FA_AMAX(NAME, HD16)                                                                            \
-  extern "C" __global__ void __launch_bounds__(128)                                                                  \
+  extern "C" __global__ void __launch_bounds__(256)                                                                  \
   NAME(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows, unsigned kv_rows, unsigned q_heads,    \
        unsigned kv_heads, unsigned head_dim, unsigned q_stride, unsigned k_stride, unsigned v_stride,               \
        unsigned o_stride, float scale, unsigned mask_mode, unsigned mask_arg, unsigned* amax_bits) {                 \

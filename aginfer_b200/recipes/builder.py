@@ -647,20 +647,18 @@ class RecipeBuilder:
                         shared_bytes=wide_smem, op=f"attention_{mask}",
                         algorithm="mma_key_split_d128" + ("_early_kv" if kv_static else ""))
             return
-        # streaming tensor-core kernel: 4, 2 or 1 warps (64, 32 or 16 query rows) per block, the most rows that still
-        # give the grid about one block per SM
-        fa_warps = next((wp for wp in (4, 2, 1) if ceil_div(q_rows, 16 * wp) * q_heads >= 96), 1)
+        fa_grid, fa_smem = (ceil_div(q_rows, 32), q_heads, 1), 4 * 256 * (head_dim + 8) + 17408
         if amax is not None:
             assert aligned and head_dim in (80, 128) and q_stride % 2 == 0 and o_stride % 2 == 0 and (q_rows > 64 or head_dim > 64)
-            self.launch(f"agi_attention_fa_amax_bf16_d{head_dim}", (ceil_div(q_rows, 16 * fa_warps), q_heads, 1), (32 * fa_warps, 1, 1),
-                        args + [amax], shared_bytes=4 * 64 * (head_dim + 8) * 2, op=f"attention_{mask}_amax",
+            self.launch(f"agi_attention_fa_amax_bf16_d{head_dim}", fa_grid, (256, 1, 1),
+                        args + [amax], shared_bytes=fa_smem, op=f"attention_{mask}_amax",
                         algorithm="mma_streaming")
             return
         if (aligned and head_dim in FA_HEAD_DIMS and q_stride % 2 == 0 and o_stride % 2 == 0
                 and algorithm in ("auto", "fa")):
-            # many query rows: streaming softmax on tensor cores, 64 rows per block, keys in tiles of 64
-            self.launch(f"agi_attention_fa_bf16_d{head_dim}", (ceil_div(q_rows, 16 * fa_warps), q_heads, 1), (32 * fa_warps, 1, 1), args,
-                        shared_bytes=4 * 64 * (head_dim + 8) * 2, op=f"attention_{mask}", algorithm="mma_streaming")
+            # many query rows: streaming softmax on tensor cores, 32 rows per block, keys in chunks of four tiles of 64
+            self.launch(f"agi_attention_fa_bf16_d{head_dim}", fa_grid, (256, 1, 1), args,
+                        shared_bytes=fa_smem, op=f"attention_{mask}", algorithm="mma_streaming")
             return
         if (aligned and q_rows <= 32 and head_dim <= 64 and rows_smem <= ATTN_SMEM_BUDGET
                 and algorithm in ("auto", "key_split")):
