@@ -19,7 +19,7 @@
 // Head width is a template parameter (16-element steps); grouped-query attention maps query head h to KV
 // head h / (q_heads / kv_heads).  Pitch of the shared tiles = head_dim + 8 elements: rows stay 16-byte
 // aligned and the eight rows of a fragment fall into different banks.
-// grid = (ceil(q_rows / 32), q_heads), block = 256, dynamic shared memory = 4 * 256 * (head_dim + 8) + 17408.
+// grid = (ceil(q_rows / 32), q_heads), block = 256, dynamic shared memory = (4 * 256 + 64) * (head_dim + 8) + 17408.
 #pragma once
 
 #include "attention.cuh"
@@ -41,6 +41,8 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
   uint4* p_frag = reinterpret_cast<uint4*>(v_chunk + kChunk * pitch);         // [2 groups][4 tiles][4 16-key steps][32 lanes]
   float* maxima = reinterpret_cast<float*>(p_frag + 2 * kTiles * 4 * 32);     // [2][4][16 rows]
   float* sums = maxima + 2 * kTiles * 16;                                     // [2][4][16]
+  bf16* q_rows_smem = reinterpret_cast<bf16*>(sums + 2 * kTiles * 16);        // [32][pitch]
+  const bool q_vec = q_stride % 8 == 0 && (reinterpret_cast<size_t>(q) & 15) == 0;
   grid_dependency_wait();
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const unsigned group = warp / kTiles, own = warp % kTiles;                  // row group; tile (then columns) of this warp
@@ -69,30 +71,38 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // does this group of rows see anything of a tile?
-  auto visits = [&](unsigned tile) {
-    const unsigned key0 = key_begin + tile * kKeyTile;
-    bool any = tile < tiles_total && warp_row < q_rows;
-    if (mask_mode == 1) any = any && key0 <= warp_last + mask_arg;
-    if (mask_mode == 2) any = any && key0 < (warp_last / mask_arg + 1) * mask_arg && key0 + kKeyTile > (warp_row / mask_arg) * mask_arg;
-    return any;
+  // keys a row sees: [lo, hi); those of the group run from its first row's lo to its last row's hi
+  auto lo_of = [&](unsigned row) { return mask_mode == 2 ? row / mask_arg * mask_arg : 0u; };
+  auto hi_of = [&](unsigned row) {
+    return mask_mode == 1 ? min(kv_rows, row + mask_arg + 1) : mask_mode == 2 ? min(kv_rows, (row / mask_arg + 1) * mask_arg) : kv_rows;
   };
+  const unsigned group_lo = lo_of(warp_row), group_hi = warp_row < q_rows ? hi_of(warp_last) : 0u;
+  auto visits = [&](unsigned tile) {   // does this group of rows see anything of a tile?
+    const unsigned key0 = key_begin + tile * kKeyTile;
+    return tile < tiles_total && key0 < group_hi && key0 + kKeyTile > group_lo;
+  };
+  // Q as stored (zero past q_rows), with the first keys; the softmax scale is applied to the fp32 scores, so no second
+  // rounding of Q.
+  if (q_vec) {
+    for (unsigned i = threadIdx.x; i < kRows * vec_per_row; i += kThreads) {
+      const unsigned j = i / vec_per_row, d = (i % vec_per_row) * 8, row = min(row_base + j, q_rows - 1);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                       static_cast<unsigned>(__cvta_generic_to_shared(q_rows_smem + j * pitch + d))),
+                   "l"(q + size_t(row) * q_stride + head * head_dim + d), "r"(row_base + j < q_rows ? 16u : 0u) : "memory");
+    }
+  } else {
+    for (unsigned i = threadIdx.x; i < kRows * head_dim / 2; i += kThreads) {
+      const unsigned j = i / (head_dim / 2), d = (i % (head_dim / 2)) * 2, row = min(row_base + j, q_rows - 1);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                       static_cast<unsigned>(__cvta_generic_to_shared(q_rows_smem + j * pitch + d))),
+                   "l"(q + size_t(row) * q_stride + head * head_dim + d), "r"(row_base + j < q_rows ? 4u : 0u) : "memory");
+    }
+  }
   stage(k_chunk, k, k_stride, 0);
   stage(v_chunk, v, v_stride, 0);
 
-  // Q fragments (A operand) as stored: rows g and g + 8 of this group's 16; zero past q_rows.  The softmax
-  // scale is applied to the fp32 scores, so no second rounding of Q.
+  const unsigned lo[2] = {lo_of(warp_row + g), lo_of(warp_row + g + 8)}, hi[2] = {hi_of(warp_row + g), hi_of(warp_row + g + 8)};
   unsigned qa[HD16][4];
-#pragma unroll
-  for (int ks = 0; ks < HD16; ++ks)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      qa[ks][r] = 0;
-      const unsigned row = warp_row + g + (r & 1) * 8, col = ks * 16 + 2 * t + (r >> 1) * 8;
-      if (row < q_rows) {
-        qa[ks][r] = *reinterpret_cast<const unsigned*>(q + size_t(row) * q_stride + head * head_dim + col);
-      }
-    }
 
   float row_max[2] = {-3.0e38f, -3.0e38f}, row_sum[2] = {0.f, 0.f}, out[kCols][4];
 #pragma unroll
@@ -104,6 +114,13 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
     const bool more = first + kTiles < tiles_total;
     asm volatile("cp.async.wait_group 1;" ::: "memory");   // K of this chunk (V may still be under way)
     __syncthreads();
+    if (first == 0) {   // Q fragments (A operand): rows g and g + 8 of this group's 16
+      const unsigned q_addr = static_cast<unsigned>(__cvta_generic_to_shared(q_rows_smem + (group * 16 + (lane & 15)) * pitch + (lane >> 4) * 8));
+#pragma unroll
+      for (int ks = 0; ks < HD16; ++ks)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(qa[ks][0]), "=r"(qa[ks][1]), "=r"(qa[ks][2]), "=r"(qa[ks][3]) : "r"(q_addr + ks * 32));
+    }
 
     // scores of this warp's tile, masked, and their row maxima
     const bool any = visits(first + own);
@@ -130,10 +147,8 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const unsigned key = key0 + nt * 8 + 2 * t + (i & 1), row = warp_row + g + (i >> 1) * 8;
-          bool visible = key < kv_rows;
-          if (mask_mode == 1) visible = visible && key <= row + mask_arg;
-          if (mask_mode == 2) visible = visible && key / mask_arg == row / mask_arg;
+          const unsigned key = key0 + nt * 8 + 2 * t + (i & 1);
+          const bool visible = key >= lo[i >> 1] && key < hi[i >> 1];
           s[nt][i] = visible ? s[nt][i] * scale : -3.0e38f;
         }
 #pragma unroll
@@ -150,26 +165,14 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
     if (more) stage(k_chunk, k, k_stride, first + kTiles);
     else asm volatile("cp.async.commit_group;" ::: "memory");
 
-    // running maximum before and after every tile, as a walk over the tiles would meet them
-    float before[kTiles][2], after[kTiles][2];
-#pragma unroll
-    for (int hr = 0; hr < 2; ++hr) {
-      float m = row_max[hr];
-#pragma unroll
-      for (unsigned i = 0; i < kTiles; ++i) {
-        before[i][hr] = m;
-        if (visits(first + i)) m = fmaxf(m, maxima[(group * kTiles + i) * 16 + g + hr * 8]);
-        after[i][hr] = m;
-      }
-      row_max[hr] = m;
-    }
     if (any) {
       unsigned pa[4][4];   // [16-key step][a0..a3]
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
-        float new_max = after[0][hr];
+        float new_max = row_max[hr];   // the running maximum a walk over the tiles would have after this one
 #pragma unroll
-        for (unsigned i = 1; i < kTiles; ++i) new_max = own == i ? after[i][hr] : new_max;
+        for (unsigned i = 0; i < kTiles; ++i)
+          if (i <= own && visits(first + i)) new_max = fmaxf(new_max, maxima[(group * kTiles + i) * 16 + g + hr * 8]);
         float tile_sum = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
@@ -194,12 +197,14 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
 
     // O += P (16 x 64 keys) . V (64 keys x this warp's columns), tile after tile; ldmatrix with transpose turns 8 x 8
     // blocks of row-major V into B fragments, two 16-key steps at a time
-#pragma unroll
+#pragma unroll 1
     for (unsigned i = 0; i < kTiles; ++i) {
       if (!visits(first + i)) continue;
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
-        const float rescale = after[i][hr] > -1.0e38f ? __expf(before[i][hr] - after[i][hr]) : 1.f;
+        const float new_max = fmaxf(row_max[hr], maxima[(group * kTiles + i) * 16 + g + hr * 8]);
+        const float rescale = new_max > -1.0e38f ? __expf(row_max[hr] - new_max) : 1.f;
+        row_max[hr] = new_max;
         row_sum[hr] = row_sum[hr] * rescale + sums[(group * kTiles + i) * 16 + g + hr * 8];
 #pragma unroll
         for (int c = 0; c < kCols; ++c) {

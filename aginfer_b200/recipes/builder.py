@@ -114,8 +114,10 @@ def tc_tiling(M: int, N: int, K: int, elem: int, splits: int | None = None) -> d
 # ---- tensor-core GEMM with tokens as the MMA's A operand (csrc/kernels/gemm_tk.cuh) ------------------------
 TK_SMEM_BUDGET = 226 * 1024
 TK_PAIR_BUDGET = 112 * 1024                       # shared memory of a CTA that shares its SM with another
-# CTAs in whole clusters that the GPCs hold, one CTA per SM
-TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 135, 4: 132, 5: 130, 6: 132, 8: 120}
+# CTAs in whole clusters that the GPCs hold, one CTA per SM (3: 135, 4: 132, 5: 130, 6: 132, 8: 120).  Behind a launch
+# that is still draining, clusters of 3, 5 and 6 find their SMs in pieces and the last of a full part's clusters starts
+# a round late: the planner leaves them room (288 tokens x 2048 x 11008 in runs of 3: 33 us at 135 CTAs, 20 us below 120).
+TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 120, 4: 132, 5: 120, 6: 120, 8: 120}
 TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3, 4, 5, 6, 8), "agi_gemm_tc_e4m3_x3": (1, 2, 4, 8),
                "agi_gemm_tcpk_e4m3": (1, 2, 3, 4, 6, 8), "agi_gemm_tc_bf16_x3": (1, 2, 4, 8)}
 TK_MAX_RING = 8
@@ -647,7 +649,7 @@ class RecipeBuilder:
                         shared_bytes=wide_smem, op=f"attention_{mask}",
                         algorithm="mma_key_split_d128" + ("_early_kv" if kv_static else ""))
             return
-        fa_grid, fa_smem = (ceil_div(q_rows, 32), q_heads, 1), 4 * 256 * (head_dim + 8) + 17408
+        fa_grid, fa_smem = (ceil_div(q_rows, 32), q_heads, 1), (4 * 256 + 64) * (head_dim + 8) + 17408
         if amax is not None:
             assert aligned and head_dim in (80, 128) and q_stride % 2 == 0 and o_stride % 2 == 0 and (q_rows > 64 or head_dim > 64)
             self.launch(f"agi_attention_fa_amax_bf16_d{head_dim}", fa_grid, (256, 1, 1),
