@@ -2,31 +2,40 @@
 // tower: 512 patch tokens, 80-wide heads, block-diagonal windows).  Streaming-softmax formulation on
 // warp-level MMAs, parallel over rows, keys and output columns:
 //
-//   * one block of 8 warps per (32 query rows, head); warps form two groups of 16 rows, four warps each;
-//   * keys are visited in chunks of four 64-key tiles, staged row-major in shared memory by 16-byte
-//     asynchronous copies (K of the next chunk lands while P.V of this one runs);
+//   * one block per (32 query rows, head): two groups of 16 rows, a warp per group and key tile, two loading warps;
+//   * keys are visited in chunks of four or five 64-key tiles, staged row-major in shared memory by 16-byte
+//     asynchronous copies: K by all warps, V by the loading warps while the others multiply Q with K (issuing the
+//     copies takes as long as the bytes do, 35 B per clock, so V behind K in the same warps delayed the scores by 2 us);
 //   * each warp of a group multiplies Q with one tile's keys, masks, and leaves the tile's row maxima in shared
 //     memory; from the maxima of the tiles before it every warp knows the running maximum its tile would have met,
 //     so it forms P = exp(S - m) and the tile's row sums at once and leaves them in shared memory too;
-//   * each warp then adds P.V of the four tiles, in order and with the streaming formulation's rescaling between
-//     them, for a quarter of the head's columns: per output the same operations in the same order as one warp
+//   * each warp then adds P.V of the chunk's tiles, in order and with the streaming formulation's rescaling between
+//     them, for its share of the head's columns: per output the same operations in the same order as one warp
 //     walking the tiles one by one, which is what this replaced;
 //   * only key tiles a block of rows can see are visited: the causal prefix, or the diagonal block(s).
 //
-// What bounds it: the chain of dependent steps per tile, not bytes or tensor cores, so the tiles of a chunk run
-// side by side and each MMA chain has seven others to hide behind (the depth loop is outermost).
+// What bounds it: a chain of loading K, scores, P, P.V of about 2000 clocks each; scores and P.V run at the rate of the
+// warp-level MMA (16 clocks each per scheduler).  288 causal tokens, 16 heads of 128:
+// 12 us with 16 rows a warp and the tiles one after the other, now 8.3; 512 patches, windows of 64, 16 heads of 80:
+// 11 us, now 6.
 //
 // Head width is a template parameter (16-element steps); grouped-query attention maps query head h to KV
 // head h / (q_heads / kv_heads).  Pitch of the shared tiles = head_dim + 8 elements: rows stay 16-byte
 // aligned and the eight rows of a fragment fall into different banks.
-// grid = (ceil(q_rows / 32), q_heads), block = 256, dynamic shared memory = (4 * 256 + 64) * (head_dim + 8) + 17408.
+// grid = (ceil(q_rows / 32), q_heads), block = 64 * tiles + 64,
+// dynamic shared memory = (256 * tiles + 64) * (head_dim + 8) + 4352 * tiles.
 #pragma once
 
 #include "attention.cuh"
 
 namespace fa {
 
-constexpr unsigned kKeyTile = 64, kTiles = 4, kChunk = kKeyTile * kTiles, kRows = 32, kThreads = 256;
+constexpr unsigned kKeyTile = 64, kRows = 32, kLoaders = 64;
+template <int HD16>
+struct Shape {
+  static constexpr unsigned kTiles = HD16 == 8 ? 5 : 4;                        // 128-wide heads: 320 keys, one block per SM
+  static constexpr unsigned kCompute = kTiles * 64, kThreads = kCompute + kLoaders, kPerSm = HD16 == 8 ? 1 : 2;
+};
 
 template <int HD16>
 __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows,
@@ -34,13 +43,16 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
                                                unsigned k_stride, unsigned v_stride, unsigned o_stride, float scale,
                                                unsigned mask_mode, unsigned mask_arg, unsigned* amax_bits = nullptr) {
   constexpr unsigned head_dim = HD16 * 16, pitch = head_dim + 8, vec_per_row = head_dim / 8;
+  constexpr unsigned kTiles = Shape<HD16>::kTiles, kChunk = kKeyTile * kTiles, kCompute = Shape<HD16>::kCompute;
   constexpr int kCols = (2 * HD16 + int(kTiles) - 1) / int(kTiles);   // 8-column output tiles of a warp, the last may be absent
+  auto block_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(Shape<HD16>::kThreads) : "memory"); };   // of both kinds of warps
+  auto compute_sync = [] { asm volatile("bar.sync 2, %0;" ::"n"(Shape<HD16>::kCompute) : "memory"); };
   extern __shared__ __align__(16) unsigned char attn_smem[];
-  bf16* k_chunk = reinterpret_cast<bf16*>(attn_smem);                         // [256][pitch]
-  bf16* v_chunk = k_chunk + kChunk * pitch;                                   // [256][pitch]
-  uint4* p_frag = reinterpret_cast<uint4*>(v_chunk + kChunk * pitch);         // [2 groups][4 tiles][4 16-key steps][32 lanes]
-  float* maxima = reinterpret_cast<float*>(p_frag + 2 * kTiles * 4 * 32);     // [2][4][16 rows]
-  float* sums = maxima + 2 * kTiles * 16;                                     // [2][4][16]
+  bf16* k_chunk = reinterpret_cast<bf16*>(attn_smem);                         // [chunk][pitch]
+  bf16* v_chunk = k_chunk + kChunk * pitch;                                   // [chunk][pitch]
+  uint4* p_frag = reinterpret_cast<uint4*>(v_chunk + kChunk * pitch);         // [2 groups][tiles][4 16-key steps][32 lanes]
+  float* maxima = reinterpret_cast<float*>(p_frag + 2 * kTiles * 4 * 32);     // [2][tiles][16 rows]
+  float* sums = maxima + 2 * kTiles * 16;                                     // [2][tiles][16]
   bf16* q_rows_smem = reinterpret_cast<bf16*>(sums + 2 * kTiles * 16);        // [32][pitch]
   const bool q_vec = q_stride % 8 == 0 && (reinterpret_cast<size_t>(q) & 15) == 0;
   grid_dependency_wait();
@@ -59,10 +71,10 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
   }
   const unsigned tiles_total = key_end > key_begin ? (key_end - key_begin + kKeyTile - 1) / kKeyTile : 0;
 
-  auto stage = [&](bf16* dst, const bf16* src, unsigned stride, unsigned first_tile) {   // up to four tiles, one commit group
+  auto stage = [&](bf16* dst, const bf16* src, unsigned stride, unsigned first_tile, unsigned thread, unsigned threads) {
     const unsigned keys = first_tile < tiles_total ? min(tiles_total - first_tile, kTiles) * kKeyTile : 0;
     const unsigned key0 = key_begin + first_tile * kKeyTile;
-    for (unsigned i = threadIdx.x; i < keys * vec_per_row; i += kThreads) {
+    for (unsigned i = thread; i < keys * vec_per_row; i += threads) {
       const unsigned j = i / vec_per_row, d = (i % vec_per_row) * 8;
       const unsigned key = key0 + j, src_row = min(key, kv_rows - 1), bytes = key < kv_rows ? 16u : 0u;  // zero-fill past the end
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
@@ -81,25 +93,34 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
     const unsigned key0 = key_begin + tile * kKeyTile;
     return tile < tiles_total && key0 < group_hi && key0 + kKeyTile > group_lo;
   };
+  if (warp >= 2 * kTiles) {   // loading warps: V of a chunk while the others multiply its K
+    for (unsigned first = 0; first < tiles_total; first += kTiles) {
+      block_sync();                                     // K has landed: V has the memory path to itself
+      stage(v_chunk, v, v_stride, first, threadIdx.x - kCompute, kLoaders);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      block_sync();
+      if (first + kTiles < tiles_total) block_sync();
+    }
+    return;
+  }
   // Q as stored (zero past q_rows), with the first keys; the softmax scale is applied to the fp32 scores, so no second
   // rounding of Q.
   if (q_vec) {
-    for (unsigned i = threadIdx.x; i < kRows * vec_per_row; i += kThreads) {
+    for (unsigned i = threadIdx.x; i < kRows * vec_per_row; i += kCompute) {
       const unsigned j = i / vec_per_row, d = (i % vec_per_row) * 8, row = min(row_base + j, q_rows - 1);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
                        static_cast<unsigned>(__cvta_generic_to_shared(q_rows_smem + j * pitch + d))),
                    "l"(q + size_t(row) * q_stride + head * head_dim + d), "r"(row_base + j < q_rows ? 16u : 0u) : "memory");
     }
   } else {
-    for (unsigned i = threadIdx.x; i < kRows * head_dim / 2; i += kThreads) {
+    for (unsigned i = threadIdx.x; i < kRows * head_dim / 2; i += kCompute) {
       const unsigned j = i / (head_dim / 2), d = (i % (head_dim / 2)) * 2, row = min(row_base + j, q_rows - 1);
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
                        static_cast<unsigned>(__cvta_generic_to_shared(q_rows_smem + j * pitch + d))),
                    "l"(q + size_t(row) * q_stride + head * head_dim + d), "r"(row_base + j < q_rows ? 4u : 0u) : "memory");
     }
   }
-  stage(k_chunk, k, k_stride, 0);
-  stage(v_chunk, v, v_stride, 0);
+  stage(k_chunk, k, k_stride, 0, threadIdx.x, kCompute);
 
   const unsigned lo[2] = {lo_of(warp_row + g), lo_of(warp_row + g + 8)}, hi[2] = {hi_of(warp_row + g), hi_of(warp_row + g + 8)};
   unsigned qa[HD16][4];
@@ -112,8 +133,8 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
 
   for (unsigned first = 0; first < tiles_total; first += kTiles) {
     const bool more = first + kTiles < tiles_total;
-    asm volatile("cp.async.wait_group 1;" ::: "memory");   // K of this chunk (V may still be under way)
-    __syncthreads();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // K of this chunk
+    block_sync();
     if (first == 0) {   // Q fragments (A operand): rows g and g + 8 of this group's 16
       const unsigned q_addr = static_cast<unsigned>(__cvta_generic_to_shared(q_rows_smem + (group * 16 + (lane & 15)) * pitch + (lane >> 4) * 8));
 #pragma unroll
@@ -161,9 +182,8 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
         if (t == 0) maxima[(group * kTiles + own) * 16 + g + hr * 8] = tile_max;
       }
     }
-    __syncthreads();                                       // maxima are there, K is no longer needed
-    if (more) stage(k_chunk, k, k_stride, first + kTiles);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
+    compute_sync();                                     // maxima are there, K is no longer needed
+    if (more) stage(k_chunk, k, k_stride, first + kTiles, threadIdx.x, kCompute);
 
     if (any) {
       unsigned pa[4][4];   // [16-key step][a0..a3]
@@ -177,8 +197,8 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
           const float s0 = s[nt][2 * hr], s1 = s[nt][2 * hr + 1];
-          const float p0 = s0 > -1.0e38f ? __expf(s0 - new_max) : 0.f;
-          const float p1 = s1 > -1.0e38f ? __expf(s1 - new_max) : 0.f;
+          const float e0 = __expf(s0 - new_max), e1 = __expf(s1 - new_max);
+          const float p0 = s0 > -1.0e38f ? e0 : 0.f, p1 = s1 > -1.0e38f ? e1 : 0.f;
           tile_sum += p0 + p1;
           const bf162 pair = __floats2bfloat162_rn(p0, p1);
           // A operand of P.V for 16-key step nt / 2: a0/a1 = rows g / g + 8 of the first 8 keys, a2/a3 of the second
@@ -192,8 +212,7 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
       for (int kk = 0; kk < 4; ++kk)
         p_frag[((group * kTiles + own) * 4 + kk) * 32 + lane] = make_uint4(pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3]);
     }
-    asm volatile("cp.async.wait_group 1;" ::: "memory");   // V of this chunk
-    __syncthreads();
+    block_sync();                                       // P, sums and V of this chunk are there
 
     // O += P (16 x 64 keys) . V (64 keys x this warp's columns), tile after tile; ldmatrix with transpose turns 8 x 8
     // blocks of row-major V into B fragments, two 16-key steps at a time
@@ -232,12 +251,10 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
           if (own + c * kTiles < 2 * HD16) skinny_mma_bf16(out[c], pb.x, pb.y, pb.z, pb.w, b[c][2], b[c][3]);
       }
     }
-    if (more) {
-      __syncthreads();                                     // V, P, sums and maxima are free
-      stage(v_chunk, v, v_stride, first + kTiles);
-    }
+    if (more) block_sync();                             // V, P, sums and maxima are free
   }
 
+  if (tiles_total == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");   // Q is under way
   float best = 0.f;   // max |o| over this thread's outputs, for a following dynamic quantisation
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
@@ -264,7 +281,7 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
 }  // namespace fa
 
 #define AGI_ATTENTION_FA(NAME, HD16)                                                                                 \
-  extern "C" __global__ void __launch_bounds__(256)                                                                  \
+  extern "C" __global__ void __launch_bounds__(fa::Shape<HD16>::kThreads, fa::Shape<HD16>::kPerSm)                                                                  \
   NAME(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows, unsigned kv_rows, unsigned q_heads,    \
        unsigned kv_heads, unsigned head_dim, unsigned q_stride, unsigned k_stride, unsigned v_stride,               \
        unsigned o_stride, float scale, unsigned mask_mode, unsigned mask_arg) {                                      \
@@ -273,7 +290,7 @@ __device__ __forceinline__ void attention_body(const bf16* q, const bf16* k, con
   }
 // the same, also folding max |o| into *amax_bits (a zero-initialised word)
 #define AGI_ATTENTION_FA_AMAX(NAME, HD16)                                                                            \
-  extern "C" __global__ void __launch_bounds__(256)                                                                  \
+  extern "C" __global__ void __launch_bounds__(fa::Shape<HD16>::kThreads, fa::Shape<HD16>::kPerSm)                                                                  \
   NAME(const bf16* q, const bf16* k, const bf16* v, bf16* o, unsigned q_rows, unsigned kv_rows, unsigned q_heads,    \
        unsigned kv_heads, unsigned head_dim, unsigned q_stride, unsigned k_stride, unsigned v_stride,               \
        unsigned o_stride, float scale, unsigned mask_mode, unsigned mask_arg, unsigned* amax_bits) {                 \

@@ -112,6 +112,11 @@ __device__ __forceinline__ float e4m3_to_float(uint8_t b) {
 }
 // Round-to-nearest-even, saturating to +-448 (never NaN for finite input).
 __device__ __forceinline__ uint8_t float_to_e4m3(float x) { return __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3); }
+// four of them, the first in the lowest byte; two values per conversion
+__device__ __forceinline__ unsigned float4_to_e4m3x4(float a, float b, float c, float d) {
+  return unsigned(__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3)) |
+         unsigned(__nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3)) << 16;
+}
 
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float inner = 0.7978845608028654f * (x + 0.044715f * x * x * x);

@@ -518,18 +518,20 @@ class RecipeBuilder:
         when the producer of ``x`` already folded max |x| into ``amax`` (a ``counter()`` slot).
         ``packed=(rows, cols)`` writes ``q`` in the packed operand layout of the bulk-copy GEMM
         (``recipes/layout.py``; ``q`` needs ``padded_token_rows(rows) * cols`` bytes)."""
-        blocks = grid_for(count // 8 + 1, 256, SM_COUNT * 4)
+        # one thread per 8 values up to a full part of threads (a 288-token prefill: 760 us
+        # with half of them, 750)
+        grid = grid_for(count // 8 + 1, 256, SM_COUNT * 8)
         if amax is None:
             amax = self.counter()
-            self.launch("agi_absmax_bf16", (blocks, 1, 1), (256, 1, 1), [x, U32(count), amax], op="absmax")
+            self.launch("agi_absmax_bf16", (min(grid, SM_COUNT * 4), 1, 1), (256, 1, 1), [x, U32(count), amax], op="absmax")
         if packed is not None:
             rows, cols = packed
             assert rows * cols == count and cols % 128 == 0
-            self.launch("agi_quantize_e4m3_packed_bf16", (grid_for(count // 16, 256, SM_COUNT * 4), 1, 1), (256, 1, 1),
+            self.launch("agi_quantize_e4m3_packed_bf16", (grid, 1, 1), (256, 1, 1),
                         [x, q, amax, scale_out, U32(rows), U32(cols), U32(padded_token_rows(rows))],
                         op="quantize_e4m3_packed")
             return
-        self.launch("agi_quantize_e4m3_bf16", (blocks, 1, 1), (256, 1, 1), [x, q, amax, scale_out, U32(count)],
+        self.launch("agi_quantize_e4m3_bf16", (grid, 1, 1), (256, 1, 1), [x, q, amax, scale_out, U32(count)],
                     op="quantize_e4m3")
 
     def rmsnorm(self, x: Pointer, gain: Pointer, y: Pointer, rows: int, cols: int, eps: float = 1e-6,
@@ -649,17 +651,19 @@ class RecipeBuilder:
                         shared_bytes=wide_smem, op=f"attention_{mask}",
                         algorithm="mma_key_split_d128" + ("_early_kv" if kv_static else ""))
             return
-        fa_grid, fa_smem = (ceil_div(q_rows, 32), q_heads, 1), (4 * 256 + 64) * (head_dim + 8) + 17408
+        fa_tiles = 5 if head_dim == 128 else 4     # key tiles of a chunk; a compute warp per tile and 16 rows, two loading warps
+        fa_grid, fa_block = (ceil_div(q_rows, 32), q_heads, 1), (64 * fa_tiles + 64, 1, 1)
+        fa_smem = (256 * fa_tiles + 64) * (head_dim + 8) + fa_tiles * (4096 + 256)
         if amax is not None:
             assert aligned and head_dim in (80, 128) and q_stride % 2 == 0 and o_stride % 2 == 0 and (q_rows > 64 or head_dim > 64)
-            self.launch(f"agi_attention_fa_amax_bf16_d{head_dim}", fa_grid, (256, 1, 1),
+            self.launch(f"agi_attention_fa_amax_bf16_d{head_dim}", fa_grid, fa_block,
                         args + [amax], shared_bytes=fa_smem, op=f"attention_{mask}_amax",
                         algorithm="mma_streaming")
             return
         if (aligned and head_dim in FA_HEAD_DIMS and q_stride % 2 == 0 and o_stride % 2 == 0
                 and algorithm in ("auto", "fa")):
-            # many query rows: streaming softmax on tensor cores, 32 rows per block, keys in chunks of four tiles of 64
-            self.launch(f"agi_attention_fa_bf16_d{head_dim}", fa_grid, (256, 1, 1), args,
+            # many query rows: streaming softmax on tensor cores, 32 rows per block, keys in chunks of tiles of 64
+            self.launch(f"agi_attention_fa_bf16_d{head_dim}", fa_grid, fa_block, args,
                         shared_bytes=fa_smem, op=f"attention_{mask}", algorithm="mma_streaming")
             return
         if (aligned and q_rows <= 32 and head_dim <= 64 and rows_smem <= ATTN_SMEM_BUDGET

@@ -133,8 +133,7 @@ def build_recipe(cfg: LayerConfig, weights, gemm_tactic: str = "auto") -> Recipe
     act_amax = r.counter() if cfg.fp8 else None
     if grouped and S > 32:
         part = lambda name: (Weight(f"{L}.{name}.weight"), None, weight_scale(name))
-        r.gemm_swiglu(operand, part("mlp.gate_proj"), part("mlp.up_proj"), act, S, I, H, dtype=dtype, scale_a=scale_a,
-                      amax=act_amax, scratch=gate_up if S > 128 else None)
+        r.gemm_swiglu(operand, part("mlp.gate_proj"), part("mlp.up_proj"), act, S, I, H, dtype=dtype, scale_a=scale_a, amax=act_amax)
     else:
         linear(normed, "mlp.gate_proj", gate_up, I, H, ldy=2 * I)
         linear(normed, "mlp.up_proj", gate_up + I * BF, I, H, ldy=2 * I)
