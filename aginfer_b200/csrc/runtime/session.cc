@@ -398,6 +398,18 @@ Status Session::Replay(CUstream stream) {
   std::vector<CachedGraph>& graphs_ = active_->graphs;
   for (CachedGraph& g : graphs_)
     if (g.key == bound_) hit = &g;
+  if (hit == nullptr && !graphs_.empty()) {
+    // Another set of addresses: a caller who allocates for every call would pay a capture each time (2.5 us a launch and
+    // more), so the first pass over a set is launched one by one and only a set that comes back gets a graph.
+    std::vector<std::vector<void*>>& seen = active_->seen;
+    const auto again = std::find(seen.begin(), seen.end(), bound_);
+    if (again == seen.end()) {
+      if (seen.size() >= kMaxCachedGraphs) seen.erase(seen.begin());
+      seen.push_back(bound_);
+      return Issue(stream);
+    }
+    seen.erase(again);
+  }
   if (hit == nullptr) {
     // The legacy null stream cannot be captured (a graph can be launched into it): the launches are recorded on a
     // stream of the session's own.

@@ -7,7 +7,8 @@
 //   * a launch that asks for more than 48 KB of dynamic shared memory gets the function
 //     attribute that permits it;
 //   * for a profile the package marks as graph-safe, the recipe is stream-captured on the
-//     caller's stream at the first Enqueue for a given set of tensor addresses and replayed
+//     caller's stream at the first Enqueue (for further sets of tensor addresses: the second
+//     time a set is passed; its first pass is issued launch by launch) and replayed
 //     with one graph launch afterwards (unless the caller is itself capturing, in which case
 //     launches are issued one by one as in the reference; for the legacy null stream, which
 //     cannot be captured, they are recorded on a stream of the session's own);
@@ -138,6 +139,7 @@ class Session {
     std::vector<CUfunction> functions;    // one per launch of the profile
     std::vector<bool> cooperative;        // per launch: kernel name starts with "agi_coop_"
     std::vector<CachedGraph> graphs;
+    std::vector<std::vector<void*>> seen; // address sets passed once since the first graph was built, oldest first
   };
   std::vector<std::unique_ptr<ProfileState>> states_;
   ProfileState* active_ = nullptr;
