@@ -506,15 +506,20 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     }
     tc_fence_before();
   }
+  // Tensor memory goes back before this CTA waits for another one.  tcgen05.alloc blocks until columns are free: if a
+  // CTA kept its columns across the cluster barrier, two clusters that share two SMs in opposite order would each hold
+  // what the other's missing rank waits for.  The epilogue warps only arrive (their partial tiles are in L2, every
+  // tcgen05.ld is complete) and do not wait for the release.
+  if (warp == kMmaWarp) {
+    asm volatile("bar.sync 2, %0;" ::"n"(kEpilogue + 32) : "memory");
+    tc_fence_after();
+    tmem_free(tmem_base, columns);
+  } else {
+    asm volatile("bar.arrive 2, %0;" ::"n"(kEpilogue + 32) : "memory");
+  }
   if (kCluster) {
     cluster_arrive();     // release: this rank's partial tiles are filed
     cluster_wait();
-  } else {
-    __syncthreads();
-  }
-  if (warp == kMmaWarp) {
-    tc_fence_after();
-    tmem_free(tmem_base, columns);
   }
   if (kCluster && warp < kMmaWarp) {
     // ---------------- this rank adds the runs of its share of the rows, in order, and finishes them ----------------
