@@ -103,12 +103,15 @@ __device__ __forceinline__ void body(const bf16* x, const Parts& parts, bf16* y,
       tc::bulk_copy(ring + i * kATile, w + (size_t(kb_begin + i) * rows_padded + n0) * 128, kATile, &weights_bar[i]);
     }
   }
+  // "This rank runs": said before tensor memory is asked for, which may block.  Paired with the wait just before the
+  // first remote store; a rank that holds its columns there must not depend on a peer that still lacks some.
+  __syncwarp();
+  if (kCluster > 1) tc::cluster_arrive();
   if (warp == 4) tc::tmem_alloc(&tmem_slot, kTokens * kAccumulators);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
   const unsigned tmem_base = tmem_slot;
-  if (kCluster > 1) tc::cluster_arrive();   // paired with the wait just before the first remote store
 
   grid_dependency_wait();
 

@@ -18,7 +18,7 @@ def body_events(name: str) -> list[str]:
     return [m.group(1) for m in EVENTS.finditer(source)]
 
 
-@pytest.mark.parametrize("name", ["gemm_tk.cuh", "gemm_tc.cuh", "gemm_tc_persist.cuh"])
+@pytest.mark.parametrize("name", ["gemm_tk.cuh", "gemm_tc.cuh", "gemm_tc_persist.cuh", "gemm_tcs.cuh"])
 def test_no_cta_waits_for_another_one_that_may_lack_tensor_memory(name):
     events = body_events(name)
     held = allocated = arrived_early = False
