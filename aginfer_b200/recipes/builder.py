@@ -192,6 +192,10 @@ def tk_tiling(M: int, widths: tuple[int, ...], K: int, elem: int, swiglu: bool =
     epilogue then overlap.  The constants are fitted to 30 000 timed tiles of 70 shapes (36 - 1024 tokens): the tile
     chosen is 3.5 % slower than the fastest one on average, 28 % at worst."""
     k_blocks = K * elem // 128
+    # Token groups of at most 512 rows (four MMA tiles), counted up from the fewest: to 16, or, beyond 4096 tokens, to
+    # groups of half that size, so that a tile with 256 weight rows or eight runs fits tensor memory at any M.
+    fewest = ceil_div(M, 512)
+    group_counts = range(fewest, max(16, 2 * fewest) + 1)
     best: dict[str, int] | None = None
     for budget, per_sm in ((TK_SMEM_BUDGET, 1), (TK_PAIR_BUDGET, 2)):
         for C in clusters:
@@ -205,7 +209,7 @@ def tk_tiling(M: int, widths: tuple[int, ...], K: int, elem: int, swiglu: bool =
                 out = NB // 2 if swiglu else NB
                 tiles = sum(ceil_div(n, out) for n in widths)
                 seen = set()
-                for groups in range(1, 17):
+                for groups in group_counts:
                     tg = ceil_div(ceil_div(M, groups), 8) * 8
                     if tg in seen or tg > 512 or (tg < 16 and M > 16):
                         continue

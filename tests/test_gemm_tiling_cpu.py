@@ -2,12 +2,14 @@
 function of the shape alone."""
 import pytest
 
+from aginfer_b200.recipes import RecipeBuilder, Tensor, qwen_vl
 from aginfer_b200.recipes.builder import TC_SCRATCH_BYTES, TK_CLUSTERS, k_runs, tk_tiling
+from aginfer_b200.recipes.package import describe
 
 SHAPES = [(16, 128), (130, 256), (2048, 2048), (11008, 2048), (2048, 11008), (3584, 18944), (151, 640)]
 
 
-@pytest.mark.parametrize("M", [33, 64, 65, 127, 128, 129, 288, 513, 1024])
+@pytest.mark.parametrize("M", [33, 64, 65, 127, 128, 129, 288, 513, 1024, 4097, 8192, 8193, 12000, 20000])
 @pytest.mark.parametrize("N,K", SHAPES)
 def test_tiles_stay_inside_the_kernels_limits(M, N, K):
     for elem in (1, 2):
@@ -23,3 +25,29 @@ def test_tiles_stay_inside_the_kernels_limits(M, N, K):
             last_slot = ring - (t["tg"] + t["NB"]) * 128
             assert 1024 + max(ring, last_slot + m_tiles * 16384) <= t["shared_bytes"] <= 227 * 1024
             assert t["C"] == 1 or t["tiles"] * t["groups"] * t["runs"] * t["NB"] * -(-t["tg"] // 32) * 128 <= TC_SCRATCH_BYTES
+
+
+@pytest.mark.parametrize("M", [8192, 8193, 8448, 30000])
+def test_products_of_many_rows_get_a_launch_from_every_entry_point(M):
+    N, K, y = 2048, 1280, Tensor("y")
+    r = RecipeBuilder({"w": ("BF16", [8])})
+    r.begin_profile("default", [], [])
+    before = r.launch_count()
+    for dtype in ("bf16", "e4m3"):
+        r.gemm(y, y, y, M, N, K, dtype=dtype)
+        r.gemm(y, y, y, M, N, K, dtype=dtype, tactic="tcgen05_wide")
+        r.gemm_group(y, [(y, None, None, y, N, N), (y, None, None, y, 256, 256)], M, K, dtype=dtype)
+        r.gemm_swiglu(y, (y, None, None), (y, None, None), y, M, N, K, dtype=dtype)
+    for tactic in ("auto", "persistent", "tcgen05_plan"):
+        r.gemm(y, y, y, M, N, K, dtype="e4m3", packed=True, tactic=tactic)
+    r.gemm_batch(y, [(y, y)] * 16, y, M, N, K, seg_stride=M * N)
+    assert r.launch_count() - before == 12
+
+
+def test_a_prefill_of_33_images_builds():
+    cfg = qwen_vl.VlConfig(images=33, text_tokens=8, v_layers=1, layers=1, vocab=64, v_full_layers=())
+    assert cfg.patches == 33 * 256
+    for packed in (False, True):
+        weights = qwen_vl.synthetic_weights(cfg)
+        r = qwen_vl.build_recipe(cfg, describe(qwen_vl.pack_checkpoint(weights) if packed else weights), packed=packed)
+        assert r.launch_count() > 20

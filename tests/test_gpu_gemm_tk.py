@@ -23,6 +23,15 @@ CASES = [
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c)))
 def test_gemm_tk_edges(tmp_path, case):
+    check_against_the_oracle(tmp_path, case)
+
+
+@pytest.mark.parametrize("kind", ["bf16", "e4m3", "packed"])
+def test_gemm_tk_of_more_than_8192_rows(tmp_path, kind):
+    check_against_the_oracle(tmp_path, (8201, 144, 256, kind, "bias_res"))
+
+
+def check_against_the_oracle(tmp_path, case):
     M, N, K, kind, epi = case
     g = torch.Generator().manual_seed(M + N + K)
     x, wf = torch.randn(M, K, generator=g).to(BF), torch.randn(N, K, generator=g) * 0.02
