@@ -181,10 +181,11 @@ def k_runs(M: int, N: int, K: int, elem: int, packed: bool = False) -> int:
 
 @functools.lru_cache(maxsize=4096)
 def tk_tiling(M: int, widths: tuple[int, ...], K: int, elem: int, swiglu: bool = False, runs: int | None = None,
-              clusters: tuple[int, ...] = (1, 2, 4, 8), rows_per_tile: int | None = None) -> Mapping[str, int]:
+              clusters: tuple[int, ...] = (1, 2, 4, 8), rows_per_tile: int | None = None,
+              must_fit: bool = True) -> Mapping[str, int] | None:
     """Tile of ``agi_gemm_tk_*`` for matrices of ``widths`` rows side by side over M tokens: weight rows ``NB``,
     token group ``tg``, cluster size ``C``, ring depth.  ``runs``: see ``k_runs``; None = one run per cluster rank,
-    whatever cluster is chosen.  ``rows_per_tile`` fixes NB.
+    whatever cluster is chosen.  ``rows_per_tile`` fixes NB.  ``must_fit=False``: None where no tile fits.
 
     Every CTA takes in NB weight rows and its tokens, and that intake sets the time, so the estimate per CTA is
     K blocks x max(intake at 57 B per clock, 650 cycles: what one SM's outstanding loads give) + set-up, epilogue and
@@ -240,7 +241,7 @@ def tk_tiling(M: int, widths: tuple[int, ...], K: int, elem: int, swiglu: bool =
                     if best is None or cost < best["cost"]:
                         best = {"C": C, "NB": NB, "tg": tg, "tiles": tiles, "groups": groups, "stages": stages, "runs": S,
                                 "per_run": per_run, "shared_bytes": shared, "cost": int(cost)}
-    assert best is not None, "no tile of the tensor-core GEMM fits"
+    assert best is not None or not must_fit, "no tile of the tensor-core GEMM fits"
     return best
 
 
@@ -810,8 +811,9 @@ class RecipeBuilder:
                     raise ValueError("cluster split-K needs M <= 64, whole 128-byte K blocks and a usable cluster size")
                 t = tk_tiling(M, (N,), K, elem, clusters=(max(n for n in (2, 4, 8) if n <= c["cluster"]),))
             elif tactic == "tcgen05_wide":
-                slices = max(n for n in (1, 2, 4, 8) if n == 1 or (n <= (splits or 1) and K * elem // 128 >= 2 * n))
-                t = tk_tiling(M, (N,), K, elem, clusters=(slices,), rows_per_tile=256)
+                # the most slices up to the number asked for that K can be cut into and the scratch holds
+                t = next(t for t in (tk_tiling(M, (N,), K, elem, clusters=(n,), rows_per_tile=256, must_fit=False)
+                                     for n in (8, 4, 2, 1) if n <= (splits or 1)) if t is not None)
             else:
                 runs = k_runs(M, N, K, elem) if fixed_order else None
                 clusters = TK_CLUSTERS[f"agi_gemm_tk_{dtype}"] if runs else (1, 2, 4, 8)

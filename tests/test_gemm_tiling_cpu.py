@@ -27,6 +27,16 @@ def test_tiles_stay_inside_the_kernels_limits(M, N, K):
             assert t["C"] == 1 or t["tiles"] * t["groups"] * t["runs"] * t["NB"] * -(-t["tg"] // 32) * 128 <= TC_SCRATCH_BYTES
 
 
+@pytest.mark.parametrize("M,N,K,splits,ranks", [(17, 1280, 1280, 8, 4), (128, 1280, 1152, 16, 4), (64, 152064, 2048, 2, 1),
+                                                (256, 2048, 2048, 8, 8), (300, 256, 1024, 3, 2), (600, 256, 64, 8, 1)])
+def test_tiles_of_256_rows_take_as_many_k_slices_as_can_be_made(M, N, K, splits, ranks):
+    r, y = RecipeBuilder({"w": ("BF16", [8])}), Tensor("y")
+    r.begin_profile("default", [], [])
+    r.gemm(y, y, y, M, N, K, tactic="tcgen05_wide", splits=splits)
+    launch = r.profiles[0].launches[-1]
+    assert launch["grid"][2] == ranks and launch["kernel"] == "agi_gemm_tk_bf16" + (f"_c{ranks}" if ranks > 1 else "")
+
+
 @pytest.mark.parametrize("M", [8192, 8193, 8448, 30000])
 def test_products_of_many_rows_get_a_launch_from_every_entry_point(M):
     N, K, y = 2048, 1280, Tensor("y")
