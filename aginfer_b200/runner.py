@@ -7,7 +7,6 @@ kernel comes from the AIM's CUBIN through the native loader.
 """
 from __future__ import annotations
 
-import weakref
 from collections import OrderedDict
 from pathlib import Path
 from typing import Mapping
@@ -34,7 +33,7 @@ class Runner:
         self.inputs = self.session.input_info()
         self.outputs = self.session.output_info()
         self._dtypes = {t.name: t.dtype for t in self.inputs + self.outputs}
-        self._bindings: OrderedDict = OrderedDict()    # tensor names and addresses -> (packed views, weak references, layouts)
+        self._bindings: OrderedDict = OrderedDict()    # tensor names and addresses -> (packed views, layouts)
         self._side = None
         self._replays = not flags & rt.NO_GRAPH_REPLAY
         # the raw handle of torch's current stream, without building a Stream object on every call
@@ -62,20 +61,17 @@ class Runner:
             options = rt.run_options(denoising_steps, view)
         key = (*inputs, *outputs, *[t.data_ptr() for t in inputs.values()], *[t.data_ptr() for t in outputs.values()])
         tensors = (*inputs.values(), *outputs.values())
+        # What the packed views say about a tensor beside its address, looked at on every call: a tensor can be given
+        # another shape or stride in place, and another one can stand at the same address.
+        layout = [(t.shape, t.stride(), t.dtype, t.storage_offset(), t.untyped_storage().nbytes()) for t in tensors]
         bound = self._bindings.get(key)
-        if bound is None or any(ref() is not t for ref, t in zip(bound[1], tensors)):
-            # another tensor at these addresses: the packed views still describe it if its layout is the same
-            layout = [(t.shape, t.stride(), t.dtype, t.untyped_storage().nbytes() - t.storage_offset() * t.element_size())
-                      for t in tensors]
-            if bound is not None and bound[2] == layout:
-                packed = bound[0]
-            else:
-                packed = self.session.bind(
-                    [rt.TensorView.from_torch(n, t, self._dtypes.get(n)) for n, t in inputs.items()],
-                    [rt.TensorView.from_torch(n, t, self._dtypes.get(n)) for n, t in outputs.items()])
+        if bound is None or bound[1] != layout:
+            packed = self.session.bind(
+                [rt.TensorView.from_torch(n, t, self._dtypes.get(n)) for n, t in inputs.items()],
+                [rt.TensorView.from_torch(n, t, self._dtypes.get(n)) for n, t in outputs.items()])
             if bound is None and len(self._bindings) >= MAX_BINDINGS:
                 self._bindings.popitem(last=False)
-            bound = self._bindings[key] = (packed, [weakref.ref(t) for t in tensors], layout)
+            bound = self._bindings[key] = (packed, layout)
         self._bindings.move_to_end(key)
         self._keep = tensors       # in use until the next call at least
         raw = self._current_stream() if stream is None else stream.cuda_stream
