@@ -86,6 +86,32 @@ def test_layernorm_and_adaln_modulation(tmp_path, modulated):
     assert ops.max_rel_err(got["y"], want) < 1e-2
 
 
+@pytest.mark.parametrize("rows,cols", [(17, 1536), (50, 1536), (3, 8), (5, 8192), (2, 8200)])
+def test_layernorm_that_fetches_its_modulation_early(tmp_path, rows, cols):
+    """Scale and shift written by the profile itself, then read ahead of the dependency wait behind a launch that
+    releases its successors only after its own wait: the values of the ordinary order, bit for bit, under programmatic
+    dependent launch, for rows that stay in registers and rows that do not."""
+    from aginfer_b200 import runtime as rt
+    from aginfer_b200.recipes import U32
+    x, mod = (randn(rows, cols, seed=4).float() * 3 + 1.5).to(BF), randn(2, cols, seed=5, std=0.3)
+
+    def body(r):
+        held, ones, late = r.alloc(4 * cols), r.alloc(2 * rows * cols), r.alloc(4 * cols)
+        copy = lambda src, dst, n: r.launch("agi_copy_rows_bf16", (64, 1, 1), (256, 1, 1),
+                                            [src, dst, U32(n // cols), U32(cols), U32(cols), U32(cols)])
+        copy(Tensor("mod"), held, 2 * cols)
+        copy(Tensor("x"), ones, rows * cols)
+        # x + 0: the launch between the modulation's writer and its early reader
+        r.launch("agi_add_rows_bf16", (64, 1, 1), (256, 1, 1), [ones, late, U32(rows), U32(cols), U32(cols), U32(1)])
+        for out, static in (("early", True), ("plain", False)):
+            r.layernorm(ones, Tensor(out), rows, cols, 1e-5, scale=held, shift=held + 2 * cols, static_modulation=static)
+
+    got, _ = run_recipe(tmp_path, {}, {"x": x, "mod": mod}, {"early": (BF, (rows, cols)), "plain": (BF, (rows, cols))}, body,
+                        flags=rt.PROGRAMMATIC_LAUNCH, repeats=3)
+    assert torch.equal(got["early"], got["plain"])
+    assert ops.max_rel_err(got["early"], ops.layernorm(x, 1e-5, mod[0], mod[1])) < 1e-2
+
+
 def test_rope_1d(tmp_path):
     rows, heads, d = 288, 18, 128  # 16 query + 2 key heads rotated, 2 value heads untouched
     x = randn(rows, (heads + 2) * d, seed=6)
