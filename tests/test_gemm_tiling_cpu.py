@@ -61,3 +61,22 @@ def test_a_prefill_of_33_images_builds():
         weights = qwen_vl.synthetic_weights(cfg)
         r = qwen_vl.build_recipe(cfg, describe(qwen_vl.pack_checkpoint(weights) if packed else weights), packed=packed)
         assert r.launch_count() > 20
+
+
+@pytest.mark.parametrize("wide,text,launches", [(False, 128, 1), (False, 160, 1), (False, 896, 1), (True, 128, 1), (True, 129, 2),
+                                                (True, 208, 2), (True, 209, 1), (True, 512, 1)])
+def test_gate_and_up_are_two_launches_only_where_that_is_faster(wide, text, launches):
+    """Row-major operands; ``text`` + 128 rows of a 3B- or a 7B-shaped layer."""
+    kw = dict(hidden=3584, heads=28, kv_heads=4, intermediate=18944) if wide else {}
+    cfg = qwen_vl.VlConfig(images=2, text_tokens=text, v_layers=1, layers=1, vocab=64, v_full_layers=(), **kw)
+    shapes = {"visual.merger.mlp.0": (5120, 5120), "visual.merger.mlp.2": (cfg.hidden, 5120), **qwen_vl.llm_linears(cfg, 0),
+              **{n: s[:2] for n, s in qwen_vl.vision_linears(cfg, 0).items()}}
+    weights = {f"{n}.weight": ("F8_E4M3", s) for n, s in shapes.items()} | {f"{n}.weight_scale": ("F32", ()) for n in shapes}
+    weights |= {n: ("BF16", (cfg.hidden,)) for n in ("model.layers.0.input_layernorm.weight", "model.norm.weight",
+                                                     "model.layers.0.post_attention_layernorm.weight")}
+    weights |= {n: ("BF16", (1280,)) for n in ("visual.blocks.0.norm1.weight", "visual.blocks.0.norm2.weight", "visual.merger.ln_q.weight")}
+    weights |= {"visual.patch_embed.proj.weight": ("BF16", (1280, cfg.patch_k)), "model.embed_tokens.weight": ("BF16", (64, cfg.hidden))}
+    r = qwen_vl.build_recipe(cfg, weights)
+    wide_products = [l for l in r.profiles[0].launches if any(a == {"scalar_u32": cfg.intermediate} for a in l["arguments"][13:])
+                     and l["kernel"].startswith("agi_gemm_t") and l["arguments"][7] == {"scalar_u32": cfg.hidden}]
+    assert len(wide_products) == launches
