@@ -31,9 +31,15 @@
 namespace fa {
 
 constexpr unsigned kKeyTile = 64, kRows = 32, kLoaders = 64;
+// Key tiles of a chunk for 128-wide heads: five, so that up to 320 keys are one chunk.  One block per SM, as with four
+// or three (165 and 126 KB).  Causal rows, us a launch with 2 (two blocks per SM) / 3 / 4 / 5 tiles, 16 query and 2 KV
+// heads: 101 rows 5.5 / 5.0 / 5.4 / 5.4, 197: 9.1 / 7.2 / 6.5 / 6.9, 288: 11.4 / 8.9 / 9.8 / 8.5, 320: 13.1 / 12.1 / 13.8 /
+// 12.4, 512: 18.8 / 21.3 / 21.7 / 22.6, 1024: 55.5 / 57.0 / 56.6 / 58.1; 28 and 4 heads: 101: 6.3 / 5.0 / 5.6 / 5.5, 288:
+// 13.1 / 15.5 / 15.8 / 14.9, 1024: 77.8 / 88.1 / 88.5 / 89.5.  Of the one-block forms five is the best at 288 keys, level
+// at 320 and up to 12 % behind three elsewhere; grids of more than a round would gain from two blocks per SM.
 template <int HD16>
 struct Shape {
-  static constexpr unsigned kTiles = HD16 == 8 ? 5 : 4;                        // 128-wide heads: 320 keys, one block per SM
+  static constexpr unsigned kTiles = HD16 == 8 ? 5 : 4;
   static constexpr unsigned kCompute = kTiles * 64, kThreads = kCompute + kLoaders, kPerSm = HD16 == 8 ? 1 : 2;
 };
 

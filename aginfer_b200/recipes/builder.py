@@ -116,7 +116,9 @@ TK_SMEM_BUDGET = 226 * 1024
 TK_PAIR_BUDGET = 112 * 1024                       # shared memory of a CTA that shares its SM with another
 # CTAs in whole clusters that the GPCs hold, one CTA per SM (3: 135, 4: 132, 5: 130, 6: 132, 8: 120).  Behind a launch
 # that is still draining, clusters of 3, 5 and 6 find their SMs in pieces and the last of a full part's clusters starts
-# a round late: the planner leaves them room (288 tokens x 2048 x 11008 in runs of 3: 33 us at 135 CTAs, 20 us below 120).
+# a round late, so the planner leaves them room.  Where that changes the tile (136 products of the FP8 stacks' shapes,
+# 33 - 1024 tokens), the full part is 4 % slower behind a gate | up launch (clusters of 3: 5.5 %, up to 43 %; 5: 3.7 %;
+# 6: 1.6 %; 288 x 2048 x 11008: 43.7 us for both launches against 37.8) and level in a chain of itself.
 TK_RESIDENT = {1: SM_COUNT, 2: SM_COUNT, 3: 120, 4: 132, 5: 120, 6: 120, 8: 120}
 TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3, 4, 5, 6, 8), "agi_gemm_tc_e4m3_x3": (1, 2, 4, 8),
                "agi_gemm_tcpk_e4m3": (1, 2, 3, 4, 6, 8), "agi_gemm_tc_bf16_x3": (1, 2, 4, 8)}
@@ -190,8 +192,8 @@ def tk_tiling(M: int, widths: tuple[int, ...], K: int, elem: int, swiglu: bool =
     Every CTA takes in NB weight rows and its tokens, and that intake sets the time, so the estimate per CTA is
     K blocks x max(intake at 57 B per clock, 650 cycles: what one SM's outstanding loads give) + set-up, epilogue and
     exchange between ranks, times the rounds over the SMs.  Half-size rings put two CTAs on an SM, whose set-up and
-    epilogue then overlap.  The constants are fitted to 30 000 timed tiles of 70 shapes (36 - 1024 tokens): the tile
-    chosen is 3.5 % slower than the fastest one on average, 28 % at worst."""
+    epilogue then overlap.  How good the choice is: on 40 shapes (36 - 1024 tokens), each timed with 28 other tiles, it is
+    3.4 % slower than the fastest one on average, 1 % in the median and 28 % at worst (768 x 2048 x 11008 in bf16)."""
     k_blocks = K * elem // 128
     # Token groups of at most 512 rows (four MMA tiles), counted up from the fewest: to 16, or, beyond 4096 tokens, to
     # groups of half that size, so that a tile with 256 weight rows or eight runs fits tensor memory at any M.
