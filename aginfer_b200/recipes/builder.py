@@ -125,60 +125,71 @@ TK_CLUSTERS = {"agi_gemm_tk_bf16": (1, 2, 3, 4, 8), "agi_gemm_tk_e4m3": (1, 2, 3
 TK_MAX_RING = 8
 
 
-def _run_estimate(rows: int, tn: int, n_tiles: int, m_tiles: int, k_blocks: int, runs: int) -> float:
-    per = ceil_div(k_blocks, runs)
-    cost = ceil_div(n_tiles * m_tiles * runs, SM_COUNT) * (per * max((rows + tn) * 128 / 28, rows // 128 * tn * 2) + 5000 + tn * 25)
-    return cost + (4000 + rows * tn * (runs + 1) // 8 if runs > 1 else 0)
+# ---- how K is summed ---------------------------------------------------------------------------------------
+# Part of a recipe's numerics: `k_runs` says into how many runs K is cut when a product inside a stack of FP8 blocks is
+# summed (each run by the tensor core in fp32, then the runs in order).  One flipped rounding in front of a per-tensor
+# amax is another quantisation of a whole tensor, so the count follows from the product's shape alone: tiles and clusters
+# may change with what the kernels cost, this rule and its constants may not.  It gives a product whose output is few
+# tiles of 128 weight rows more runs, so that they can be shared out over 148 SMs:
+#   up to 64 rows    the most of 2, 4, 8 (bf16 also 3 and 6) runs of at least two 128-byte blocks of K that keep
+#                    tiles x runs within 148; one where there are none, or where the last run would be empty;
+#   65 to 127 rows   enough runs of at least two blocks for 148 tiles x runs, up to 16; one from 120 tiles on;
+#   from 128 rows    the count of 1, 2, 3, 4, 6, 8, in runs of at least four blocks, with the least `_order_cost` over
+#                    tiles of 128 or 256 weight rows by 16 to 256 tokens: rounds of the tiles over 148 SMs times a
+#                    run's length, plus what adding the runs takes;
+#   packed operands  the last rule from one row on, but one run while K has at most 48 blocks, from 768 rows on, or
+#                    where tiles of 128 rows alone make two rounds.
+# In every case the runs' partial sums fit 32 MiB of scratch.
+def _filled_runs(k_blocks: int, runs: int) -> int:
+    """The runs that have a block of K when it is cut into equal lengths for ``runs`` of them."""
+    return ceil_div(k_blocks, ceil_div(k_blocks, max(1, min(runs, k_blocks))))
+
+
+def _order_cost(rows: int, tokens: int, tiles: int, k_blocks: int, runs: int) -> float:
+    """Clocks of ``tiles`` output tiles of ``rows`` x ``tokens`` in ``runs`` runs each: 28 bytes of operands or two
+    accumulator columns a clock, and 5000 + 25 a token of set-up and epilogue; then the exchange of the partial sums."""
+    block = max((rows + tokens) * 128 / 28, rows // 128 * tokens * 2)
+    clocks = ceil_div(tiles * runs, SM_COUNT) * (ceil_div(k_blocks, runs) * block + 5000 + tokens * 25)
+    return clocks + (4000 + rows * tokens * (runs + 1) // 8 if runs > 1 else 0)
+
+
+def _token_tiles(M: int) -> list[int]:
+    """Token tiles of at most 256 rows, a multiple of 16, that split M evenly; the widest first."""
+    return list(dict.fromkeys(ceil_div(ceil_div(M, ceil_div(M, cap)), 16) * 16 for cap in range(256, 48, -16)))
 
 
 @functools.lru_cache(maxsize=4096)
 def k_runs(M: int, N: int, K: int, elem: int, packed: bool = False) -> int:
-    """Into how many runs K is cut when a product of this shape is summed (each run by the tensor core in fp32, then the
-    runs in order).  Part of a recipe's numerics, a function of the shape alone: FP8 block stacks turn one flipped
-    rounding into another quantisation of a whole tensor, so tiles and clusters may change with the hardware's costs, the
-    order of the sum may not.  More runs where a product has few output tiles for its K."""
-    k_blocks = K * elem // 128
+    """Runs in which K is summed, see above; ``elem``: bytes of an operand's element."""
+    k_blocks, tiles = K * elem // 128, ceil_div(N, 128)
     if M <= 64 and not packed:
-        c = tc_cluster_tiling(M, N, K, elem, "e4m3" if elem == 1 else "bf16")
-        return c["cluster"] if c is not None else 1
+        runs = max((c for c in ((2, 4, 8) if elem == 1 else (2, 3, 4, 6, 8)) if tiles * c <= SM_COUNT and k_blocks >= 2 * c),
+                   default=1)
+        return runs if _filled_runs(k_blocks, runs) == runs else 1
     if M < 128 and not packed:
-        runs = tc_tiling(M, N, K, elem)["splits"]
-        while runs > 1 and runs * M * ceil_div(N, 128) * 512 > TC_SCRATCH_BYTES:
-            runs = tc_tiling(M, N, K, elem, runs // 2)["splits"]
+        runs = _filled_runs(k_blocks, 1 if tiles >= 120 else max(1, min(16, ceil_div(SM_COUNT, tiles), k_blocks // 2)))
+        while runs > 1 and runs * M * tiles * 512 > TC_SCRATCH_BYTES:
+            runs = _filled_runs(k_blocks, runs // 2)
         return runs
-    best: tuple[float, int] | None = None
-    for rows in (128, 256):
-        if rows == 256 and N < 256:
-            continue
-        n_tiles, seen = ceil_div(N, rows), set()
-        for cap in range(256, 48, -16):
-            m_tiles = ceil_div(M, cap)
-            tn = ceil_div(ceil_div(M, m_tiles), 16) * 16
-            if tn in seen:
-                continue
-            seen.add(tn)
-            for runs in (1, 2, 3, 4, 6, 8):
-                per = ceil_div(k_blocks, runs)
-                if ceil_div(k_blocks, per) != runs or (runs > 1 and (per < 4 or runs * M * n_tiles * rows * 4 > TC_SCRATCH_BYTES)):
-                    continue
-                if n_tiles * m_tiles * 4 > TC_COUNTER_BYTES:
-                    continue
-                cost = _run_estimate(rows, tn, n_tiles, m_tiles, k_blocks, runs)
-                if best is None or cost < best[0]:
-                    best = (cost, runs)
-    assert best is not None
-    runs = best[1]
-    if packed and runs > 1:
-        # one run while K is short, or where enough tokens fill the SMs without cutting it
-        tiles, least = 0, None
-        for mt in range(ceil_div(M, 256), ceil_div(M, 256) + PERSIST_TOKEN_SPLITS):
-            tn = ceil_div(ceil_div(M, mt), 16) * 16
-            cost = ceil_div(ceil_div(N, 128) * mt, SM_COUNT) * max((16384 + tn * 128) / 40, 2 * tn)
-            if tn >= 16 and (least is None or cost < least):
-                least, tiles = cost, ceil_div(N, 128) * mt
-        if tiles >= 2 * SM_COUNT or k_blocks <= 48 or M >= 768:
-            return 1
+    options = [(_order_cost(rows, tn, ceil_div(N, rows) * ceil_div(M, tn), k_blocks, runs), order, runs)
+               for order, (rows, tn, runs) in enumerate((r, t, c) for r in (128, 256) for t in _token_tiles(M) for c in (1, 2, 3, 4, 6, 8))
+               if (rows == 128 or N >= 256) and _filled_runs(k_blocks, runs) == runs
+               and (runs == 1 or (ceil_div(k_blocks, runs) >= 4 and runs * M * ceil_div(N, rows) * rows * 4 <= TC_SCRATCH_BYTES))
+               and ceil_div(N, rows) * ceil_div(M, tn) * 4 <= TC_COUNTER_BYTES]
+    assert options, "a product inside an FP8 stack has at most 4096 output tiles"
+    runs = min(options)[2]
+    if packed and runs > 1 and (k_blocks <= 48 or M >= 768 or _plain_tiles(M, N) >= 2 * SM_COUNT):
+        return 1
     return runs
+
+
+def _plain_tiles(M: int, N: int) -> int:
+    """Output tiles of 128 weight rows by the token tile (of the fewest counts) that takes the least time in one run."""
+    least = (math.inf, 0)
+    for groups in range(ceil_div(M, 256), ceil_div(M, 256) + PERSIST_TOKEN_SPLITS):
+        tn, tiles = ceil_div(ceil_div(M, groups), 16) * 16, ceil_div(N, 128) * groups
+        least = min(least, (ceil_div(tiles, SM_COUNT) * max((16384 + tn * 128) / 40, 2 * tn), tiles))
+    return least[1]
 
 
 @functools.lru_cache(maxsize=4096)

@@ -80,3 +80,36 @@ def test_gate_and_up_are_two_launches_only_where_that_is_faster(wide, text, laun
     wide_products = [l for l in r.profiles[0].launches if any(a == {"scalar_u32": cfg.intermediate} for a in l["arguments"][13:])
                      and l["kernel"].startswith("agi_gemm_t") and l["arguments"][7] == {"scalar_u32": cfg.hidden}]
     assert len(wide_products) == launches
+
+
+# (N, K, bytes an element, packed): the row counts from which on K is cut into another number of runs, up to 1600 rows.
+# Recorded when FP8 stacks were first held to it; a change here changes the output bits of packaged models.
+K_RUNS = {
+    (1280, 1280, 1, False): "1:4 65:5 128:1",
+    (3840, 1280, 1, False): "1:4 65:5 128:1",
+    (1280, 3456, 1, False): "1:1 65:9 128:4 193:3 321:2 561:1",
+    (5120, 5120, 1, False): "1:2 65:4 128:3 129:1 145:3 161:1",
+    (2048, 5120, 1, False): "1:8 65:10 128:4 129:3 145:4 161:3 241:2 257:3 289:2 321:3 337:2 449:3 481:1",
+    (3584, 5120, 1, False): "1:4 65:6 128:2 225:1",
+    (2048, 2048, 1, False): "1:8 128:4 129:3 193:1",
+    (11008, 2048, 1, False): "1:1 65:2 128:1",
+    (2048, 11008, 1, False): "1:8 65:10 128:4 129:3 145:4 161:3 1249:2 1297:3 1345:2",
+    (3584, 3584, 1, False): "1:4 65:6 128:2 193:1",
+    (18944, 3584, 1, False): "1:1",
+    (3584, 18944, 1, False): "1:4 65:6 128:4 321:3 337:4 353:3 769:2 1171:1",
+    (1280, 1216, 2, False): "1:1 65:7 128:4 193:3 257:2 449:1",
+    (2048, 11008, 1, True): "1:8 65:4 129:3 145:4 161:3 768:1",
+    (3584, 18944, 1, True): "1:4 321:3 337:4 353:3 768:1",
+}
+
+
+@pytest.mark.parametrize("shape", K_RUNS, ids=lambda s: "x".join(map(str, s)))
+def test_the_order_of_the_sum_over_k_is_the_recorded_one(shape):
+    N, K, elem, packed = shape
+    found, last = [], None
+    for M in range(1, 1601):
+        runs = k_runs(M, N, K, elem, packed)
+        if runs != last:
+            found.append(f"{M}:{runs}")
+        last = runs
+    assert " ".join(found) == K_RUNS[shape]
