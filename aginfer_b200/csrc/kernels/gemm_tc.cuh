@@ -1,11 +1,12 @@
 // Tensor-core GEMM for sm_100a: Y[M, N] = epilogue(X[M, K] . W[N, K]^T), bf16 or E4M3 operands,
-// fp32 accumulation in tensor memory (TMEM) with tcgen05.mma.
+// fp32 accumulation in tensor memory (TMEM) with tcgen05.mma.  The kernel of `agi_gemm_bf16_static_scratch` and of an
+// explicit tactic="tcgen05"; recipes that leave the choice open get gemm_tk.cuh from 33 tokens on, which shares the
+// helpers defined here.
 //
 // Orientation.  The weight matrix is the MMA's A operand: a CTA owns 128 consecutive rows of
 // W (128 output features) and `TN` tokens, TN a multiple of 16 up to 256.  The accumulator
-// tile D[128 x TN] has one output feature per TMEM lane and one token per column.  This way
-// a batch-1 action head (17 or 50 tokens) and a 1024-token prefill run the same code: few
-// tokens only make the tile narrower, the 128-row weight stream per CTA stays the same.
+// tile D[128 x TN] has one output feature per TMEM lane and one token per column: few tokens
+// only make the tile narrower, the 128-row weight stream per CTA stays the same.
 //
 // Data movement.  W is checkpoint bytes, [N, K] row-major, i.e. already K-major.  The kernel
 // ABI passes only pointers and scalars, so no tensor-map object can be handed to the kernel;
@@ -143,10 +144,6 @@ __device__ __forceinline__ void tmem_load16(unsigned addr, float v[16]) {
 // Thread-block cluster helpers (split-K slices of one output tile form a cluster along grid z).
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_sync() {
-  cluster_arrive();
-  cluster_wait();
-}
 // Address of `local_smem_addr` in the shared memory of cluster rank `rank`.
 __device__ __forceinline__ unsigned peer_smem(unsigned local_smem_addr, unsigned rank) {
   unsigned remote;

@@ -42,7 +42,7 @@ using namespace tc;
 
 constexpr unsigned kMaxRing = 8;
 // kW weight warps, kW token warps (all of them: epilogue), 1 MMA warp.
-__host__ __device__ constexpr unsigned threads(unsigned kW) { return (2 * kW + 1) * 32; }
+constexpr unsigned kW = 4, kMmaWarp = 2 * kW, kEpilogue = 64 * kW, kThreads = kEpilogue + 32;
 
 struct Part {
   const uint8_t* w;
@@ -84,7 +84,7 @@ enum Finish { kScale, kScaleBias, kScaleResidual, kScaleBiasResidual, kGateUp, k
 // Rows [0, count) of the staged fp32 tile (P floats apart) are tokens m ... of features n0 ... n0 + 8 * groups - 1 (with
 // kGateUp the up products follow the gate products in the row).  Eight features a thread, consecutive threads along a
 // row.  Returns max |y| over what this thread stored, before rounding (rounding is monotonic), where it is asked for.
-template <int kMode, unsigned kEpilogue>
+template <int kMode>
 __device__ __forceinline__ float finish_tile(const float* tile, unsigned P, unsigned count, unsigned groups, unsigned m,
                                              unsigned n0, const Out& o) {
   constexpr bool kGen = kMode == kGeneral;
@@ -186,7 +186,7 @@ __device__ __forceinline__ float finish_tile(const float* tile, unsigned P, unsi
 // Adds `runs` filed partial tiles, in order, over `count` rows and 4 * `quads` columns into the staged tile.  Item =
 // (four columns, row), rows fastest; a thread's items are kEpilogue apart, kBatch at a time, and kRuns loads of each are
 // in flight together (eight 16-byte loads a thread: more spill at the 96 registers that let two CTAs share an SM).
-template <unsigned kBatch, unsigned kRuns, unsigned kEpilogue>
+template <unsigned kBatch, unsigned kRuns>
 __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsigned P, unsigned count, unsigned quads,
                                          unsigned R, unsigned runs) {
   if (count == 0) return;
@@ -227,19 +227,19 @@ __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsig
   }
 }
 
-// grid = (weight tiles of all parts, token groups of `tg` rows, ranks), block = threads(kW).  NB: weight rows of a tile, a
+// grid = (weight tiles of all parts, token groups of `tg` rows, ranks), block = kThreads.  NB: weight rows of a tile, a
 // multiple of 16 (of 32 with kFlagSwiglu) up to 256; tg a multiple of 8, ceil(tg / 128) * NB' * (runs a rank takes) <=
 // 512 with NB' = NB rounded up to 32.  Dynamic shared memory: 1024 + the larger of the ring, stages * (tg + NB) * 128 plus what the last
 // slot's A tiles overhang (rows past the tokens are read by the MMA, never stored), and the epilogue's tile,
 // min(tg, 128) (in a cluster: ceil(tg / (8 ranks)) * 8) * (NB + 4) * 4.  `partial` holds
 // gridDim.x * gridDim.y * runs * NB * (tg rounded up to 32) floats for a cluster.
-template <bool kFp8, bool kPacked, bool kCluster, unsigned kW>
+template <bool kFp8, bool kPacked, bool kCluster>
 __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, const bf16* other, float* partial,
                                      unsigned* amax_bits, unsigned* status, unsigned M, unsigned K, unsigned ldx,
                                      unsigned flags, unsigned NB, unsigned stages, unsigned tg, unsigned runs,
                                      unsigned per_run, const Part& p0,
                                      const Part& p1, const Part& p2, unsigned tile = blockIdx.x) {
-  constexpr unsigned kMmaWarp = 2 * kW, kEpilogue = 64 * kW, kRowStep = 4 * kW;   // kRowStep: rows a copy pass covers
+  constexpr unsigned kRowStep = 4 * kW;   // rows a copy pass covers
   extern __shared__ unsigned char dynamic_smem[];
   __shared__ __align__(8) unsigned long long full_bar[kMaxRing], empty_bar[kMaxRing], accum_bar;
   __shared__ unsigned tmem_slot;
@@ -441,13 +441,13 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
   auto finish = [&](unsigned count, unsigned m) {
     const unsigned groups = nb_out / 8;
     switch (mode) {
-      case kScale: finish_tile<kScale, kEpilogue>(tile_rows, P, count, groups, m, n0, o); break;
-      case kScaleBias: finish_tile<kScaleBias, kEpilogue>(tile_rows, P, count, groups, m, n0, o); break;
-      case kScaleResidual: finish_tile<kScaleResidual, kEpilogue>(tile_rows, P, count, groups, m, n0, o); break;
-      case kScaleBiasResidual: finish_tile<kScaleBiasResidual, kEpilogue>(tile_rows, P, count, groups, m, n0, o); break;
-      case kGateUp: best = fmaxf(best, finish_tile<kGateUp, kEpilogue>(tile_rows, P, count, groups, m, n0, o)); break;
-      case kTimesSilu: best = fmaxf(best, finish_tile<kTimesSilu, kEpilogue>(tile_rows, P, count, groups, m, n0, o)); break;
-      default: best = fmaxf(best, finish_tile<kGeneral, kEpilogue>(tile_rows, P, count, groups, m, n0, o)); break;
+      case kScale: finish_tile<kScale>(tile_rows, P, count, groups, m, n0, o); break;
+      case kScaleBias: finish_tile<kScaleBias>(tile_rows, P, count, groups, m, n0, o); break;
+      case kScaleResidual: finish_tile<kScaleResidual>(tile_rows, P, count, groups, m, n0, o); break;
+      case kScaleBiasResidual: finish_tile<kScaleBiasResidual>(tile_rows, P, count, groups, m, n0, o); break;
+      case kGateUp: best = fmaxf(best, finish_tile<kGateUp>(tile_rows, P, count, groups, m, n0, o)); break;
+      case kTimesSilu: best = fmaxf(best, finish_tile<kTimesSilu>(tile_rows, P, count, groups, m, n0, o)); break;
+      default: best = fmaxf(best, finish_tile<kGeneral>(tile_rows, P, count, groups, m, n0, o)); break;
     }
   };
   const unsigned R = (tg + 31u) & ~31u;      // rows of a filed partial tile: [run][column / 4][row] float4
@@ -526,9 +526,9 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     const unsigned share = ((rows + ranks * 8 - 1) / (ranks * 8)) * 8;
     const unsigned first = min(rank * share, rows), count = min(share, rows - first);
     const float4* from = filed + first;
-    if (runs <= 2) add_runs<4, 2, kEpilogue>(from, tile_rows, P, count, NB / 4, R, runs);
-    else if (runs <= 4) add_runs<2, 4, kEpilogue>(from, tile_rows, P, count, NB / 4, R, runs);
-    else add_runs<1, 8, kEpilogue>(from, tile_rows, P, count, NB / 4, R, runs);
+    if (runs <= 2) add_runs<4, 2>(from, tile_rows, P, count, NB / 4, R, runs);
+    else if (runs <= 4) add_runs<2, 4>(from, tile_rows, P, count, NB / 4, R, runs);
+    else add_runs<1, 8>(from, tile_rows, P, count, NB / 4, R, runs);
     asm volatile("bar.sync 1, %0;" ::"n"(kEpilogue) : "memory");
     finish(count, m0 + first);
   }
@@ -541,7 +541,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
 }  // namespace tk
 
 #define AGI_TK_KERNEL(NAME, CLUSTER, TYPE, FP8, PACKED, IN_CLUSTER)                                                   \
-  extern "C" __global__ void CLUSTER __launch_bounds__(tk::threads(4), 2)                                            \
+  extern "C" __global__ void CLUSTER __launch_bounds__(tk::kThreads, 2)                                              \
   NAME(const TYPE* x, const float* scale_a, const bf16* other, float* partial, unsigned* amax_bits,                  \
        unsigned* status, unsigned M, unsigned K, unsigned ldx, unsigned flags, unsigned NB, unsigned stages,         \
        unsigned tg, unsigned runs, unsigned per_run, const TYPE* w0, const bf16* bias0, const float* sw0, void* y0,   \
@@ -550,7 +550,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     const tk::Part p0 = {reinterpret_cast<const uint8_t*>(w0), bias0, sw0, y0, N0, ldy0};                            \
     const tk::Part p1 = {reinterpret_cast<const uint8_t*>(w1), bias1, sw1, y1, N1, ldy1};                            \
     const tk::Part p2 = {reinterpret_cast<const uint8_t*>(w2), bias2, sw2, y2, N2, ldy2};                            \
-    tk::body<FP8, PACKED, IN_CLUSTER, 4>(reinterpret_cast<const uint8_t*>(x), scale_a, other, partial, amax_bits,    \
+    tk::body<FP8, PACKED, IN_CLUSTER>(reinterpret_cast<const uint8_t*>(x), scale_a, other, partial, amax_bits,       \
                                          status, M, K, ldx, flags, NB, stages, tg, runs, per_run, p0, p1, p2);       \
   }
 // The ranks that share K: grid z = C.  Up to 15 clusters of 8, 33 of 4, 74 of 2 are resident at once.
@@ -589,7 +589,7 @@ AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 8)
 // Up to 16 independent bf16 GEMMs that share the activation matrix (the K and V projections of every cross-attention
 // block over the context tokens, every block's AdaLN projection) as ONE launch: grid.x = segments * ceil(N / NB);
 // segment s multiplies by w[s], adds bias[s] and writes y + s * seg_stride elements.
-extern "C" __global__ void __launch_bounds__(tk::threads(4), 2)
+extern "C" __global__ void __launch_bounds__(tk::kThreads, 2)
 agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsigned N, unsigned K, unsigned ldx,
                      unsigned ldy, unsigned flags, unsigned NB, unsigned stages, unsigned tg, unsigned seg_stride,
                      const bf16* w0, const bf16* w1, const bf16* w2, const bf16* w3, const bf16* w4, const bf16* w5,
@@ -610,6 +610,6 @@ agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsig
     default: w = w15; b = b15; break;
   }
   const tk::Part part = {reinterpret_cast<const uint8_t*>(w), b, nullptr, y + size_t(seg) * seg_stride, N, ldy};
-  tk::body<false, false, false, 4>(reinterpret_cast<const uint8_t*>(x), nullptr, nullptr, nullptr, nullptr, status, M, K,
+  tk::body<false, false, false>(reinterpret_cast<const uint8_t*>(x), nullptr, nullptr, nullptr, nullptr, status, M, K,
                                ldx, flags, NB, stages, tg, 1, K / 64, part, part, part, blockIdx.x % tiles);
 }

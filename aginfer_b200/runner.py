@@ -76,7 +76,9 @@ class Runner:
         self._keep = tensors       # in use until the next call at least
         raw = self._current_stream() if stream is None else stream.cuda_stream
         if raw == 0 and not self._replays:
-            # Plain launches go to a stream of their own, ordered after and before the work on the default stream.
+            # Replay switched off: every launch goes to a stream of its own, ordered after and before the work on the
+            # default stream.  With replay on, graphs and the first pass over a further set of addresses (launched one
+            # by one) go into the default stream itself.
             import torch
             if self._side is None:
                 self._side = torch.cuda.Stream()
