@@ -28,7 +28,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import Sequence
 
-from .builder import SM_COUNT, RecipeBuilder, Tensor, U32, Weight, ceil_div, grid_for, io, k_runs
+from .builder import RecipeBuilder, Tensor, U32, Weight, ceil_div, grid_for, io, k_runs
 from .layout import pack_kblock_swizzled, padded_token_rows
 
 
@@ -284,11 +284,13 @@ def build_recipe(cfg: VlConfig, weights, gemm_tactic: str = "auto", trace: bool 
                               Weight(f"{mlp}.{n}.weight_scale"))
             # narrow pairs sum K in one run, wide ones as one of them alone would
             runs = 1 if 2 * cols <= 8192 else k_runs(rows, cols, K, 1, packed)
-            # One launch, except where a row-major pair's tiles (128 gate and 128 up rows) alone fill the SMs and the rows
-            # make three token groups: three rounds, where each of two launches takes one.  Prefill of 4 (3B) or 2 (7B)
-            # decoder layers, one launch / two: 11008 x 2048 at 260 to 1024 rows 0.93 - 0.99; 18944 x 3584 at 257 rows
-            # 546 / 478 us, 288: 984 / 894 (4 layers), 336: 594 / 549, 352: 543 / 540, 400: 549 / 552, 640: 744 / 817.
-            two = not packed and ceil_div(cols, 128) >= SM_COUNT and 256 < rows <= 336
+            # One launch, except for wide row-major pairs whose rows make three token groups (257 to 336).  Where a pair's
+            # tiles (128 gate and 128 up rows) alone fill the SMs, three groups are three rounds, and each of two launches
+            # takes one: prefill with 2 decoder layers of 18944 x 3584, one launch / two, 257 rows 546 / 478 us, 336: 594 /
+            # 549, 352: 543 / 540, 400: 549 / 552, 640: 744 / 817.  The other width in use, 11008 x 2048, would be 1 - 8 %
+            # faster as one launch there too (4 layers, 288 rows: 511 / 552; 450: 629 / 638; 768: 816 / 848) and keeps two
+            # up to 336 rows so that the plan of the 288-token prefill, which packages in use carry, stays as it is.
+            two = not packed and 2 * cols > 8192 and 256 < rows <= 336
             r.gemm_swiglu(quant, part("gate_proj"), part("up_proj"), out, rows, cols, K, dtype="e4m3", scale_a=scale,
                           packed=packed, amax=amax, scratch=scratch if two else None, runs=runs)
         else:
