@@ -27,8 +27,8 @@
 // letting it wait for itself.  A wait that runs out records a code in the status word; every CTA sees the word
 // at its next wait and leaves, so a fault surfaces as a status and wrong numbers, never as a hang.
 //
-// Measured on B200 (16 blocks x 1536, 17 tokens; SM-clock stamps of two CTAs): about 57 us per block, 3.9 ms per
-// action chunk, against 2.9 ms for the same blocks as 27 separate launches chained by programmatic dependent
+// Measured on B200 (16 blocks x 1536, 17 tokens; SM-clock stamps of two CTAs): about 57 us per block, 3.85 ms per
+// action chunk, against 2.38 ms for the same blocks as 27 separate launches chained by programmatic dependent
 // launch - so recipes use it only on request.  Where a block's 57 us go, on the CTA with the most work:
 //   * warp-level MMA: an m16n8k16 keeps a sub-core's tensor pipe ~30 cycles on this part, so the nine 16-row
 //     units a CTA owns per block cost ~1.1 us each in the pipe alone (1.7 us with ring waits): 16 us;

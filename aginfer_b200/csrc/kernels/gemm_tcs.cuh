@@ -27,8 +27,8 @@
 // running ones (two GEMMs need 256 KB of weights per SM); they enter only as CTAs exit, the last of them 6-9 us
 // after the first, and the wait is released when the last one is in: 9.2-10.9 us per launch against 7.0 / 10.5 us
 // of the bulk-stream kernel, whose smaller CTAs (16 rows, 73-104 KB, three or two per SM) hand the SMs over more
-// evenly.  Inside the action head's graph the packed path therefore costs 3.57 ms per chunk against 2.93 ms
-// (per matrix family: output projection +0.01 ms, Q|K|V +0.08, MLP up +0.25, MLP down +0.30), and recipes use
+// evenly.  Inside the action head's graph the packed path therefore costs 3.13 ms per chunk against 2.38 ms (the
+// MLP matrices make up most of it, the output projection almost nothing), and recipes use
 // it only when the checkpoint was packaged in the packed layout.  Two things tried on the way and dropped,
 // neither of which shortened a launch: an L2 prefetch (cp.async.bulk.prefetch.L2 or
 // prefetch.global.L2) of the next launch's weights issued by every CTA, and a single accumulator (an MMA of

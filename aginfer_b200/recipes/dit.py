@@ -140,7 +140,7 @@ def build_recipe(cfg: DitConfig = DitConfig(), weights: Mapping[str, tuple[str, 
                  step_profiles: Sequence[int] = ()) -> RecipeBuilder:
     """``block_kernel``: run each denoising step's blocks as one launch of the persistent block kernel
     (78 launches per chunk instead of 506).  Off by default: measured on B200 it is the slower of the two
-    (3.9 ms per chunk against 2.9 ms), see the kernel's header for where its time goes.
+    (3.85 ms per chunk against 2.38 ms), see the kernel's header for where its time goes.
     ``step_profiles``: further numbers of Euler steps to package as sibling profiles ``<profile>/steps=<n>``
     (same tensors; the loader runs one of them when the caller's RunOptions ask for n denoising steps).
     ``stream_profile``: also emit the measurement profiles of the dominant kernel."""
