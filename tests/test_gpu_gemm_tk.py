@@ -79,33 +79,35 @@ def quantised(x):
     (130, 144, 1536, 3, 1), (130, 144, 1536, 3, 2), (130, 144, 1536, 3, 3), (33, 160, 3072, 6, 6), (33, 160, 3072, 6, 4),
     (257, 80, 1792, 7, 4), (257, 80, 1792, 7, 6), (129, 48, 1664, 4, 4), (129, 48, 1664, 4, 1), (96, 1536, 1536, 6, 3),
     (96, 1536, 1536, 6, 2), (513, 2048, 1536, 3, 3), (513, 2048, 1536, 3, 1), (600, 1536, 1024, 2, 2), (450, 3584, 1536, 3, 3)])
-@pytest.mark.parametrize("dtype", ["bf16", "e4m3"])
-def test_the_sum_over_k_does_not_depend_on_the_cluster(tmp_path, dtype, M, N, K, runs, ranks):
+@pytest.mark.parametrize("kind", ["bf16", "e4m3", "packed"])
+def test_the_sum_over_k_does_not_depend_on_the_cluster(tmp_path, kind, M, N, K, runs, ranks):
     """K in 3 to 10 runs, kept by one CTA or shared by 2 to 8 ranks that hold one run, several, or unequal counts: the
     same bits as one CTA that adds all of them, and the oracle's values."""
     from aginfer_b200.recipes.builder import FLAG_BIAS, FLAG_SCALED, TK_CLUSTERS, tk_tiling
 
-    family, elem = f"agi_gemm_tk_{dtype}", 2 if dtype == "bf16" else 1
+    packed, elem = kind == "packed", 2 if kind == "bf16" else 1
+    family = "agi_gemm_tcpk_e4m3" if packed else f"agi_gemm_tk_{kind}"
     if ranks not in TK_CLUSTERS[family]:
         pytest.skip("no such cluster for this type")
     g = torch.Generator().manual_seed(K + M)
     x, wf, bias = torch.randn(M, K, generator=g).to(BF), torch.randn(N, K, generator=g).to(BF), torch.randn(N, generator=g).to(BF)
-    if dtype == "bf16":
+    if kind == "bf16":
         weights, want = {"w": wf, "b": bias}, ops.gemm(x, wf, bias=bias)
     else:
         (xq, xs), (wq, ws) = quantised(x), quantised(wf)
-        weights, want = {"w": wq, "b": bias, "s": ws}, ops.gemm(xq, wq, scale_a=xs, scale_w=ws, bias=bias)
+        weights = {"w": pack_kblock_swizzled(wq) if packed else wq, "b": bias, "s": ws}
+        want = ops.gemm(xq, wq, scale_a=xs, scale_w=ws, bias=bias)
 
     def body(r):
         src, scale = Tensor("x"), None
-        if dtype == "e4m3":
-            src, scale = r.alloc(M * K), r.alloc(4)
-            r.quantize_e4m3(Tensor("x"), src, scale, M * K)
+        if kind != "bf16":
+            src, scale = r.alloc((padded_token_rows(M) if packed else M) * K), r.alloc(4)
+            r.quantize_e4m3(Tensor("x"), src, scale, M * K, packed=(M, K) if packed else None)
         for out, C in (("y", ranks), ("one", 1)):
             t = tk_tiling(M, (N,), K, elem, runs=runs, clusters=(C,))
             assert t["C"] == C and t["runs"] == runs
             r._gemm_tk(family, "gemm", t, src, [(Weight("w"), Weight("b"), Weight("s") if scale else None, Tensor(out), N, N)],
-                       M, K, K, FLAG_BIAS | (FLAG_SCALED if scale else 0), scale_a=scale)
+                       M, K, padded_token_rows(M) if packed else K, FLAG_BIAS | (FLAG_SCALED if scale else 0), scale_a=scale)
         r.export_status(Tensor("status"))
 
     got, _ = run_recipe(tmp_path, weights, {"x": x}, {"y": (BF, (M, N)), "one": (BF, (M, N)), "status": (torch.int32, (1,))}, body,
