@@ -51,20 +51,30 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("{ .reg .b64 t; mbarrier.arrive.shared::cta.b64 t, [%0]; }" ::"r"(smem_u32(bar)) : "memory");
 }
 // Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
-// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.
+// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.  One loop in
+// one statement: a wait that finds its phase complete takes ~70 cycles; as a C++ loop around try_wait it took ~195, and the
+// thread that issues the MMAs waits once per slot of its ring.
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
-  const unsigned addr = smem_u32(bar);
-  for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
-    unsigned done;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  atomicCAS(status, 0u, code);
-  return false;
+  unsigned done;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .u32 n;\n"
+      "mov.u32 n, 0;\n"
+      "WAIT:\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "@p bra DONE;\n"
+      "add.u32 n, n, 1;\n"
+      "setp.lt.u32 p, n, %3;\n"
+      "@p bra WAIT;\n"
+      "DONE:\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity), "n"(kSpinLimit)
+      : "memory");
+  if (__builtin_expect(done == 0, 0)) atomicCAS(status, 0u, code);
+  return done != 0;
 }
 
 __device__ __forceinline__ void cp_async_16(unsigned dst, const void* src) {
