@@ -433,6 +433,7 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
   auto stage = [&](unsigned first, unsigned last) {
     if ((threadIdx.x % kDtiles) >= vec_per_row) return;
     const unsigned d = (threadIdx.x % kDtiles) * 8;
+#pragma unroll 2
     for (unsigned j = first + threadIdx.x / kDtiles; j < last; j += blockDim.x / kDtiles) {
       const unsigned src_row = min(j, kv_rows - 1), bytes = j < kv_rows ? 16u : 0u;
       const unsigned kd = static_cast<unsigned>(__cvta_generic_to_shared(k_tile + j * pitch + d));
@@ -477,6 +478,15 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[nt][i] = 0.f;
   const unsigned dtiles = 2 * ksteps;      // <= kDtiles
+  // Keys that rows g, g + 8 may see are one range each, worked out once: a division per score is 15 KB of code for a launch
+  // that runs it once, and instructions that are fetched for the first time cost more than they compute.
+  unsigned key_lo[2], key_hi[2];
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) {
+    const unsigned row = row_base + g + hr * 8, lo = mask_mode == 2 ? row / mask_arg * mask_arg : 0u;
+    key_lo[hr] = lo;
+    key_hi[hr] = mask_mode == 0 ? kv_rows : min(kv_rows, mask_mode == 1 ? row + mask_arg + 1 : lo + mask_arg);
+  }
   // Few keys (at most two 16-key blocks, e.g. self-attention over 17 tokens): splitting the keys over warps would
   // leave six warps idle and still pay the merge.  Instead every warp w < dtiles scores ALL keys (the same few
   // MMAs in each warp) and multiplies P with the 8 value columns of ITS tile only: no merge, no second barrier,
@@ -486,6 +496,7 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
   const unsigned first_key = by_dims ? 0u : warp * 16u, key_step = by_dims ? 16u : 128u;
   constexpr int kGroup = 3;   // 16-key blocks scored together: their MMAs are independent, one rescale per group
 
+#pragma unroll 1
   for (unsigned base = first_key; base < kv16; base += key_step * kGroup) {
     float s[kGroup][2][4];
     unsigned k_addr[kGroup];   // lanes 0-7 | 8-15 | 16-23 | 24-31: 8 x 8 blocks (keys 0, depth 0) | (0, 8) | (8, 0) | (8, 8)
@@ -519,11 +530,8 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
       for (int half = 0; half < 2; ++half)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const unsigned key = key0 + half * 8 + 2 * t + (i & 1), row = row_base + g + (i >> 1) * 8;
-          bool visible = key < kv_rows;
-          if (mask_mode == 1) visible = visible && key <= row + mask_arg;
-          if (mask_mode == 2) visible = visible && key / mask_arg == row / mask_arg;
-          if (!visible) s[b][half][i] = -3.0e38f;
+          const unsigned key = key0 + half * 8 + 2 * t + (i & 1);
+          if (key < key_lo[i >> 1] || key >= key_hi[i >> 1]) s[b][half][i] = -3.0e38f;
         }
     }
     // per-row maximum over the group's keys (own values, then across the quad), one rescale of the running state
@@ -569,15 +577,11 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
     for (int b = 0; b < kGroup; ++b) {
       const unsigned key0 = base + b * key_step;
       if (key0 >= kv16) continue;
-      if (by_dims) {
-#pragma unroll
-        for (int nt = 0; nt < kDtiles; ++nt)
-          if (nt == int(warp)) {
-            const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(v_tile + (key0 + (lane & 15)) * pitch + nt * 8));
-            unsigned b0, b1;
-            asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
-            skinny_mma_bf16(out[nt], pa[b][0], pa[b][1], pa[b][2], pa[b][3], b0, b1);
-          }
+      if (by_dims) {     // this warp's value tile accumulates in out[0]
+        const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(v_tile + (key0 + (lane & 15)) * pitch + warp * 8));
+        unsigned b0, b1;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
+        skinny_mma_bf16(out[0], pa[b][0], pa[b][1], pa[b][2], pa[b][3], b0, b1);
         continue;
       }
 #pragma unroll
@@ -597,17 +601,13 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
   if (by_dims) {
     // this warp's 8 output columns of rows g, g + 8, normalised and stored from the accumulators
 #pragma unroll
-    for (int nt = 0; nt < kDtiles; ++nt)
-      if (nt == int(warp)) {
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          const unsigned row = row_base + g + hr * 8;
-          if (row >= q_rows) continue;
-          const float inv = row_sum[hr] > 0.f ? 1.f / row_sum[hr] : 0.f;
-          *reinterpret_cast<bf162*>(o + size_t(row) * o_stride + head * head_dim + nt * 8 + 2 * t) =
-              __floats2bfloat162_rn(out[nt][2 * hr] * inv, out[nt][2 * hr + 1] * inv);
-        }
-      }
+    for (int hr = 0; hr < 2; ++hr) {
+      const unsigned row = row_base + g + hr * 8;
+      if (row >= q_rows) continue;
+      const float inv = row_sum[hr] > 0.f ? 1.f / row_sum[hr] : 0.f;
+      *reinterpret_cast<bf162*>(o + size_t(row) * o_stride + head * head_dim + warp * 8 + 2 * t) =
+          __floats2bfloat162_rn(out[0][2 * hr] * inv, out[0][2 * hr + 1] * inv);
+    }
     return;
   }
 
@@ -644,6 +644,7 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
       den += weight[w] * merge[(w * 16 + r) * mp + head_dim + 1];
     }
     const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll 1
     for (unsigned d = c; d < head_dim; d += 16) {
       float num = 0.f;
 #pragma unroll
