@@ -35,6 +35,7 @@
 #pragma once
 
 #include "gemm_tc.cuh"
+#include "gemm_ts.cuh"
 
 namespace tk {
 
@@ -44,18 +45,8 @@ constexpr unsigned kMaxRing = 8;
 // kW weight warps, kW token warps (all of them: epilogue), 1 MMA warp.
 constexpr unsigned kW = 4, kMmaWarp = 2 * kW, kEpilogue = 64 * kW, kThreads = kEpilogue + 32;
 
-struct Part {
-  const uint8_t* w;
-  const bf16* bias;
-  const float* scale;
-  void* y;
-  unsigned N, ldy;
-};
+using ts::Part;
 
-// Arrives at `bar` once every cp.async this thread has issued so far has landed.
-__device__ __forceinline__ void cp_async_arrive(unsigned long long* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void tmem_load16_nowait(unsigned addr, unsigned r[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -326,7 +317,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     for (unsigned i = 0; i < nkb; ++i) {
       if (i >= stages) mbar_wait(&empty_bar[s], phase, status, kTimeoutEmpty | s);
       copy(i, s);
-      cp_async_arrive(&full_bar[s]);
+      ts::arrive_async(smem_u32(&full_bar[s]));
       if (++s == stages) { s = 0; phase ^= 1; }
     }
   };
@@ -576,9 +567,6 @@ AGI_TK_CLUSTER(agi_gemm_tcpk_e4m3, uint8_t, true, true, 6)
 AGI_TK_CLUSTER(agi_gemm_tcpk_e4m3, uint8_t, true, true, 8)
 // the names under which projections that share their input run as one launch (Q | K | V, gate | up)
 AGI_TK_KERNEL(agi_gemm_tc_bf16_x3, , bf16, false, false, false)
-AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 2)
-AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 4)
-AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 8)
 AGI_TK_KERNEL(agi_gemm_tc_e4m3_x3, , uint8_t, true, false, false)
 AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 2)
 AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 4)
