@@ -44,24 +44,43 @@ extern "C" __global__ void agi_absmax_bf16(const bf16* x, unsigned count, unsign
   if (threadIdx.x == 0) atomicMax(amax_bits, __float_as_uint(best));
 }
 
+__device__ __forceinline__ uint2 quantize8(const Bf16x8& x, const Divisor& divide) {
+  float f[8];
+  unpack8(x, f);
+  if (divide.plain) {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {     // rotates through the values: one division's code
+      const float a = __fdiv_rn(f[0], divide.y), b = __fdiv_rn(f[1], divide.y);
+      f[0] = f[2]; f[1] = f[3]; f[2] = f[4]; f[3] = f[5]; f[4] = f[6]; f[5] = f[7]; f[6] = a; f[7] = b;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = divide(f[j]);
+  }
+  return make_uint2(float4_to_e4m3x4(f[0], f[1], f[2], f[3]), float4_to_e4m3x4(f[4], f[5], f[6], f[7]));
+}
+
 // Per-tensor dynamic quantisation: scale = amax / 448 (1 when amax is 0), q = e4m3(x / scale)
-// with IEEE division and round-to-nearest-even, saturating.  Block 0 publishes `scale`.
+// to the bits of IEEE division and round-to-nearest-even, saturating.  Block 0 publishes `scale`.  Bound by latency: the first
+// values are requested beside amax and not behind it, and the quotients come from one reciprocal (`Divisor`): 77 x 2048
+// values take 1.6 us of a layer's chain, with a division per value behind amax 2.1.
 extern "C" __global__ void agi_quantize_e4m3_bf16(const bf16* x, uint8_t* q, const unsigned* amax_bits,
                                                    float* scale_out, unsigned count) {
+  const unsigned vectors = count / 8, first = blockIdx.x * blockDim.x + threadIdx.x;
+  const Bf16x8* xv = reinterpret_cast<const Bf16x8*>(x);
+  uint2* qv = reinterpret_cast<uint2*>(q);
   grid_dependency_wait();
+  // the first values are on their way while amax is
+  Bf16x8 next;
+  if (first < vectors) next = xv[first];
   const float amax = __uint_as_float(*amax_bits);
   const float scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
   if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
-  const unsigned vectors = count / 8;
-  const Bf16x8* xv = reinterpret_cast<const Bf16x8*>(x);
-  uint2* qv = reinterpret_cast<uint2*>(q);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < vectors; i += gridDim.x * blockDim.x) {
-    float f[8];
-    unpack8(xv[i], f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __fdiv_rn(f[j], scale);
-    const unsigned lo = float4_to_e4m3x4(f[0], f[1], f[2], f[3]), hi = float4_to_e4m3x4(f[4], f[5], f[6], f[7]);
-    qv[i] = make_uint2(lo, hi);
+  const Divisor divide(scale);
+#pragma unroll 1
+  for (unsigned i = first; i < vectors; i += gridDim.x * blockDim.x) {
+    if (i != first) next = xv[i];
+    qv[i] = quantize8(next, divide);
   }
   for (unsigned i = vectors * 8 + blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
     q[i] = float_to_e4m3(__fdiv_rn(__bfloat162float(x[i]), scale));
@@ -69,27 +88,27 @@ extern "C" __global__ void agi_quantize_e4m3_bf16(const bf16* x, uint8_t* q, con
 
 // The same quantisation, written in the packed operand layout of the bulk-copy tensor-core GEMM
 // ("K-block-major, swizzled"): the 128-byte K block kb of row r goes to ((kb * rows_padded + r) * 128), its
-// 16-byte chunk c to position c ^ (r & 7).  One thread converts 8 consecutive values = half a chunk: the divisions are a
-// latency chain, so more threads with less each are faster (a 288-token prefill with 33 of these launches: 781 us with 16
-// values a thread, 750 us with 8).
+// 16-byte chunk c to position c ^ (r & 7).  One thread converts 8 consecutive values = half a chunk: more threads with less
+// each are faster (a 288-token prefill with 33 of these launches: 781 us with 16 values a thread, 750 us with 8).
 // cols % 16 == 0; rows past `rows` (up to rows_padded) are left as they are: the GEMM never stores them.
 extern "C" __global__ void agi_quantize_e4m3_packed_bf16(const bf16* x, uint8_t* q, const unsigned* amax_bits,
                                                           float* scale_out, unsigned rows, unsigned cols,
                                                           unsigned rows_padded) {
+  const unsigned per_row = cols / 8, total = rows * per_row, first = blockIdx.x * blockDim.x + threadIdx.x;
+  const Bf16x8* xv = reinterpret_cast<const Bf16x8*>(x);
   grid_dependency_wait();
+  Bf16x8 next;
+  if (first < total) next = xv[first];
   const float amax = __uint_as_float(*amax_bits);
   const float scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
   if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
-  const unsigned per_row = cols / 8, total = rows * per_row;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+  const Divisor divide(scale);
+#pragma unroll 1
+  for (unsigned i = first; i < total; i += gridDim.x * blockDim.x) {
     const unsigned r = i / per_row, part = i % per_row;
-    float f[8];
-    unpack8(reinterpret_cast<const Bf16x8*>(x)[i], f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __fdiv_rn(f[j], scale);
-    const unsigned lo = float4_to_e4m3x4(f[0], f[1], f[2], f[3]), hi = float4_to_e4m3x4(f[4], f[5], f[6], f[7]);
+    if (i != first) next = xv[i];
     uint8_t* dst = q + (size_t(part >> 4) * rows_padded + r) * 128 + ((((part >> 1) & 7) ^ (r & 7)) << 4) + (part & 1) * 8;
-    *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
+    *reinterpret_cast<uint2*>(dst) = quantize8(next, divide);
   }
 }
 
@@ -109,7 +128,7 @@ __device__ __forceinline__ void swiglu_body(const bf16* gate, const bf16* up, bf
     unpack8(*reinterpret_cast<const Bf16x8*>(up + size_t(r) * in_stride + c), u);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      g[j] = silu(g[j]) * u[j];
+      g[j] = silu_bf16(g[j]) * u[j];
       if (kAmax) best = fmaxf(best, fabsf(g[j]));
     }
     *reinterpret_cast<Bf16x8*>(out + size_t(r) * out_stride + c) = pack8(g);

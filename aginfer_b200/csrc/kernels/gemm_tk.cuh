@@ -133,11 +133,11 @@ __device__ __forceinline__ float finish_tile(const float* tile, unsigned P, unsi
         unpack8(pack8(v), gr);
         unpack8(pack8(ur), ur);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = silu(gr[j]) * ur[j];
+        for (int j = 0; j < 8; ++j) v[j] = silu_bf16(gr[j]) * ur[j];
       } else if (kMode == kTimesSilu || (kGen && (o.flags & kFlagMulSilu))) {
         unpack8(pack8(v), v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] *= silu(other[j]);
+        for (int j = 0; j < 8; ++j) v[j] *= silu_bf16(other[j]);
       } else {
         if (kGen && (o.flags & kFlagActMask)) {
 #pragma unroll 1
