@@ -218,7 +218,9 @@ __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsig
   }
 }
 
-// grid = (weight tiles of all parts, token groups of `tg` rows, ranks), block = kThreads.  NB: weight rows of a tile, a
+// grid = (token groups of `tg` rows, weight tiles of all parts, ranks): the groups of a weight tile run side by side, so that
+// its weights come from HBM once (tiles first, a gate and up pair of 90 MB came in three times for 288 tokens, L2 held none of
+// it until the next group: 49 us instead of 45).  block = kThreads.  NB: weight rows of a tile, a
 // multiple of 16 (of 32 with kFlagSwiglu) up to 256; tg a multiple of 8, ceil(tg / 128) * NB' * (runs a rank takes) <=
 // 512 with NB' = NB rounded up to 32.  Dynamic shared memory: 1024 + the larger of the ring, stages * (tg + NB) * 128 plus what the last
 // slot's A tiles overhang (rows past the tokens are read by the MMA, never stored), and the epilogue's tile,
@@ -229,7 +231,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
                                      unsigned* amax_bits, unsigned* status, unsigned M, unsigned K, unsigned ldx,
                                      unsigned flags, unsigned NB, unsigned stages, unsigned tg, unsigned runs,
                                      unsigned per_run, const Part& p0,
-                                     const Part& p1, const Part& p2, unsigned tile = blockIdx.x) {
+                                     const Part& p1, const Part& p2, unsigned tile = blockIdx.y) {
   constexpr unsigned kRowStep = 4 * kW;   // rows a copy pass covers
   extern __shared__ unsigned char dynamic_smem[];
   __shared__ __align__(8) unsigned long long full_bar[kMaxRing], empty_bar[kMaxRing], accum_bar;
@@ -245,7 +247,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
   if (tile >= t0 + t1) { part = p2; tile -= t0 + t1; }
   else if (tile >= t0) { part = p1; tile -= t0; }
   const unsigned n0 = tile * nb_out;
-  const unsigned m0 = blockIdx.y * tg, rows = min(tg, M - m0), m_tiles = (rows + 127) / 128;
+  const unsigned m0 = blockIdx.x * tg, rows = min(tg, M - m0), m_tiles = (rows + 127) / 128;
   const unsigned rank = kCluster ? blockIdx.z : 0, ranks = kCluster ? gridDim.z : 1;
   const unsigned k_blocks = (K * elem) / kRowBytes;
   const unsigned run0 = rank * runs / ranks, my_runs = (rank + 1) * runs / ranks - run0;
@@ -575,7 +577,7 @@ AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 8)
 #undef AGI_TK_KERNEL
 
 // Up to 16 independent bf16 GEMMs that share the activation matrix (the K and V projections of every cross-attention
-// block over the context tokens, every block's AdaLN projection) as ONE launch: grid.x = segments * ceil(N / NB);
+// block over the context tokens, every block's AdaLN projection) as ONE launch: grid = (token groups, segments * ceil(N / NB));
 // segment s multiplies by w[s], adds bias[s] and writes y + s * seg_stride elements.
 extern "C" __global__ void __launch_bounds__(tk::kThreads, 2)
 agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsigned N, unsigned K, unsigned ldx,
@@ -587,7 +589,7 @@ agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsig
                      const bf16* b6, const bf16* b7, const bf16* b8, const bf16* b9, const bf16* b10,
                      const bf16* b11, const bf16* b12, const bf16* b13, const bf16* b14, const bf16* b15) {
   const unsigned tiles = (N + NB - 1) / NB;
-  const unsigned seg = blockIdx.x / tiles;
+  const unsigned seg = blockIdx.y / tiles;
   const bf16 *w, *b;
   switch (seg) {
     case 0: w = w0; b = b0; break;    case 1: w = w1; b = b1; break;    case 2: w = w2; b = b2; break;
@@ -599,5 +601,5 @@ agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsig
   }
   const tk::Part part = {reinterpret_cast<const uint8_t*>(w), b, nullptr, y + size_t(seg) * seg_stride, N, ldy};
   tk::body<false, false, false>(reinterpret_cast<const uint8_t*>(x), nullptr, nullptr, nullptr, nullptr, status, M, K,
-                               ldx, flags, NB, stages, tg, 1, K / 64, part, part, part, blockIdx.x % tiles);
+                               ldx, flags, NB, stages, tg, 1, K / 64, part, part, part, blockIdx.y % tiles);
 }

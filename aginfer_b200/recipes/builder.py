@@ -891,7 +891,8 @@ class RecipeBuilder:
         for i in range(3):
             w, bias, scale, y, N, ldy = parts[i] if i < len(parts) else (dummy, None, None, dummy, 0, 0)
             args += [w, bias or dummy, scale or dummy, y, U32(N), U32(ldy)]
-        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (t["tiles"], t["groups"], t.get("slices", t["C"])), (288, 1, 1), args,
+        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (t["tiles"], 1, t["slices"]) if "slices" in t
+                    else (t["groups"], t["tiles"], t["C"]), (288, 1, 1), args,
                     shared_bytes=t["shared_bytes"], op=op,
                     algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_r{t['runs']}_c{t['C']}" + (f"_x{len(parts)}" if len(parts) > 1 else ""))
 
@@ -1005,7 +1006,7 @@ class RecipeBuilder:
         dummy = Arena(0)
         ws = [p[0] for p in parts] + [dummy] * (16 - len(parts))
         bs = [p[1] for p in parts] + [dummy] * (16 - len(parts))
-        self.launch("agi_gemm_tc_bf16_x16", (t["tiles"], t["groups"], 1), (288, 1, 1),
+        self.launch("agi_gemm_tc_bf16_x16", (t["groups"], t["tiles"], 1), (288, 1, 1),
                     [x, y, Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(ldx or K), U32(N), U32(FLAG_BIAS), U32(t["NB"]),
                      U32(t["stages"]), U32(t["tg"]), U32(seg_stride), *ws, *bs], shared_bytes=t["shared_bytes"],
                     op="gemm_bf16_batch", algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_x{len(parts)}")
