@@ -30,7 +30,6 @@ enum : unsigned {
   kFlagSwiglu = 1u << 13,     // the first two matrices are gate and up of the same width: y = silu(gate) * up
   kFlagMulSilu = 1u << 14,    // y = silu(gate[m, n]) * (...), the gate (bf16, pitch of y) in place of the residual
   kFlagAmax = 1u << 15,       // fold max |y| of the rounded outputs into a zero-initialised word
-  kFlagSplit = 1u << 16,      // few-token tensor-core GEMM: leave the slices of K unadded in the fp32 scratch
 };
 
 // Programmatic dependent launch: when the loader launches with programmatic stream

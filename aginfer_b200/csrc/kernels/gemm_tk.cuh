@@ -35,7 +35,6 @@
 #pragma once
 
 #include "gemm_tc.cuh"
-#include "gemm_ts.cuh"
 
 namespace tk {
 
@@ -45,8 +44,18 @@ constexpr unsigned kMaxRing = 8;
 // kW weight warps, kW token warps (all of them: epilogue), 1 MMA warp.
 constexpr unsigned kW = 4, kMmaWarp = 2 * kW, kEpilogue = 64 * kW, kThreads = kEpilogue + 32;
 
-using ts::Part;
+struct Part {
+  const uint8_t* w;
+  const bf16* bias;
+  const float* scale;
+  void* y;
+  unsigned N, ldy;
+};
 
+// Arrives at `bar` once every cp.async this thread has issued so far has landed.
+__device__ __forceinline__ void cp_async_arrive(unsigned long long* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void tmem_load16_nowait(unsigned addr, unsigned r[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -218,9 +227,13 @@ __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsig
   }
 }
 
+// Whether the grid's first dimension is the token groups.
+__device__ __forceinline__ bool groups_first(unsigned M, unsigned tg) { return (gridDim.x - 1) * tg < M && gridDim.x * tg >= M; }
+
 // grid = (token groups of `tg` rows, weight tiles of all parts, ranks): the groups of a weight tile run side by side, so that
 // its weights come from HBM once (tiles first, a gate and up pair of 90 MB came in three times for 288 tokens, L2 held none of
-// it until the next group: 49 us instead of 45).  block = kThreads.  NB: weight rows of a tile, a
+// it until the next group: 49 us instead of 45).  One group, or more tiles than fit the second dimension: grid = (weight
+// tiles, token groups, ranks).  block = kThreads.  NB: weight rows of a tile, a
 // multiple of 16 (of 32 with kFlagSwiglu) up to 256; tg a multiple of 8, ceil(tg / 128) * NB' * (runs a rank takes) <=
 // 512 with NB' = NB rounded up to 32.  Dynamic shared memory: 1024 + the larger of the ring, stages * (tg + NB) * 128 plus what the last
 // slot's A tiles overhang (rows past the tokens are read by the MMA, never stored), and the epilogue's tile,
@@ -231,7 +244,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
                                      unsigned* amax_bits, unsigned* status, unsigned M, unsigned K, unsigned ldx,
                                      unsigned flags, unsigned NB, unsigned stages, unsigned tg, unsigned runs,
                                      unsigned per_run, const Part& p0,
-                                     const Part& p1, const Part& p2, unsigned tile = blockIdx.y) {
+                                     const Part& p1, const Part& p2, unsigned tile) {
   constexpr unsigned kRowStep = 4 * kW;   // rows a copy pass covers
   extern __shared__ unsigned char dynamic_smem[];
   __shared__ __align__(8) unsigned long long full_bar[kMaxRing], empty_bar[kMaxRing], accum_bar;
@@ -247,7 +260,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
   if (tile >= t0 + t1) { part = p2; tile -= t0 + t1; }
   else if (tile >= t0) { part = p1; tile -= t0; }
   const unsigned n0 = tile * nb_out;
-  const unsigned m0 = blockIdx.x * tg, rows = min(tg, M - m0), m_tiles = (rows + 127) / 128;
+  const unsigned m0 = (groups_first(M, tg) ? blockIdx.x : blockIdx.y) * tg, rows = min(tg, M - m0), m_tiles = (rows + 127) / 128;
   const unsigned rank = kCluster ? blockIdx.z : 0, ranks = kCluster ? gridDim.z : 1;
   const unsigned k_blocks = (K * elem) / kRowBytes;
   const unsigned run0 = rank * runs / ranks, my_runs = (rank + 1) * runs / ranks - run0;
@@ -319,7 +332,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     for (unsigned i = 0; i < nkb; ++i) {
       if (i >= stages) mbar_wait(&empty_bar[s], phase, status, kTimeoutEmpty | s);
       copy(i, s);
-      ts::arrive_async(smem_u32(&full_bar[s]));
+      cp_async_arrive(&full_bar[s]);
       if (++s == stages) { s = 0; phase ^= 1; }
     }
   };
@@ -544,7 +557,8 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     const tk::Part p1 = {reinterpret_cast<const uint8_t*>(w1), bias1, sw1, y1, N1, ldy1};                            \
     const tk::Part p2 = {reinterpret_cast<const uint8_t*>(w2), bias2, sw2, y2, N2, ldy2};                            \
     tk::body<FP8, PACKED, IN_CLUSTER>(reinterpret_cast<const uint8_t*>(x), scale_a, other, partial, amax_bits,       \
-                                         status, M, K, ldx, flags, NB, stages, tg, runs, per_run, p0, p1, p2);       \
+                                         status, M, K, ldx, flags, NB, stages, tg, runs, per_run, p0, p1, p2,         \
+                                         tk::groups_first(M, tg) ? blockIdx.y : blockIdx.x);                                         \
   }
 // The ranks that share K: grid z = C.  Up to 15 clusters of 8, 33 of 4, 74 of 2 are resident at once.
 #define AGI_TK_CLUSTER(NAME, TYPE, FP8, PACKED, C) AGI_TK_KERNEL(NAME##_c##C, __cluster_dims__(1, 1, C), TYPE, FP8, PACKED, true)
@@ -569,6 +583,9 @@ AGI_TK_CLUSTER(agi_gemm_tcpk_e4m3, uint8_t, true, true, 6)
 AGI_TK_CLUSTER(agi_gemm_tcpk_e4m3, uint8_t, true, true, 8)
 // the names under which projections that share their input run as one launch (Q | K | V, gate | up)
 AGI_TK_KERNEL(agi_gemm_tc_bf16_x3, , bf16, false, false, false)
+AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 2)
+AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 4)
+AGI_TK_CLUSTER(agi_gemm_tc_bf16_x3, bf16, false, false, 8)
 AGI_TK_KERNEL(agi_gemm_tc_e4m3_x3, , uint8_t, true, false, false)
 AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 2)
 AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 4)
@@ -589,7 +606,7 @@ agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsig
                      const bf16* b6, const bf16* b7, const bf16* b8, const bf16* b9, const bf16* b10,
                      const bf16* b11, const bf16* b12, const bf16* b13, const bf16* b14, const bf16* b15) {
   const unsigned tiles = (N + NB - 1) / NB;
-  const unsigned seg = blockIdx.y / tiles;
+  const unsigned at = tk::groups_first(M, tg) ? blockIdx.y : blockIdx.x, seg = at / tiles;
   const bf16 *w, *b;
   switch (seg) {
     case 0: w = w0; b = b0; break;    case 1: w = w1; b = b1; break;    case 2: w = w2; b = b2; break;
@@ -601,5 +618,5 @@ agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsig
   }
   const tk::Part part = {reinterpret_cast<const uint8_t*>(w), b, nullptr, y + size_t(seg) * seg_stride, N, ldy};
   tk::body<false, false, false>(reinterpret_cast<const uint8_t*>(x), nullptr, nullptr, nullptr, nullptr, status, M, K,
-                               ldx, flags, NB, stages, tg, 1, K / 64, part, part, part, blockIdx.y % tiles);
+                               ldx, flags, NB, stages, tg, 1, K / 64, part, part, part, at % tiles);
 }

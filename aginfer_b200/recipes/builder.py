@@ -30,7 +30,7 @@ SM_COUNT = 148
 
 FLAG_BIAS, FLAG_RESIDUAL, FLAG_OUT_F32, FLAG_SCALED = 1, 2, 1 << 8, 1 << 9
 FLAG_LAYERNORM, FLAG_LN_MODULATE, FLAG_SLAB = 1 << 10, 1 << 11, 1 << 12
-FLAG_SWIGLU, FLAG_MUL_SILU, FLAG_AMAX, FLAG_SPLIT = 1 << 13, 1 << 14, 1 << 15, 1 << 16
+FLAG_SWIGLU, FLAG_MUL_SILU, FLAG_AMAX = 1 << 13, 1 << 14, 1 << 15
 ACT = {None: 0, "gelu_tanh": 1 << 4, "silu": 2 << 4, "relu": 3 << 4}
 PLAN_DTYPE_BYTES = {"F32": 4, "F16": 2, "BF16": 2, "F8_E4M3": 1, "I32": 4}
 
@@ -330,37 +330,10 @@ def tcs_tiling(M: int, tiles: int, K: int, cluster: int | None = None, groups: i
             "shared_bytes": kb * 20480 + 1024 + gather}
 
 
-# ---- few tokens on the tensor core (csrc/kernels/gemm_ts.cuh) -----------------------------------------------
-TS_MAX_TOKENS = 64
-TS_RANKS = (1, 2, 3, 4, 6, 8)                     # compiled cluster sizes
-TS_MAX_SLICES = 8                                 # slices whose partial tiles the next launch adds
-TS_SMEM = 111 * 1024                              # a CTA and its successor's share an SM: the successor's weights land early
-
-
-def ts_tiling(M: int, widths: Sequence[int], K: int, elem: int, *, swiglu: bool = False, split: bool = False,
-              rows: int | None = None, slices: int | None = None, smem: int = TS_SMEM) -> dict[str, int] | None:
-    """Geometry of the ``agi_gemm_ts_*``, under the names of ``tk_tiling``: weight rows of a tile, the slices
-    of K of a tile (a cluster of ``C``, or, ``split``, left unadded) and the ring depth.  ``rows`` / ``slices`` fix them."""
-    if M > TS_MAX_TOKENS or (K * elem) % 128:
-        return None
-    k_blocks, held = K * elem // 128, ceil_div(M, 8) * 8
-    best = None
-    for TR in ((rows,) if rows else (64, 128)):
-        tiles = sum(ceil_div(n, TR // 2 if swiglu else TR) for n in widths)
-        for S in ((slices,) if slices else range(1, TS_MAX_SLICES + 1) if split else TS_RANKS):
-            if S > k_blocks or (S > 1 and tiles * S > SM_COUNT):
-                continue
-            per, block, TN = ceil_div(k_blocks, S), (TR + held) * 128, held if TR == 64 else ceil_div(M, 16) * 16
-            gather = 0 if split else S * ceil_div(M, S) * TR * 4
-            room = max(2, min(per, (smem - 2048 - gather) // block))          # K blocks that the ring holds
-            depth = per if room == per and per <= 4 else max(1, min(4, room // 2)) if room < 8 else min(4, room // 3)
-            stages = min(12, room // depth if room < per else ceil_div(per, depth))
-            cost = ceil_div(tiles * S, SM_COUNT) * per * max(4 * max(25 if TR == 64 else 41, TN // 2), TR * 128 // 25)
-            cost += S * 125 if split else 0 if S == 1 else 700 + 130 * S
-            if best is None or cost < best["cost"]:
-                best = {"C": 1 if split else S, "slices": S, "NB": TR, "tg": TN, "tiles": tiles, "groups": 1, "stages": stages, "runs": S,
-                        "per_run": depth, "shared_bytes": 2048 + max(stages * depth * block, M * TR * 4) + gather, "cost": cost}
-    return best
+def tk_grid(t: Mapping[str, int]) -> tuple[int, int]:
+    """Token groups of a weight tile side by side, unless there is one or the tiles do not fit the grid's second dimension."""
+    tiles, groups = t["tiles"], t["groups"]
+    return (tiles, groups) if groups == 1 or tiles > 65535 else (groups, tiles)
 
 
 STREAM_SPLITS = (4, 2)          # compiled cluster sizes of agi_gemm_stream_bf16_t{1..4}_k{S}
@@ -880,19 +853,17 @@ class RecipeBuilder:
     def _gemm_tk(self, family: str, op: str, t: Mapping[str, int], x: Pointer,
                  parts: Sequence[tuple[Pointer, Pointer | None, Pointer | None, Pointer, int, int]], M: int, K: int, ldx: int,
                  flags: int, *, scale_a: Pointer | None = None, other: Pointer | None = None,
-                 amax: Pointer | None = None, scratch: Pointer | None = None) -> None:
+                 amax: Pointer | None = None) -> None:
         """One launch of ``agi_gemm_tk_*`` (or a family with the same parameters) with the tile ``t``.
-        ``parts``: (weight, bias, weight scale, y, N, ldy); ``other``: residual, or the gate of FLAG_MUL_SILU;
-        ``scratch``: where partial tiles go, by default the common scratch."""
+        ``parts``: (weight, bias, weight scale, y, N, ldy); ``other``: residual, or the gate of FLAG_MUL_SILU."""
         dummy = Arena(0)
-        args: list[Any] = [x, scale_a or dummy, other or dummy, scratch or self._tc_scratch[0], amax or dummy, Arena(STATUS_WORD),
-                           U32(M), U32(K), U32(ldx), U32(flags | (FLAG_AMAX if amax is not None else 0)), U32(t["NB"]),
+        args: list[Any] = [x, scale_a or dummy, other or dummy, self._tc_scratch[0], amax or dummy, Arena(STATUS_WORD), U32(M),
+                           U32(K), U32(ldx), U32(flags | (FLAG_AMAX if amax is not None else 0)), U32(t["NB"]),
                            U32(t["stages"]), U32(t["tg"]), U32(t["runs"]), U32(t["per_run"])]
         for i in range(3):
             w, bias, scale, y, N, ldy = parts[i] if i < len(parts) else (dummy, None, None, dummy, 0, 0)
             args += [w, bias or dummy, scale or dummy, y, U32(N), U32(ldy)]
-        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (t["tiles"], 1, t["slices"]) if "slices" in t
-                    else (t["groups"], t["tiles"], t["C"]), (288, 1, 1), args,
+        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (*tk_grid(t), t["C"]), (288, 1, 1), args,
                     shared_bytes=t["shared_bytes"], op=op,
                     algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_r{t['runs']}_c{t['C']}" + (f"_x{len(parts)}" if len(parts) > 1 else ""))
 
@@ -915,13 +886,11 @@ class RecipeBuilder:
         widths = tuple(p[4] for p in parts)
         family = "agi_gemm_tcpk_e4m3" if packed else f"agi_gemm_tc_{dtype}_x3"
         c = tc_cluster_tiling(M, 128 * sum(ceil_div(n, 128) for n in widths), K, elem, dtype, sizes=(2, 4, 8))
-        if dtype == "bf16" and M <= TS_MAX_TOKENS and c is not None:
+        if dtype == "bf16" and M <= 64 and c is not None:
             # few tokens: 128-row tiles would leave most SMs idle, so the K slices of every tile form a cluster
-            t = ts_tiling(M, widths, K, elem, rows=128, slices=c["cluster"])
+            t = tk_tiling(M, widths, K, elem, clusters=(c["cluster"],), rows_per_tile=128)
         else:
             t = tk_tiling(M, widths, K, elem, runs=runs, clusters=TK_CLUSTERS[family] if split and runs is None else (1,))
-            if dtype == "bf16" and t["C"] > 1:
-                family = "agi_gemm_tk_bf16"
         self._gemm_tk(family, f"gemm_{dtype}_group" + ("_packed" if packed else ""), t, x,
                       [(w, bias, sw, y, N, ldy) for w, bias, sw, y, N, ldy in parts], M, K,
                       padded_token_rows(M) if packed else (ldx or K), flags, scale_a=scale_a)
@@ -946,56 +915,15 @@ class RecipeBuilder:
                           scale_a=scale_a, other=scratch, amax=amax)
             return
         family = "agi_gemm_tcpk_e4m3" if packed else f"agi_gemm_tc_{dtype}_x3"
-        if dtype == "bf16" and M <= TS_MAX_TOKENS:
+        if dtype == "bf16" and M <= 64:
             c = tc_cluster_tiling(M, 2 * 128 * ceil_div(I, 128), K, elem, dtype, sizes=(2, 4, 8))
-            t = (ts_tiling(M, (I,), K, elem, swiglu=True, rows=128, slices=c["cluster"]) if c is not None
-                 else tk_tiling(M, (I,), K, elem, swiglu=True, clusters=(1,)))
+            t = tk_tiling(M, (I,), K, elem, swiglu=True, clusters=(c["cluster"] if c is not None else 1,))
         elif packed and not runs:
             t = tk_tiling(M, (I,), K, elem, swiglu=True)
         else:
             t = tk_tiling(M, (I,), K, elem, swiglu=True, runs=runs or 1, clusters=TK_CLUSTERS[family] if packed else (1,))
         self._gemm_tk(family, f"gemm_{dtype}_swiglu", t, x, [(*gate, out, I, I), (*up, out, I, I)], M, K, ldx,
                       flags | FLAG_SWIGLU, scale_a=scale_a, amax=amax)
-
-    def gemm_split(self, x: Pointer, weights: Sequence[tuple[Pointer, int]], partial: Pointer, M: int, K: int,
-                   ldx: int | None = None, **tile: int) -> tuple[int, int]:
-        """The slices of K of ``x . [W0 | W1 | W2]^T`` (up to three (matrix, rows), bf16, at most 64 tokens), unadded in fp32:
-        ``partial`` [slice][tile of features][token][tile], which the launch that reads the product adds (``layernorm_sum``,
-        ``rmsnorm_sum``).  Returns (slices, tile)."""
-        t = ts_tiling(M, [n for _, n in weights], K, 2, split=True, **tile)
-        assert t is not None and ((ldx or K) * 2) % 16 == 0
-        self._gemm_tk("agi_gemm_ts_bf16", "gemm_bf16_split", t, x, [(w, None, None, Arena(0), n, n) for w, n in weights], M, K,
-                      ldx or K, FLAG_SPLIT, scratch=partial)
-        return t["slices"], t["NB"]
-
-    def gemm_few(self, x: Pointer, parts: Sequence[tuple[Pointer, Pointer | None, Pointer, int, int]], M: int, K: int, *,
-                 act: str | None = None, residual: Pointer | None = None, ldx: int | None = None, **tile: int) -> None:
-        """Up to three bf16 products over one activation matrix of at most 64 tokens, (weight, bias or None, y, N, ldy): the
-        few-token tensor-core GEMM, the slices of K of a tile in a cluster."""
-        t = ts_tiling(M, [p[3] for p in parts], K, 2, **tile)
-        assert t is not None and ((ldx or K) * 2) % 16 == 0 and len({p[1] is None for p in parts}) == 1
-        flags = ACT[act] | (FLAG_BIAS if parts[0][1] is not None else 0) | (FLAG_RESIDUAL if residual else 0)
-        self._gemm_tk("agi_gemm_ts_bf16", "gemm_bf16_few", t, x, [(w, b, None, y, n, ldy) for w, b, y, n, ldy in parts], M, K,
-                      ldx or K, flags, other=residual)
-
-    def layernorm_sum(self, residual: Pointer, partial: Pointer, bias: Pointer | None, out: Pointer, y: Pointer, rows: int, cols: int,
-                      slices: tuple[int, int], eps: float = 1e-5, scale: Pointer | None = None, shift: Pointer | None = None,
-                      static_modulation: bool = False) -> None:
-        """``out = residual + bias + sum of a split product's slices`` (``gemm_split``), ``y = layernorm(out)``."""
-        assert cols % 128 == 0 and cols <= 2048 and slices[0] <= TS_MAX_SLICES
-        dummy = Arena(0)
-        flags = (1 if bias is not None else 0) | (0 if scale is None else 6 if static_modulation else 2)
-        self.launch("agi_layernorm_sum_bf16", (rows, 1, 1), (cols // 4, 1, 1),
-                    [residual, partial, bias or dummy, scale or dummy, shift or dummy, out, y, U32(rows), U32(cols), U32(slices[0]),
-                     U32(slices[1]), F32(eps), U32(flags)], op="layernorm_sum")
-
-    def rmsnorm_sum(self, residual: Pointer, partial: Pointer, bias: Pointer | None, gain: Pointer, out: Pointer, y: Pointer, rows: int,
-                    cols: int, slices: tuple[int, int], eps: float = 1e-6) -> None:
-        """``out = residual + bias + sum of a split product's slices``, ``y = rmsnorm(out) * gain``."""
-        assert cols % 128 == 0 and cols <= 2048 and slices[0] <= TS_MAX_SLICES
-        self.launch("agi_rmsnorm_sum_bf16", (rows, 1, 1), (cols // 4, 1, 1),
-                    [residual, partial, bias or Arena(0), gain, out, y, U32(rows), U32(cols), U32(slices[0]), U32(slices[1]), F32(eps),
-                     U32(1 if bias is not None else 0)], op="rmsnorm_sum")
 
     def gemm_batch(self, x: Pointer, parts: Sequence[tuple[Pointer, Pointer]], y: Pointer, M: int, N: int, K: int,
                    seg_stride: int, ldx: int | None = None) -> None:
@@ -1006,7 +934,7 @@ class RecipeBuilder:
         dummy = Arena(0)
         ws = [p[0] for p in parts] + [dummy] * (16 - len(parts))
         bs = [p[1] for p in parts] + [dummy] * (16 - len(parts))
-        self.launch("agi_gemm_tc_bf16_x16", (t["groups"], t["tiles"], 1), (288, 1, 1),
+        self.launch("agi_gemm_tc_bf16_x16", (*tk_grid(t), 1), (288, 1, 1),
                     [x, y, Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(ldx or K), U32(N), U32(FLAG_BIAS), U32(t["NB"]),
                      U32(t["stages"]), U32(t["tg"]), U32(seg_stride), *ws, *bs], shared_bytes=t["shared_bytes"],
                     op="gemm_bf16_batch", algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_x{len(parts)}")

@@ -23,8 +23,7 @@ from __future__ import annotations
 from dataclasses import dataclass, replace
 from typing import Mapping, Sequence
 
-from .builder import (TS_MAX_SLICES, TS_MAX_TOKENS, Arena, F32, RecipeBuilder, Tensor, U32, Weight, dit_block_geometry, io,
-                      grid_for)
+from .builder import Arena, F32, RecipeBuilder, Tensor, U32, Weight, dit_block_geometry, io, grid_for
 
 
 @dataclass(frozen=True)
@@ -271,21 +270,6 @@ def _emit_chunk(r: RecipeBuilder, cfg: DitConfig, profile: str | None, gemm_tact
             r.store_pointers(table, l * 16, row)
         cross_mask = sum(1 << l for l in range(cfg.layers) if cfg.is_cross(l))
 
-    # Few tokens: the products in front of a norm leave the slices of a split K to it.
-    blocks = [f"{P}.dit.blocks.{l}" for l in range(cfg.layers)]
-    few = (fuse and gemm_tactic == "auto" and not block_kernel and T <= TS_MAX_TOKENS and D % 128 == 0 and D <= 2048 and cfg.mlp % 64 == 0
-           and not any(r.is_packed(Weight(n)) for n in packed_names(cfg)))
-    part_sums = r.alloc(TS_MAX_SLICES * T * D * 4) if few else None
-
-    def few_gemms(l: int, attend, norm) -> tuple[int, int]:
-        """The four products of block ``l`` for few tokens, with what runs between them; the last one's slices are unadded."""
-        b, names = blocks[l], ["attn.to_q"] if cfg.is_cross(l) else ["attn.to_q", "attn.to_k", "attn.to_v"]
-        r.gemm_few(h, [(Weight(f"{b}.{n}.weight"), Weight(f"{b}.{n}.bias"), qkv + i * D * BF, D, 3 * D) for i, n in enumerate(names)], T, D)
-        attend()
-        norm(r.gemm_split(attn, [(Weight(f"{b}.attn.to_out.weight"), D)], part_sums, T, D))
-        r.gemm_few(h, [(Weight(f"{b}.ff.fc1.weight"), Weight(f"{b}.ff.fc1.bias"), ff, cfg.mlp, cfg.mlp)], T, D, act="gelu_tanh")
-        return r.gemm_split(ff, [(Weight(f"{b}.ff.fc2.weight"), D)], part_sums, T, cfg.mlp)
-
     for step in range(S):
         mod_row = step * 2 * D * BF       # this step's (scale | shift) row inside each mods[l]
         # action encoder: tokens 1..H of the sequence
@@ -302,51 +286,30 @@ def _emit_chunk(r: RecipeBuilder, cfg: DitConfig, profile: str | None, gemm_tact
             r.dit_blocks(table, seq, qkv, attn, ff, layers=cfg.layers, T=T, D=D, heads=cfg.heads, head_dim=cfg.head_dim,
                          mlp=cfg.mlp, ctx=cfg.backbone_tokens, cross_mask=cross_mask, mod_offset=step * 2 * D,
                          eps=cfg.ln_eps)
-        def attend(l: int) -> None:
-            # the context keys / values were projected before this step's position-embedding add (a launch that
-            # releases its successors only after its own wait): safe to request ahead of the dependency wait
-            k_buf, v_buf, kv_rows, kv_stride = ((*kv[l], cfg.backbone_tokens, D) if cfg.is_cross(l)
-                                                else (qkv + D * BF, qkv + 2 * D * BF, T, 3 * D))
-            r.attention(qkv, k_buf, v_buf, attn, q_rows=T, kv_rows=kv_rows, q_heads=cfg.heads, kv_heads=cfg.heads,
-                        head_dim=cfg.head_dim, q_stride=3 * D, k_stride=kv_stride, v_stride=kv_stride, o_stride=D,
-                        kv_static=cfg.is_cross(l))
-
-        down = None       # slices of the last down projection that are still to be added
-
-        def modulated_norm(l: int) -> None:
-            """``h`` = the AdaLN of the residual stream in front of block ``l`` (or of the output projection)."""
-            ln = dict(scale=mods[l] + mod_row, shift=mods[l] + (mod_row + D * BF), static_modulation=True)
-            if down is None:
-                r.layernorm(seq, h, T, D, cfg.ln_eps, **ln)
-            else:
-                r.layernorm_sum(seq, part_sums, Weight(f"{blocks[l - 1]}.ff.fc2.bias"), seq, h, T, D, down, cfg.ln_eps, **ln)
-
-        for l in range(cfg.layers if few else 0):
-            modulated_norm(l)
-            down = few_gemms(l, lambda: attend(l), lambda slices: r.layernorm_sum(
-                seq, part_sums, Weight(f"{blocks[l]}.attn.to_out.bias"), seq, h, T, D, slices, cfg.ln_eps))
-        for l in range(0 if block_kernel or few else cfg.layers):
+        for l in range(0 if block_kernel else cfg.layers):
             b = f"{P}.dit.blocks.{l}"
             adaln = {"eps": cfg.ln_eps, "scale": mods[l] + mod_row, "shift": mods[l] + (mod_row + D * BF), "static": True}
             part = lambda name, n: (Weight(f"{b}.{name}.weight"), Weight(f"{b}.{name}.bias"), n)
             if cfg.is_cross(l):
                 r.fused_linear(seq, [part("attn.to_q", D)], qkv, T, D, ln=adaln, ln_scratch=h, ldy=3 * D, fuse=fuse)
+                k_buf, v_buf, kv_rows, kv_stride = (*kv[l], cfg.backbone_tokens, D)
             else:
                 r.fused_linear(seq, [part("attn.to_q", D), part("attn.to_k", D), part("attn.to_v", D)], qkv, T, D,
                                ln=adaln, ln_scratch=h, ldy=3 * D, fuse=fuse)
-            attend(l)
+                k_buf, v_buf, kv_rows, kv_stride = qkv + D * BF, qkv + 2 * D * BF, T, 3 * D
+            # the context keys / values were projected before this step's position-embedding add (a launch that
+            # releases its successors only after its own wait): safe to request ahead of the dependency wait
+            r.attention(qkv, k_buf, v_buf, attn, q_rows=T, kv_rows=kv_rows, q_heads=cfg.heads, kv_heads=cfg.heads,
+                        head_dim=cfg.head_dim, q_stride=3 * D, k_stride=kv_stride, v_stride=kv_stride, o_stride=D,
+                        kv_static=cfg.is_cross(l))
             lin(attn, f"{b}.attn.to_out", seq, T, D, D, residual=seq)
             r.fused_linear(seq, [part("ff.fc1", cfg.mlp)], ff, T, D, ln={"eps": cfg.ln_eps}, ln_scratch=h,
                            act="gelu_tanh", fuse=fuse)
             lin(ff, f"{b}.ff.fc2", seq, T, D, cfg.mlp, residual=seq)
 
-        if few:
-            modulated_norm(cfg.layers)
-            lin(h, f"{P}.dit.proj_out", out_hid, T, cfg.out_dim, D)
-        else:
-            r.fused_linear(seq, [(Weight(f"{P}.dit.proj_out.weight"), Weight(f"{P}.dit.proj_out.bias"), cfg.out_dim)],
-                           out_hid, T, D, ln={"eps": cfg.ln_eps, "scale": mods[cfg.layers] + mod_row,
-                                              "shift": mods[cfg.layers] + (mod_row + D * BF), "static": True}, ln_scratch=h, fuse=fuse)
+        r.fused_linear(seq, [(Weight(f"{P}.dit.proj_out.weight"), Weight(f"{P}.dit.proj_out.bias"), cfg.out_dim)],
+                       out_hid, T, D, ln={"eps": cfg.ln_eps, "scale": mods[cfg.layers] + mod_row,
+                                          "shift": mods[cfg.layers] + (mod_row + D * BF), "static": True}, ln_scratch=h, fuse=fuse)
         lin(out_hid + cfg.out_dim * BF, f"{P}.action_decoder.fc1", dec_hid, H, cfg.encoder_hidden, cfg.out_dim, act="relu")
         lin(dec_hid, f"{P}.action_decoder.fc2", velocity, H, cfg.action_dim, cfg.encoder_hidden)
         elementwise("agi_euler_step", [x_f32, velocity, x_bf, F32(1.0 / S), U32(H * cfg.action_dim)],
@@ -380,9 +343,7 @@ def _emit_chunk(r: RecipeBuilder, cfg: DitConfig, profile: str | None, gemm_tact
         # left out; activations are whatever the arena holds).  Timing it gives the
         # weight-streaming rate of the dominant kernel in isolation.
         r.begin_profile("gemm_stream", [io("token", "I32", [1])], [io("status", "I32", [1])])
-        for l in range(cfg.layers if few else 0):
-            few_gemms(l, lambda: None, lambda slices: None)
-        for l in range(0 if few else cfg.layers):
+        for l in range(cfg.layers):
             b = f"{P}.dit.blocks.{l}"
             part = lambda name, n: (Weight(f"{b}.{name}.weight"), Weight(f"{b}.{name}.bias"), n)
             names = ["attn.to_q"] if cfg.is_cross(l) else ["attn.to_q", "attn.to_k", "attn.to_v"]
