@@ -227,8 +227,8 @@ __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsig
   }
 }
 
-// Whether the grid's first dimension is the token groups.
-__device__ __forceinline__ bool groups_first(unsigned M, unsigned tg) { return (gridDim.x - 1) * tg < M && gridDim.x * tg >= M; }
+// Whether the grid's first dimension is the token groups (never more than 65535): the builder's `tk_grid`.
+__device__ __forceinline__ bool groups_first(unsigned M, unsigned tg) { return M > tg && gridDim.x <= 65535; }
 
 // grid = (token groups of `tg` rows, weight tiles of all parts, ranks): the groups of a weight tile run side by side, so that
 // its weights come from HBM once (tiles first, a gate and up pair of 90 MB came in three times for 288 tokens, L2 held none of

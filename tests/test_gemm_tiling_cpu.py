@@ -3,7 +3,7 @@ function of the shape alone."""
 import pytest
 
 from aginfer_b200.recipes import RecipeBuilder, Tensor, qwen_vl
-from aginfer_b200.recipes.builder import TC_SCRATCH_BYTES, TK_CLUSTERS, k_runs, tk_tiling
+from aginfer_b200.recipes.builder import TC_SCRATCH_BYTES, TK_CLUSTERS, k_runs, tk_grid, tk_tiling
 from aginfer_b200.recipes.package import describe
 
 SHAPES = [(16, 128), (130, 256), (2048, 2048), (11008, 2048), (2048, 11008), (3584, 18944), (151, 640)]
@@ -113,3 +113,9 @@ def test_the_order_of_the_sum_over_k_is_the_recorded_one(shape):
             found.append(f"{M}:{runs}")
         last = runs
     assert " ".join(found) == K_RUNS[shape]
+
+
+@pytest.mark.parametrize("tiles,groups,grid", [(96, 1, (96, 1)), (96, 3, (3, 96)), (1, 4, (4, 1)), (65535, 2, (2, 65535)),
+                                               (65536, 2, (65536, 2)), (70000, 1, (70000, 1))])
+def test_token_groups_run_side_by_side_where_the_grid_takes_the_tiles(tiles, groups, grid):
+    assert tk_grid({"tiles": tiles, "groups": groups}) == grid
