@@ -26,20 +26,31 @@ extern "C" __global__ void agi_copy_u32(const unsigned* in, unsigned* out, unsig
 
 // amax_bits = max(amax_bits, bits(max |x|)).  Non-negative floats order like their bit
 // patterns, so an integer atomicMax on a zero-initialised word accumulates the maximum.
+// Pairs of bf16 are compared as they are: exact, and NaN loses as in fmaxf.  Bound by the latency of its loads, so four are
+// in flight a thread and not one.
 extern "C" __global__ void agi_absmax_bf16(const bf16* x, unsigned count, unsigned* amax_bits) {
   __shared__ float scratch[32];
+  const unsigned vectors = count / 8, step = gridDim.x * blockDim.x;
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
+  unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   grid_dependency_wait();
-  float best = 0.f;
-  const unsigned vectors = count / 8;
-  const Bf16x8* xv = reinterpret_cast<const Bf16x8*>(x);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < vectors; i += gridDim.x * blockDim.x) {
-    float f[8];
-    unpack8(xv[i], f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) best = fmaxf(best, fabsf(f[j]));
+  bf162 top = __float2bfloat162_rn(0.f);
+  auto fold = [&](const uint4& v) {
+    const bf162* p = reinterpret_cast<const bf162*>(&v);
+    top = __hmax2(top, __hmax2(__hmax2(__habs2(p[0]), __habs2(p[1])), __hmax2(__habs2(p[2]), __habs2(p[3]))));
+  };
+#pragma unroll 1
+  for (; i + 3 * step < vectors; i += 4 * step) {
+    const uint4 a = xv[i], b = xv[i + step], c = xv[i + 2 * step], d = xv[i + 3 * step];
+    fold(a); fold(b); fold(c); fold(d);
   }
-  for (unsigned i = vectors * 8 + blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    best = fmaxf(best, fabsf(__bfloat162float(x[i])));
+  uint4 rest[3];      // at most three more
+#pragma unroll
+  for (unsigned j = 0; j < 3; ++j) rest[j] = i + j * step < vectors ? xv[i + j * step] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (unsigned j = 0; j < 3; ++j) fold(rest[j]);
+  float best = fmaxf(__low2float(top), __high2float(top));
+  for (i = vectors * 8 + blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) best = fmaxf(best, fabsf(__bfloat162float(x[i])));
   best = block_max(best, scratch);
   if (threadIdx.x == 0) atomicMax(amax_bits, __float_as_uint(best));
 }
