@@ -227,7 +227,8 @@ __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsig
   }
 }
 
-// Whether the grid's first dimension is the token groups (never more than 65535): the builder's `tk_grid`.
+// Whether the grid's first dimension is the token groups: the builder's `tk_grid`.  It puts groups first only where neither
+// they nor the tiles are more than 65535; more groups stand in the second dimension, where no launch takes them.
 __device__ __forceinline__ bool groups_first(unsigned M, unsigned tg) { return M > tg && gridDim.x <= 65535; }
 
 // grid = (token groups of `tg` rows, weight tiles of all parts, ranks): the groups of a weight tile run side by side, so that

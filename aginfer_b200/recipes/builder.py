@@ -330,10 +330,15 @@ def tcs_tiling(M: int, tiles: int, K: int, cluster: int | None = None, groups: i
             "shared_bytes": kb * 20480 + 1024 + gather}
 
 
+GRID_SECOND = 65535          # the most a grid's second and third dimensions take
+
+
 def tk_grid(t: Mapping[str, int]) -> tuple[int, int]:
-    """Token groups of a weight tile side by side, unless there is one or the tiles do not fit the grid's second dimension."""
+    """Token groups of a weight tile side by side, unless there is one, or the second dimension does not take the tiles, or
+    it would not take the groups either: the kernel tells the order from a first dimension of at most 65535, so more groups
+    than that stay where a launch refuses them."""
     tiles, groups = t["tiles"], t["groups"]
-    return (tiles, groups) if groups == 1 or tiles > 65535 else (groups, tiles)
+    return (tiles, groups) if groups == 1 or tiles > GRID_SECOND or groups > GRID_SECOND else (groups, tiles)
 
 
 STREAM_SPLITS = (4, 2)          # compiled cluster sizes of agi_gemm_stream_bf16_t{1..4}_k{S}

@@ -116,6 +116,20 @@ def test_the_order_of_the_sum_over_k_is_the_recorded_one(shape):
 
 
 @pytest.mark.parametrize("tiles,groups,grid", [(96, 1, (96, 1)), (96, 3, (3, 96)), (1, 4, (4, 1)), (65535, 2, (2, 65535)),
-                                               (65536, 2, (65536, 2)), (70000, 1, (70000, 1))])
+                                               (65536, 2, (65536, 2)), (70000, 1, (70000, 1)), (1, 65535, (65535, 1)),
+                                               (1, 65536, (1, 65536)), (16, 65792, (16, 65792)), (65535, 89241, (65535, 89241)),
+                                               (70000, 70000, (70000, 70000))])
 def test_token_groups_run_side_by_side_where_the_grid_takes_the_tiles(tiles, groups, grid):
     assert tk_grid({"tiles": tiles, "groups": groups}) == grid
+
+
+def test_more_token_groups_than_a_grid_takes_stay_where_the_launch_refuses_them():
+    M, N, K, y = 33554432, 64, 64, Tensor("y")
+    r = RecipeBuilder({"w": ("BF16", [8])})
+    r.begin_profile("default", [], [])
+    before = r.launch_count()
+    r.gemm(y, y, y, M, N, K)
+    r.gemm_group(y, [(y, None, None, y, N, N)] * 2, M, K)
+    r.gemm_batch(y, [(y, y)] * 2, y, M, N, K, seg_stride=M * N)
+    launches = r.profiles[0].launches[before:]
+    assert len(launches) == 3 and all(l["grid"][0] <= 4 and l["grid"][1] > 65535 for l in launches)
