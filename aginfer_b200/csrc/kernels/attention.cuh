@@ -478,14 +478,15 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[nt][i] = 0.f;
   const unsigned dtiles = 2 * ksteps;      // <= kDtiles
-  // Keys that rows g, g + 8 may see are one range each, worked out once: a division per score is 15 KB of code for a launch
-  // that runs it once, and instructions that are fetched for the first time cost more than they compute.
-  unsigned key_lo[2], key_hi[2];
+  // Keys that rows g, g + 8 may see are one range each, worked out once: a launch runs this code once, and a division per
+  // score is more instructions to fetch than the launch has time for.  Last keys are inclusive: behind `row + mask_arg` may
+  // be no further 32-bit number.
+  unsigned key_lo[2], key_last[2];
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
     const unsigned row = row_base + g + hr * 8, lo = mask_mode == 2 ? row / mask_arg * mask_arg : 0u;
     key_lo[hr] = lo;
-    key_hi[hr] = mask_mode == 0 ? kv_rows : min(kv_rows, mask_mode == 1 ? row + mask_arg + 1 : lo + mask_arg);
+    key_last[hr] = mask_mode == 0 ? kv_rows - 1 : min(kv_rows - 1, mask_mode == 1 ? row + mask_arg : lo + (mask_arg - 1));
   }
   // Few keys (at most two 16-key blocks, e.g. self-attention over 17 tokens): splitting the keys over warps would
   // leave six warps idle and still pay the merge.  Instead every warp w < dtiles scores ALL keys (the same few
@@ -531,7 +532,7 @@ __device__ __forceinline__ void attention_mma_body(const bf16* q, const bf16* k,
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const unsigned key = key0 + half * 8 + 2 * t + (i & 1);
-          if (key < key_lo[i >> 1] || key >= key_hi[i >> 1]) s[b][half][i] = -3.0e38f;
+          if (key < key_lo[i >> 1] || key > key_last[i >> 1]) s[b][half][i] = -3.0e38f;
         }
     }
     // per-row maximum over the group's keys (own values, then across the quad), one rescale of the running state

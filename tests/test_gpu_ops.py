@@ -216,6 +216,37 @@ def test_attention_with_keys_requested_ahead_of_the_dependency_wait(tmp_path, ca
     assert ops.max_rel_err(got["o_early"], want.reshape(sq, -1)) < MAX_REL
 
 
+FEW_ROW_CASES = [
+    # at most 32 keys and heads up to 64 wide: the split by value columns; otherwise the split by keys
+    (17, 17, 4, 4, 48, "causal", 0),
+    (24, 30, 4, 2, 64, "causal", 6),
+    (20, 20, 4, 4, 32, "block", 7),
+    (30, 20, 2, 2, 48, "block", 10),                     # rows 20 - 29: their block begins behind the last key
+    (64, 33, 2, 1, 16, "block", 11),                     # the same, keys split
+    (50, 70, 4, 2, 128, "block", 33),                    # wide heads, last block cut by the keys
+    (50, 40, 2, 2, 96, "block", 45),                     # ... and a row block of which some rows see keys and some none
+    (17, 30, 2, 2, 48, "causal", 2 ** 32 - 17),          # the last row's offset is the largest 32-bit number: every key
+    (33, 70, 2, 1, 64, "causal", 2 ** 32 - 33),
+    (20, 40, 2, 1, 128, "causal", 2 ** 32 - 20),
+]
+
+
+@pytest.mark.parametrize("case", FEW_ROW_CASES, ids=lambda c: "x".join(map(str, c)))
+def test_attention_of_few_rows_sees_the_masks_keys(tmp_path, case):
+    sq, skv, hq, hkv, d, mask, arg = case
+    q, k, v = randn(sq, hq * d, seed=9), randn(skv, hkv * d, seed=10), randn(skv, hkv * d, seed=11)
+
+    def body(r):
+        r.attention(Tensor("q"), Tensor("k"), Tensor("v"), Tensor("o"), q_rows=sq, kv_rows=skv, q_heads=hq, kv_heads=hkv,
+                    head_dim=d, q_stride=hq * d, k_stride=hkv * d, v_stride=hkv * d, o_stride=hq * d, mask=mask, mask_arg=arg,
+                    algorithm="mma")
+        assert r.profiles[0].launches[-1]["kernel"].startswith("agi_attention_mma_bf16")
+
+    got, _ = run_recipe(tmp_path, {}, {"q": q, "k": k, "v": v}, {"o": (BF, (sq, hq * d))}, body)
+    want = ops.attention(q.view(sq, hq, d), k.view(skv, hkv, d), v.view(skv, hkv, d), mask=mask, mask_arg=arg)
+    assert ops.max_rel_err(got["o"], want.nan_to_num(0.0).reshape(sq, -1)) < MAX_REL      # no visible key: zeros
+
+
 FA_CASES = [
     (288, 288, 16, 2, 128, "causal", 0),     # decoder prefill: grouped-query, 4.5 key tiles
     (512, 512, 16, 16, 80, "block", 64),     # vision windows
