@@ -30,6 +30,7 @@ enum : unsigned {
   kFlagSwiglu = 1u << 13,     // the first two matrices are gate and up of the same width: y = silu(gate) * up
   kFlagMulSilu = 1u << 14,    // y = silu(gate[m, n]) * (...), the gate (bf16, pitch of y) in place of the residual
   kFlagAmax = 1u << 15,       // fold max |y| of the rounded outputs into a zero-initialised word
+  kFlagGroupsFirst = 1u << 16,  // the token groups of a weight tile are neighbours in the grid (or walk), not the tiles of a group
 };
 
 // Programmatic dependent launch: when the loader launches with programmatic stream

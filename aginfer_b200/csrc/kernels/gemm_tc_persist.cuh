@@ -48,6 +48,7 @@ __device__ __forceinline__ void persistent_body(const uint8_t* x, const uint8_t*
 
   const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned n_tiles = (N + kTileN - 1) / kTileN, m_tiles = (M + TN - 1) / TN, tiles = n_tiles * m_tiles;
+  const bool groups_first = (flags & kFlagGroupsFirst) != 0;
   const unsigned nkb = K / kRowBytes;                       // E4M3: one byte per element
   const unsigned stage_bytes = kATileBytes + TN * kRowBytes;
   const unsigned ring = (smem_u32(dynamic_smem) + 1023u) & ~1023u;
@@ -80,8 +81,8 @@ __device__ __forceinline__ void persistent_body(const uint8_t* x, const uint8_t*
       unsigned s = 0, phase = 1, dst = ring;                 // ring position, running across tiles
       const size_t w_block = size_t(w_rows_padded) * kRowBytes, x_block = size_t(ldx) * kRowBytes;
       for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const uint8_t* w_src = w + size_t((tile / m_tiles) * kTileN) * kRowBytes;
-        const uint8_t* x_src = x + size_t((tile % m_tiles) * TN) * kRowBytes;
+        const uint8_t* w_src = w + size_t((groups_first ? tile / m_tiles : tile % n_tiles) * kTileN) * kRowBytes;
+        const uint8_t* x_src = x + size_t((groups_first ? tile % m_tiles : tile / n_tiles) * TN) * kRowBytes;
         for (unsigned kb = 0; kb < nkb; ++kb) {
           wait_or_give_up(&empty_bar[s], phase, status, kTimeoutEmpty | s, &gave_up);
           expect_bytes(&full_bar[s], stage_bytes);
@@ -128,7 +129,8 @@ __device__ __forceinline__ void persistent_body(const uint8_t* x, const uint8_t*
     unsigned it = 0;
     for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
       const unsigned buf = it & 1, use = it >> 1;
-      const unsigned n0 = (tile / m_tiles) * kTileN, m0 = (tile % m_tiles) * TN;
+      const unsigned n0 = (groups_first ? tile / m_tiles : tile % n_tiles) * kTileN;
+      const unsigned m0 = (groups_first ? tile % m_tiles : tile / n_tiles) * TN;
       const unsigned n = n0 + quarter * 32 + lane;
       const float bias_v = ((flags & kFlagBias) && n < N) ? __bfloat162float(bias[n]) : 0.f;
       wait_or_give_up(&acc_full[buf], use & 1, status, kTimeoutAccum | buf, &gave_up);

@@ -227,14 +227,8 @@ __device__ __forceinline__ void add_runs(const float4* filed, float* tile, unsig
   }
 }
 
-// Whether the grid's first dimension is the token groups: the builder's `tk_grid`.  It puts groups first only where neither
-// they nor the tiles are more than 65535; more groups stand in the second dimension, where no launch takes them.
-__device__ __forceinline__ bool groups_first(unsigned M, unsigned tg) { return M > tg && gridDim.x <= 65535; }
-
-// grid = (token groups of `tg` rows, weight tiles of all parts, ranks): the groups of a weight tile run side by side, so that
-// its weights come from HBM once (tiles first, a gate and up pair of 90 MB came in three times for 288 tokens, L2 held none of
-// it until the next group: 49 us instead of 45).  One group, or more tiles than fit the second dimension: grid = (weight
-// tiles, token groups, ranks).  block = kThreads.  NB: weight rows of a tile, a
+// grid = (weight tiles of all parts, token groups of `tg` rows, ranks); with kFlagGroupsFirst the first two change places, so that
+// the groups of a weight tile run side by side (the builder's `groups_first` says when).  block = kThreads.  NB: weight rows of a tile, a
 // multiple of 16 (of 32 with kFlagSwiglu) up to 256; tg a multiple of 8, ceil(tg / 128) * NB' * (runs a rank takes) <=
 // 512 with NB' = NB rounded up to 32.  Dynamic shared memory: 1024 + the larger of the ring, stages * (tg + NB) * 128 plus what the last
 // slot's A tiles overhang (rows past the tokens are read by the MMA, never stored), and the epilogue's tile,
@@ -261,7 +255,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
   if (tile >= t0 + t1) { part = p2; tile -= t0 + t1; }
   else if (tile >= t0) { part = p1; tile -= t0; }
   const unsigned n0 = tile * nb_out;
-  const unsigned m0 = (groups_first(M, tg) ? blockIdx.x : blockIdx.y) * tg, rows = min(tg, M - m0), m_tiles = (rows + 127) / 128;
+  const unsigned m0 = ((flags & kFlagGroupsFirst) ? blockIdx.x : blockIdx.y) * tg, rows = min(tg, M - m0), m_tiles = (rows + 127) / 128;
   const unsigned rank = kCluster ? blockIdx.z : 0, ranks = kCluster ? gridDim.z : 1;
   const unsigned k_blocks = (K * elem) / kRowBytes;
   const unsigned run0 = rank * runs / ranks, my_runs = (rank + 1) * runs / ranks - run0;
@@ -559,7 +553,7 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
     const tk::Part p2 = {reinterpret_cast<const uint8_t*>(w2), bias2, sw2, y2, N2, ldy2};                            \
     tk::body<FP8, PACKED, IN_CLUSTER>(reinterpret_cast<const uint8_t*>(x), scale_a, other, partial, amax_bits,       \
                                          status, M, K, ldx, flags, NB, stages, tg, runs, per_run, p0, p1, p2,         \
-                                         tk::groups_first(M, tg) ? blockIdx.y : blockIdx.x);                                         \
+                                         (flags & kFlagGroupsFirst) ? blockIdx.y : blockIdx.x);                                      \
   }
 // The ranks that share K: grid z = C.  Up to 15 clusters of 8, 33 of 4, 74 of 2 are resident at once.
 #define AGI_TK_CLUSTER(NAME, TYPE, FP8, PACKED, C) AGI_TK_KERNEL(NAME##_c##C, __cluster_dims__(1, 1, C), TYPE, FP8, PACKED, true)
@@ -595,7 +589,7 @@ AGI_TK_CLUSTER(agi_gemm_tc_e4m3_x3, uint8_t, true, false, 8)
 #undef AGI_TK_KERNEL
 
 // Up to 16 independent bf16 GEMMs that share the activation matrix (the K and V projections of every cross-attention
-// block over the context tokens, every block's AdaLN projection) as ONE launch: grid = (token groups, segments * ceil(N / NB));
+// block over the context tokens, every block's AdaLN projection) as ONE launch: grid = (segments * ceil(N / NB), token groups), or the other way round;
 // segment s multiplies by w[s], adds bias[s] and writes y + s * seg_stride elements.
 extern "C" __global__ void __launch_bounds__(tk::kThreads, 2)
 agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsigned N, unsigned K, unsigned ldx,
@@ -607,7 +601,7 @@ agi_gemm_tc_bf16_x16(const bf16* x, bf16* y, unsigned* status, unsigned M, unsig
                      const bf16* b6, const bf16* b7, const bf16* b8, const bf16* b9, const bf16* b10,
                      const bf16* b11, const bf16* b12, const bf16* b13, const bf16* b14, const bf16* b15) {
   const unsigned tiles = (N + NB - 1) / NB;
-  const unsigned at = tk::groups_first(M, tg) ? blockIdx.y : blockIdx.x, seg = at / tiles;
+  const unsigned at = (flags & kFlagGroupsFirst) ? blockIdx.y : blockIdx.x, seg = at / tiles;
   const bf16 *w, *b;
   switch (seg) {
     case 0: w = w0; b = b0; break;    case 1: w = w1; b = b1; break;    case 2: w = w2; b = b2; break;

@@ -30,7 +30,7 @@ SM_COUNT = 148
 
 FLAG_BIAS, FLAG_RESIDUAL, FLAG_OUT_F32, FLAG_SCALED = 1, 2, 1 << 8, 1 << 9
 FLAG_LAYERNORM, FLAG_LN_MODULATE, FLAG_SLAB = 1 << 10, 1 << 11, 1 << 12
-FLAG_SWIGLU, FLAG_MUL_SILU, FLAG_AMAX = 1 << 13, 1 << 14, 1 << 15
+FLAG_SWIGLU, FLAG_MUL_SILU, FLAG_AMAX, FLAG_GROUPS_FIRST = 1 << 13, 1 << 14, 1 << 15, 1 << 16
 ACT = {None: 0, "gelu_tanh": 1 << 4, "silu": 2 << 4, "relu": 3 << 4}
 PLAN_DTYPE_BYTES = {"F32": 4, "F16": 2, "BF16": 2, "F8_E4M3": 1, "I32": 4}
 
@@ -331,14 +331,33 @@ def tcs_tiling(M: int, tiles: int, K: int, cluster: int | None = None, groups: i
 
 
 GRID_SECOND = 65535          # the most a grid's second and third dimensions take
+L2_HALF = 63 << 20           # what one of the two halves of L2 holds
+
+
+def side_by_side(t: Mapping[str, int]) -> bool:
+    """Whether the token groups of a weight tile may be neighbours in the grid: there are some, and the second dimension takes
+    the tiles; more groups than it would take stay there, where a launch refuses them."""
+    return 1 < t["groups"] <= GRID_SECOND >= t["tiles"]
 
 
 def tk_grid(t: Mapping[str, int]) -> tuple[int, int]:
-    """Token groups of a weight tile side by side, unless there is one, or the second dimension does not take the tiles, or
-    it would not take the groups either: the kernel tells the order from a first dimension of at most 65535, so more groups
-    than that stay where a launch refuses them."""
-    tiles, groups = t["tiles"], t["groups"]
-    return (tiles, groups) if groups == 1 or tiles > GRID_SECOND or groups > GRID_SECOND else (groups, tiles)
+    return (t["groups"], t["tiles"]) if side_by_side(t) else (t["tiles"], t["groups"])
+
+
+def groups_first(M: int, N: int, K: int, elem: int, ctas: int) -> bool:
+    """Whether the token groups of a weight tile run side by side, and not the tiles of a token group: a round of CTAs over the
+    SMs then passes over all tokens with a few weight tiles, so weights come from HBM once and tokens once a round, unless L2
+    keeps them.  Not where the tokens are the larger operand, more than half of L2 holds, and there are several rounds:
+    16384 x 2048 x 11008 takes 460 us with the tiles side by side, 487 with the groups (FP8 packed 216, 288), 16384 x 11008 x
+    2048 569 and 612; 4096 x 11008 x 2048 150 and 143, 16384 x 1280 x 1280 66.7 and 64.7."""
+    return M <= N or M * K * elem <= L2_HALF or ctas <= SM_COUNT
+
+
+def tk_order(t: Mapping[str, int], M: int, N: int, K: int, elem: int) -> tuple[tuple[int, int], int]:
+    """(grid, flag) of a product with the tile ``t`` and ``N`` weight rows in all."""
+    if side_by_side(t) and groups_first(M, N, K, elem, t["tiles"] * t["groups"] * t["C"]):
+        return tk_grid(t), FLAG_GROUPS_FIRST
+    return (t["tiles"], t["groups"]), 0
 
 
 STREAM_SPLITS = (4, 2)          # compiled cluster sizes of agi_gemm_stream_bf16_t{1..4}_k{S}
@@ -761,8 +780,8 @@ class RecipeBuilder:
                 self.launch("agi_gemm_tcq_e4m3", (min(tiles, SM_COUNT), 1, 1), (192, 1, 1),
                             [x, w, y, bias or dummy, residual or dummy, scale_a or dummy, scale_w or dummy,
                              Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(padded_token_rows(M)), U32(ldy or N),
-                             U32(flags), U32(TN), U32(stages)], shared_bytes=stages * stage_bytes + 1024,
-                            op="gemm_e4m3_packed", algorithm=f"tcgen05_persistent_128x{TN}_s{stages}")
+                             U32(flags | (FLAG_GROUPS_FIRST if groups_first(M, N, K, 1, tiles) else 0)), U32(TN), U32(stages)],
+                            shared_bytes=stages * stage_bytes + 1024, op="gemm_e4m3_packed", algorithm=f"tcgen05_persistent_128x{TN}_s{stages}")
                 return
             self._gemm_tk("agi_gemm_tcpk_e4m3", "gemm_e4m3_packed", t, x, [(w, bias, scale_w, y, N, ldy or N)], M, K,
                           padded_token_rows(M), flags, scale_a=scale_a, other=residual)
@@ -868,7 +887,9 @@ class RecipeBuilder:
         for i in range(3):
             w, bias, scale, y, N, ldy = parts[i] if i < len(parts) else (dummy, None, None, dummy, 0, 0)
             args += [w, bias or dummy, scale or dummy, y, U32(N), U32(ldy)]
-        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (*tk_grid(t), t["C"]), (288, 1, 1), args,
+        grid, order = tk_order(t, M, sum(p[4] for p in parts), K, 1 if "e4m3" in family else 2)
+        args[9] = U32(args[9].value | order)
+        self.launch(family if t["C"] == 1 else f"{family}_c{t['C']}", (*grid, t["C"]), (288, 1, 1), args,
                     shared_bytes=t["shared_bytes"], op=op,
                     algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_r{t['runs']}_c{t['C']}" + (f"_x{len(parts)}" if len(parts) > 1 else ""))
 
@@ -939,8 +960,9 @@ class RecipeBuilder:
         dummy = Arena(0)
         ws = [p[0] for p in parts] + [dummy] * (16 - len(parts))
         bs = [p[1] for p in parts] + [dummy] * (16 - len(parts))
-        self.launch("agi_gemm_tc_bf16_x16", (*tk_grid(t), 1), (288, 1, 1),
-                    [x, y, Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(ldx or K), U32(N), U32(FLAG_BIAS), U32(t["NB"]),
+        grid, order = tk_order(t, M, N * len(parts), K, 2)
+        self.launch("agi_gemm_tc_bf16_x16", (*grid, 1), (288, 1, 1),
+                    [x, y, Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(ldx or K), U32(N), U32(FLAG_BIAS | order), U32(t["NB"]),
                      U32(t["stages"]), U32(t["tg"]), U32(seg_stride), *ws, *bs], shared_bytes=t["shared_bytes"],
                     op="gemm_bf16_batch", algorithm=f"tcgen05_{t['tg']}x{t['NB']}_s{t['stages']}_x{len(parts)}")
 

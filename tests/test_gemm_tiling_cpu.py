@@ -3,7 +3,7 @@ function of the shape alone."""
 import pytest
 
 from aginfer_b200.recipes import RecipeBuilder, Tensor, qwen_vl
-from aginfer_b200.recipes.builder import TC_SCRATCH_BYTES, TK_CLUSTERS, k_runs, tk_grid, tk_tiling
+from aginfer_b200.recipes.builder import FLAG_GROUPS_FIRST, TC_SCRATCH_BYTES, TK_CLUSTERS, k_runs, tk_grid, tk_tiling
 from aginfer_b200.recipes.package import describe
 
 SHAPES = [(16, 128), (130, 256), (2048, 2048), (11008, 2048), (2048, 11008), (3584, 18944), (151, 640)]
@@ -133,3 +133,32 @@ def test_more_token_groups_than_a_grid_takes_stay_where_the_launch_refuses_them(
     r.gemm_batch(y, [(y, y)] * 2, y, M, N, K, seg_stride=M * N)
     launches = r.profiles[0].launches[before:]
     assert len(launches) == 3 and all(l["grid"][0] <= 4 and l["grid"][1] > 65535 for l in launches)
+
+
+def order(M, N, K, emit):
+    """(grid, groups first) of the launch that ``emit`` adds for token rows M."""
+    y, r = Tensor("y"), RecipeBuilder({"w": ("BF16", [8])})
+    r.begin_profile("default", [], [])
+    emit(r, y, M, N, K)
+    launch = r.profiles[0].launches[-1]
+    flags = launch["arguments"][{"agi_gemm_tcq_e4m3": 13, "agi_gemm_tc_bf16_x16": 8}.get(launch["kernel"], 9)]["scalar_u32"]
+    return launch["grid"], bool(flags & FLAG_GROUPS_FIRST)
+
+
+EMIT = {"gemm": lambda r, y, M, N, K: r.gemm(y, y, y, M, N, K),
+        "group": lambda r, y, M, N, K: r.gemm_group(y, [(y, None, None, y, N // 2, N // 2)] * 2, M, K),
+        "swiglu": lambda r, y, M, N, K: r.gemm_swiglu(y, (y, None, None), (y, None, None), y, M, N // 2, K),
+        "batch": lambda r, y, M, N, K: r.gemm_batch(y, [(y, y)] * 2, y, M, N // 2, K, seg_stride=M * N),
+        "persistent": lambda r, y, M, N, K: r.gemm(y, y, y, M, N, 2 * K, dtype="e4m3", packed=True, tactic="persistent")}
+
+
+@pytest.mark.parametrize("kind", EMIT)
+@pytest.mark.parametrize("M,N,K,first", [(288, 22016, 2048, True), (4096, 2048, 2048, True), (16384, 2048, 1280, True),
+                                         (16384, 2048, 2048, False), (16384, 11008, 2048, False), (16384, 22016, 2048, True)])
+def test_token_groups_run_side_by_side_unless_the_tokens_are_the_larger_operand_and_pass_l2(kind, M, N, K, first):
+    grid, flag = order(M, N, K, EMIT[kind])
+    assert flag == first
+    if kind != "persistent":
+        t = tk_tiling(M, (N,) if kind == "gemm" else (N // 2,) if kind == "swiglu" else (N // 2,) * 2, K, 2, swiglu=kind == "swiglu",
+                      clusters=(1, 2, 4, 8) if kind == "gemm" else (1,))
+        assert grid == [*((t["groups"], t["tiles"]) if first else (t["tiles"], t["groups"])), t["C"]]
