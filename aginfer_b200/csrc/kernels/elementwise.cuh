@@ -26,8 +26,10 @@ extern "C" __global__ void agi_copy_u32(const unsigned* in, unsigned* out, unsig
 
 // amax_bits = max(amax_bits, bits(max |x|)).  Non-negative floats order like their bit
 // patterns, so an integer atomicMax on a zero-initialised word accumulates the maximum.
-// Pairs of bf16 are compared as they are: exact, and NaN loses as in fmaxf.  Bound by the latency of its loads, so four are
-// in flight a thread and not one.
+// Pairs of bf16 are compared as they are: exact, and NaN loses as in fmaxf.  Bound by the latency of its loads: a thread's last
+// three vectors are requested together, and from 4.9 million values up (592 blocks of 256) four at a time before them.  288 x 2048
+// values are one vector a thread, 1024 x 2048 two; there it is the shorter comparison that counts (FP8 sweep of 288 tokens
+// 79.2 -> 78.5 us).
 extern "C" __global__ void agi_absmax_bf16(const bf16* x, unsigned count, unsigned* amax_bits) {
   __shared__ float scratch[32];
   const unsigned vectors = count / 8, step = gridDim.x * blockDim.x;

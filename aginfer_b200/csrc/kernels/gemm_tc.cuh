@@ -52,8 +52,8 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
 }
 // Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
 // hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.  One loop in
-// one statement: a wait that finds its phase complete takes ~70 cycles; as a C++ loop around try_wait it took ~195, and the
-// thread that issues the MMAs waits once per slot of its ring.
+// one statement and not a C++ loop around try_wait: the thread that issues the MMAs waits once per slot of its ring (FP8
+// sweep of 288 tokens 79.9 -> 78.9 us, FP8 prefill of 288 rows 746 -> 740).
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
   unsigned done;
   asm volatile(
