@@ -53,7 +53,8 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
 // Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
 // hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.  One loop in
 // one statement and not a C++ loop around try_wait: the thread that issues the MMAs waits once per slot of its ring (FP8
-// sweep of 288 tokens 79.9 -> 78.9 us, FP8 prefill of 288 rows 746 -> 740).
+// sweep of 288 tokens 79.6 -> 78.2 us, packed prefill of 288 rows 699 -> 694, 50-token chunk 551 -> 538).  Long products, whose
+// waiters mostly find nothing, lose by it: from 4096 rows up 1 - 2 % (bf16 16384 x 2048 x 11008 457 -> 464 us).
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
   unsigned done;
   asm volatile(

@@ -331,7 +331,6 @@ def tcs_tiling(M: int, tiles: int, K: int, cluster: int | None = None, groups: i
 
 
 GRID_SECOND = 65535          # the most a grid's second and third dimensions take
-L2_HALF = 63 << 20           # what one of the two halves of L2 holds
 
 
 def side_by_side(t: Mapping[str, int]) -> bool:
@@ -344,13 +343,19 @@ def tk_grid(t: Mapping[str, int]) -> tuple[int, int]:
     return (t["groups"], t["tiles"]) if side_by_side(t) else (t["tiles"], t["groups"])
 
 
-def groups_first(M: int, N: int, K: int, elem: int, ctas: int) -> bool:
+def groups_first(M: int, N: int, K: int, elem: int, ctas: int, persistent: bool = False) -> bool:
     """Whether the token groups of a weight tile run side by side, and not the tiles of a token group: a round of CTAs over the
-    SMs then passes over all tokens with a few weight tiles, so weights come from HBM once and tokens once a round, unless L2
-    keeps them.  Not where the tokens are the larger operand, more than half of L2 holds, and there are several rounds:
-    16384 x 2048 x 11008 takes 460 us with the tiles side by side, 487 with the groups (FP8 packed 216, 288), 16384 x 11008 x
-    2048 569 and 612; 4096 x 11008 x 2048 150 and 143, 16384 x 1280 x 1280 66.7 and 64.7."""
-    return M <= N or M * K * elem <= L2_HALF or ctas <= SM_COUNT
+    SMs then passes over all tokens with a few weight tiles, so weights come from HBM once, and tokens once a round unless L2
+    keeps them.  Groups | tiles side by side, us:
+    one CTA a tile, several rounds: 4096 x 18944 x 3584 358 | 402, 8192 x 11008 x 2048 291 | 299 (tokens of 32 MB), 12288 x
+    2048 x 11008 360 | 351, 16384 x 11008 x 2048 618 | 576 (64 MB), 32768 x 2048 x 11008 1081 | 835; with more weights than
+    tokens 12288 x 18944 x 3584 1157 | 1202.  The line for tokens lies between FP8 8192 x 2048 x 5504 (43 MB) 74.4 | 76.6 and
+    12288 x 1280 x 5120 (60 MB) 72.9 | 72.0.
+    The persistent walk, FP8, has no second side: 8192 x 2048 x 5504 (43 MB) 63.7 | 68.4, 16384 x 18944 x 3584 (56 MB) 786 | 683,
+    32768 x 2048 x 11008 748 | 428; against it only 16384 x 11008 x 2048 (32 MB) 247 | 236 and 1 - 3 % at 4096 rows."""
+    if ctas <= SM_COUNT:
+        return True
+    return M * K * elem <= 48 << 20 if persistent else M <= N or M * K * elem <= 56 << 20
 
 
 def tk_order(t: Mapping[str, int], M: int, N: int, K: int, elem: int) -> tuple[tuple[int, int], int]:
@@ -780,7 +785,7 @@ class RecipeBuilder:
                 self.launch("agi_gemm_tcq_e4m3", (min(tiles, SM_COUNT), 1, 1), (192, 1, 1),
                             [x, w, y, bias or dummy, residual or dummy, scale_a or dummy, scale_w or dummy,
                              Arena(STATUS_WORD), U32(M), U32(N), U32(K), U32(padded_token_rows(M)), U32(ldy or N),
-                             U32(flags | (FLAG_GROUPS_FIRST if groups_first(M, N, K, 1, tiles) else 0)), U32(TN), U32(stages)],
+                             U32(flags | (FLAG_GROUPS_FIRST if groups_first(M, N, K, 1, tiles, persistent=True) else 0)), U32(TN), U32(stages)],
                             shared_bytes=stages * stage_bytes + 1024, op="gemm_e4m3_packed", algorithm=f"tcgen05_persistent_128x{TN}_s{stages}")
                 return
             self._gemm_tk("agi_gemm_tcpk_e4m3", "gemm_e4m3_packed", t, x, [(w, bias, scale_w, y, N, ldy or N)], M, K,

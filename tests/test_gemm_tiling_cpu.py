@@ -154,10 +154,11 @@ EMIT = {"gemm": lambda r, y, M, N, K: r.gemm(y, y, y, M, N, K),
 
 @pytest.mark.parametrize("kind", EMIT)
 @pytest.mark.parametrize("M,N,K,first", [(288, 22016, 2048, True), (4096, 2048, 2048, True), (16384, 2048, 1280, True),
-                                         (16384, 2048, 2048, False), (16384, 11008, 2048, False), (16384, 22016, 2048, True)])
+                                         (16384, 2048, 2048, False), (16384, 11008, 2048, False), (16384, 22016, 2048, True),
+                                         (8192, 2048, 3072, True), (8192, 2048, 3840, False)])
 def test_token_groups_run_side_by_side_unless_the_tokens_are_the_larger_operand_and_pass_l2(kind, M, N, K, first):
     grid, flag = order(M, N, K, EMIT[kind])
-    assert flag == first
+    assert flag == (first and not (kind == "persistent" and M * 2 * K > 48 << 20))
     if kind != "persistent":
         t = tk_tiling(M, (N,) if kind == "gemm" else (N // 2,) if kind == "swiglu" else (N // 2,) * 2, K, 2, swiglu=kind == "swiglu",
                       clusters=(1, 2, 4, 8) if kind == "gemm" else (1,))

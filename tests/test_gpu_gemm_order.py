@@ -41,7 +41,7 @@ def test_both_orders_give_the_same_product(tmp_path, monkeypatch, M, N, K):
         grids[first] = [tuple(l["grid"]) for l in r.profiles[0].launches if l["kernel"].startswith("agi_gemm_tk_bf16")]
 
     for first in (True, False):
-        monkeypatch.setattr(builder, "groups_first", lambda *a: first)
+        monkeypatch.setattr(builder, "groups_first", lambda *a, **kw: first)
         out = {n: (BF, (M, N)) for n in (*bf, "swiglu", *f8)} | {"status": (torch.int32, (1,))}
         (tmp_path / str(first)).mkdir()
         got[first], _ = run_recipe(tmp_path / str(first), weights, {"x": x.to(BF)}, out, body)
