@@ -51,31 +51,21 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("{ .reg .b64 t; mbarrier.arrive.shared::cta.b64 t, [%0]; }" ::"r"(smem_u32(bar)) : "memory");
 }
 // Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
-// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.  One loop in
-// one statement and not a C++ loop around try_wait: the thread that issues the MMAs waits once per slot of its ring (FP8
-// sweep of 288 tokens 79.6 -> 78.2 us, packed prefill of 288 rows 699 -> 694, 50-token chunk 551 -> 538).  Long products, whose
-// waiters mostly find nothing, lose by it: from 4096 rows up 1 - 2 % (bf16 16384 x 2048 x 11008 457 -> 464 us).
+// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.  Every thread
+// leaves by itself: a warp that goes on to a `.sync.aligned` instruction meets first (`__syncwarp`).
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
-  unsigned done;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      ".reg .u32 n;\n"
-      "mov.u32 n, 0;\n"
-      "WAIT:\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "@p bra DONE;\n"
-      "add.u32 n, n, 1;\n"
-      "setp.lt.u32 p, n, %3;\n"
-      "@p bra WAIT;\n"
-      "DONE:\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity), "n"(kSpinLimit)
-      : "memory");
-  if (__builtin_expect(done == 0, 0)) atomicCAS(status, 0u, code);
-  return done != 0;
+  const unsigned addr = smem_u32(bar);
+  for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
+    unsigned done;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  atomicCAS(status, 0u, code);
+  return false;
 }
 
 __device__ __forceinline__ void cp_async_16(unsigned dst, const void* src) {
@@ -402,6 +392,7 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
   // ---------------- epilogue (warps 0-3: TMEM lanes 32 * warp ... +31) ----------------
   if (warp < 4) {
     if (nkb > 0) mbar_wait(&accum_bar, 0, status, kTimeoutAccum);
+    __syncwarp();
     tc_fence_after();
     const unsigned n = n0 + warp * 32 + lane;
     const float alpha = (flags & kFlagScaled) ? (*scale_a) * (*scale_w) : 1.f;
