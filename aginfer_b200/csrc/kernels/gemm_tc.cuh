@@ -51,8 +51,7 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("{ .reg .b64 t; mbarrier.arrive.shared::cta.b64 t, [%0]; }" ::"r"(smem_u32(bar)) : "memory");
 }
 // Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
-// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.  Every thread
-// leaves by itself: a warp that goes on to a `.sync.aligned` instruction meets first (`__syncwarp`).
+// hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
   const unsigned addr = smem_u32(bar);
   for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
@@ -392,7 +391,6 @@ __device__ __forceinline__ void gemm_body(const uint8_t* x, const uint8_t* w, vo
   // ---------------- epilogue (warps 0-3: TMEM lanes 32 * warp ... +31) ----------------
   if (warp < 4) {
     if (nkb > 0) mbar_wait(&accum_bar, 0, status, kTimeoutAccum);
-    __syncwarp();
     tc_fence_after();
     const unsigned n = n0 + warp * 32 + lane;
     const float alpha = (flags & kFlagScaled) ? (*scale_a) * (*scale_w) : 1.f;

@@ -134,7 +134,6 @@ __device__ __forceinline__ void persistent_body(const uint8_t* x, const uint8_t*
       const unsigned n = n0 + quarter * 32 + lane;
       const float bias_v = ((flags & kFlagBias) && n < N) ? __bfloat162float(bias[n]) : 0.f;
       wait_or_give_up(&acc_full[buf], use & 1, status, kTimeoutAccum | buf, &gave_up);
-      __syncwarp();
       tc_fence_after();
       const unsigned lane_addr = tmem_base + buf * acc_columns + ((quarter * 32u) << 16);
       for (unsigned c0 = 0; c0 < TN; c0 += 16) {

@@ -165,7 +165,6 @@ __device__ __forceinline__ void body(const bf16* x, const Parts& parts, bf16* y,
     float v[32];
     if (nkb > 0) {
       tc::mbar_wait(&accum_bar, 0, status, kTimeoutAccum);
-      __syncwarp();
       tc::tc_fence_after();
       const unsigned lane_addr = tmem_base + ((warp * 32u) << 16);
       tc::tmem_load16(lane_addr, v);

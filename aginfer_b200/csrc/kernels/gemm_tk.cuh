@@ -463,7 +463,6 @@ __device__ __forceinline__ void body(const uint8_t* x, const float* scale_a, con
       if (swiglu) o.alpha2 = (*scale_a) * (*p1.scale);
     }
     if (nkb > 0) mbar_wait(&accum_bar, 0, status, kTimeoutAccum);
-    __syncwarp();
     tc_fence_after();
     for (unsigned mt = 0; mt < m_tiles; ++mt) {
       if (mt * 128 + quarter * 32 < rows) {        // not for a warp whose rows are all past the tokens
