@@ -52,6 +52,8 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
 }
 // Bounded wait; on expiry writes `code` to the status word once and returns false.  try_wait suspends the thread in
 // hardware until the phase completes or a short limit passes: it wakes sooner than a polling loop that sleeps.
+// Not one asm statement with the loop inside: that is 1 - 2 % faster in sweeps and prefills, but with it an episode of 28 decoder and
+// 18 expert layers ended in an illegal memory access, why is not known.
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* status, unsigned code) {
   const unsigned addr = smem_u32(bar);
   for (unsigned spin = 0; spin < kSpinLimit; ++spin) {
